@@ -26,6 +26,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = [
     ("rk4.cu", True),
     ("rk4_shoot.cu", True),
+    ("rk4_exact.cu", True),
     ("sums_fp64.cu", True),
     ("sums_mixed.cu", False),
     ("queue.cu", False),

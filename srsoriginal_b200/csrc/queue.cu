@@ -458,8 +458,8 @@ srs_status srs_trajectory_batch(const srs_field *fields, int32_t nfields, const 
   if (nfields > 0) SRS_CUDA(cudaMemcpyAsync(df.ptr, fields, sizeof(srs_field) * nfields, cudaMemcpyHostToDevice, s));
   SRS_CUDA(cudaMemcpyAsync(dp.ptr, particles, sizeof(srs_particle) * nparticles, cudaMemcpyHostToDevice, s));
   SRS_CUDA(cudaMemcpyAsync(ds.ptr, specs.data(), sizeof(TrajSpec) * nparticles, cudaMemcpyHostToDevice, s));
-  SRS_CUDA(launch_rk4_specs(df.as<srs_field>(), nfields, dp.as<srs_particle>(), ds.as<TrajSpec>(), nparticles, s,
-                            nfields > 0 ? grid_stage_doubles(fields, nfields) : 0, has_electric(fields, nfields)));
+  SRS_CUDA(launch_trajectories(df.as<srs_field>(), nfields, dp.as<srs_particle>(), nparticles, 0.0, 0, 0, nullptr,
+                               nullptr, nullptr, ds.as<TrajSpec>(), specs.data(), s, fields, particles));
   return SRS_OK;
 }
 

@@ -371,50 +371,29 @@ bool has_electric(const srs_field *host_fields, int nfields) {
 
 cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                        double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
-                       cudaStream_t s, int64_t stage_doubles, bool electric) {
+                       cudaStream_t s, int64_t stage_doubles, bool electric, const TrajSpec *d_specs,
+                       const int *d_skip) {
   if (nparticles <= 0) return cudaSuccess;
   if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
   const size_t smem = sizeof(double) * (size_t)stage_doubles;
   const int G = group_size(nparticles, nfields);
   // grouped lanes while there are few particles per SM (the serial chain is the limit); one thread
   // per particle when there are enough particles to fill the SMs (issue rate is the limit)
-  if (G <= 32 && (int64_t)nparticles * G <= 148 * 32 * 48) {
-    if (cudaError_t e = launch_warp_rk4(G, d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a,
-                                        nullptr, stage_doubles, s, nullptr, electric))
-      return e;
-  } else {
-    const int threads = 64;
-    if (electric) {
-      if (cudaError_t e = allow_smem(rk4_thread_kernel<true>, smem)) return e;
-      rk4_thread_kernel<true><<<(nparticles + threads - 1) / threads, threads, smem, s>>>(
-          d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, stage_doubles);
-    } else {
-      if (cudaError_t e = allow_smem(rk4_thread_kernel<false>, smem)) return e;
-      rk4_thread_kernel<false><<<(nparticles + threads - 1) / threads, threads, smem, s>>>(
-          d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, stage_doubles);
-    }
+  if (d_specs || d_skip || (int64_t)nparticles * G <= 148 * 32 * 48) {
+    if (G > 32) return cudaErrorInvalidValue;
+    return launch_warp_rk4(G, d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, d_specs,
+                           stage_doubles, s, d_skip, electric);
   }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_rk4_unless(const srs_field *d_fields, int nfields, const srs_particle *d_particles, double dt,
-                              int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a, cudaStream_t s,
-                              int64_t stage_doubles, const int *d_skip) {
-  if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
-  return launch_warp_rk4(group_size(1, nfields), d_fields, nfields, d_particles, 1, dt, nfwd, nbwd, d_x, d_b, d_a,
-                         nullptr, stage_doubles, s, d_skip);
-}
-
-cudaError_t launch_rk4_specs(const srs_field *d_fields, int nfields, const srs_particle *d_particles,
-                             const TrajSpec *d_specs, int nparticles, cudaStream_t s, int64_t stage_doubles,
-                             bool electric) {
-  if (nparticles <= 0) return cudaSuccess;
-  if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
-  const int G = group_size(nparticles, nfields);
-  if (G > 32) return cudaErrorInvalidValue;
-  if (cudaError_t e = launch_warp_rk4(G, d_fields, nfields, d_particles, nparticles, 0.0, 0, 0, nullptr, nullptr,
-                                      nullptr, d_specs, stage_doubles, s, nullptr, electric))
-    return e;
+  const int threads = 64;
+  if (electric) {
+    if (cudaError_t e = allow_smem(rk4_thread_kernel<true>, smem)) return e;
+    rk4_thread_kernel<true><<<(nparticles + threads - 1) / threads, threads, smem, s>>>(
+        d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, stage_doubles);
+  } else {
+    if (cudaError_t e = allow_smem(rk4_thread_kernel<false>, smem)) return e;
+    rk4_thread_kernel<false><<<(nparticles + threads - 1) / threads, threads, smem, s>>>(
+        d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, stage_doubles);
+  }
   return cudaGetLastError();
 }
 

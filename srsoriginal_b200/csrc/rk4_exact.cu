@@ -1,0 +1,607 @@
+// The serial RK4 trajectory, bit for bit, integrated parallel in time (compiled with -fmad=false).
+//
+// rk4.cu integrates one particle as one chain of ~0.9 us per step (20001 points: 17.3 ms) that no
+// width of the GPU shortens: bound by the latency of ~80 dependent FP64 operations, shuffles and a
+// sine per step.  Almost all of that work depends on the state only weakly: with the state (p, v) at
+// a step's start known approximately, the increments hh*a1, hh*a2, h*a3 and h6*(a1 + a4 + 2(a2 + a3))
+// that the step adds to v are known to a relative error of that size, and what remains serial is one
+// rounded addition per component and step:
+//     v' = RN(v + d),   p' = RN(p + h6*((v + v4) + 2(v3 + v2))),  v2 = RN(v + hh*a1), ...
+// So the recurrence is solved by fixed-point (Picard) iteration on the states of all steps:
+//
+//   pit_pass_kernel    one block per kStepsPerBlock steps: every thread forms its step's increments from
+//                      the last iterate, then the block re-adds its steps in order from its start
+//                      state.  Every block sums the mismatches that the last iteration left between
+//                      the blocks before it and moves its start state by them.  From straight flight
+//                      two iterations gain 3-4 digits for ultra-relativistic particles; the components
+//                      along the flight direction settle on their exact bits here.
+//   pit_steps_kernel   every step's increments from the current states, and the check: the step from
+//                      state j, in the serial kernel's arithmetic, must give state j + 1 bit for bit.
+//                      If that holds for all steps then, by induction from the exact start state,
+//                      the states ARE the serial trajectory.  Also writes the trajectory arrays.
+//   pit_chain_kernel   the additions of a whole chain in order (one warp for v, one for p, tile after
+//                      tile, the other warps feeding them): one rounded addition, 8 cycles, per step
+//                      where the serial kernel needs ~1700.
+//
+// Steps and chain alternate until the check holds; the serial kernel runs if it never does (slow
+// particles in strong fields, where the iteration does not contract): the result is always the serial
+// trajectory, bit for bit.  Both chains of the trajectory (forward from t0, backward) and several
+// particles are integrated side by side.
+//
+// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.28 ms, 40001
+// through two 39.0 -> 0.69 ms, 12001 through a field map in two chains 14.1 -> 0.17 ms, 24 particles of
+// 10001 points 9.1 -> 0.68 ms, 300 points 0.28 -> 0.12 ms.  A pass is bound by latency (~8 us: launch,
+// loads, four field evaluations, 2 x 128 additions in order), the chain by its 20001 additions (~0.1 ms).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "rk4_fields.cuh"
+#include "srs_internal.h"
+
+namespace srs {
+namespace {
+
+constexpr int kStepsPerBlock = 128;  // steps (and threads) of a pass block
+constexpr int kChainTile = 256;      // steps per tile of the chain kernel
+constexpr int kChainThreads = 512;
+constexpr int kPasses = 14;          // passes launched (they return at once when the item is ready)
+constexpr int kContracted = 4;       // by this pass a contracting iteration is far below 1e-4 of the speed
+constexpr int kSweeps = 4;           // exact sweeps before the serial kernel takes over
+
+// One chain of one particle.
+struct Item {
+  int64_t m;       // steps
+  int nblk;        // pass blocks
+  double h, qomg;
+  double s0[6];    // start state: position, velocity
+  double *x, *b, *a;
+  int64_t n;       // points per component
+  int64_t first;   // stored index of state 0 (forward) or of state 1 (backward)
+  int dir;         // +1 forward, -1 backward
+};
+
+// The trajectories to integrate: common settings, or one spec per particle.
+struct Job {
+  const srs_particle *particles;
+  const TrajSpec *specs;
+  double dt;
+  int64_t nfwd, nbwd;
+  double *x, *b, *a;
+  int nparticles, chains;  // chains per particle (2 when some particle has points before t0)
+  int64_t stride;          // doubles per component of an item's states
+  int maxblk;              // pass blocks of the longest chain
+};
+
+struct Scratch {
+  double *S;      // [item][6][stride]: states
+  double *R;      // [item][12][stride]: increments hh*a1, hh*a2, h*a3, d (three components each)
+  double *T[2], *E[2];        // [item][maxblk][6]: start state of a block, state after its last step (pass k: k & 1)
+  int *ready;                 // per item: the pass that found nothing left to settle, or kPasses
+  int *done, *all_ticket;     // the whole job verified; blocks of the steps kernel finished
+  unsigned long long *bad;    // steps that do not reproduce (reset by the last block)
+  int *failed;                // an item whose passes did not converge
+  Prepared *prep;
+};
+
+__device__ inline Item item_of(const Job &J, int it) {
+  Item I;
+  const int p = it / J.chains, chain = it - p * J.chains;
+  const srs_particle &P = J.particles[p];
+  int64_t nf = J.nfwd, nb = J.nbwd;
+  double dt = J.dt;
+  I.n = nf + nb;
+  I.x = J.x + (int64_t)p * 3 * I.n;
+  I.b = J.b + (int64_t)p * 3 * I.n;
+  I.a = J.a + (int64_t)p * 3 * I.n;
+  if (J.specs) {
+    const TrajSpec &s = J.specs[p];
+    nf = s.nfwd;
+    nb = s.nbwd;
+    dt = s.dt;
+    I.n = nf + nb;
+    I.x = s.x;
+    I.b = s.beta;
+    I.a = s.aoc;
+  }
+  I.m = chain == 0 ? (nf > 0 ? nf - 1 : 0) : nb;
+  I.nblk = (int)((I.m + kStepsPerBlock - 1) / kStepsPerBlock);
+  I.h = chain == 0 ? dt : -dt;
+  I.qomg = P.qomg;
+  for (int c = 0; c < 3; ++c) {
+    I.s0[c] = P.x0[c];
+    I.s0[3 + c] = P.beta0[c] * kC;
+  }
+  I.first = chain == 0 ? nb : nb - 1;
+  I.dir = chain == 0 ? 1 : -1;
+  return I;
+}
+
+// The quantities of one serial RK4 step that depend on the state only weakly (OSCARSSR.cc:826-874; the
+// operations and their order are those of rk4.cu): r1 = hh*a1, r2 = hh*a2, r3 = h*a3,
+// d = h6*(a1 + a4 + 2(a3 + a2)).
+struct Increments {
+  V3 r1, r2, r3, d, a1;
+};
+
+__device__ inline V3 scaled(double s, V3 a) { return v3(s * a.x, s * a.y, s * a.z); }
+
+// One copy of the field code: a step evaluates it four times, and a cold instruction cache costs a pass
+// more than the calls.
+__device__ __noinline__ V3 field_total(const Prepared *sp, const srs_field *sf, int nfields, V3 x) {
+  V3 s = v3(0, 0, 0);
+  for (int f = 0; f < nfields; ++f) s = s + field_one(sp[f], sf[f], x);
+  return s;
+}
+
+// The field list and its prepared constants into shared memory, word by word.
+__device__ __forceinline__ void copy_fields(srs_field *sf, Prepared *sp, const srs_field *gf, const Prepared *gp,
+                                            int nfields) {
+  static_assert(sizeof(srs_field) % 8 == 0 && sizeof(Prepared) % 8 == 0, "copied as 8-byte words");
+  const long long *a = reinterpret_cast<const long long *>(gf), *b = reinterpret_cast<const long long *>(gp);
+  long long *c = reinterpret_cast<long long *>(sf), *d = reinterpret_cast<long long *>(sp);
+  for (int k = threadIdx.x; k < nfields * (int)(sizeof(srs_field) / 8); k += blockDim.x) c[k] = a[k];
+  for (int k = threadIdx.x; k < nfields * (int)(sizeof(Prepared) / 8); k += blockDim.x) d[k] = b[k];
+}
+
+__device__ __forceinline__ Increments increments(const Prepared *sp, const srs_field *sf, int nfields, double qomg,
+                                                 double h, V3 pos, V3 vel) {
+  auto B = [&](V3 x) { return field_total(sp, sf, nfields, x); };
+  const double hh = h * 0.5, h6 = h / 6.0;
+  Increments o;
+  o.a1 = force(qomg, vel, B(pos));
+  o.r1 = scaled(hh, o.a1);
+  const V3 v2 = vel + o.r1;
+  const V3 a2 = force(qomg, v2, B(vadd_scaled(pos, hh, vel)));
+  o.r2 = scaled(hh, a2);
+  const V3 v3_ = vel + o.r2;
+  const V3 a3 = force(qomg, v3_, B(vadd_scaled(pos, hh, v2)));
+  o.r3 = scaled(h, a3);
+  const V3 v4 = vel + o.r3;
+  const V3 a4 = force(qomg, v4, B(vadd_scaled(pos, h, v3_)));
+  const V3 m = a3 + a2;
+  o.d = v3(h6 * (o.a1.x + a4.x + 2.0 * m.x), h6 * (o.a1.y + a4.y + 2.0 * m.y), h6 * (o.a1.z + a4.z + 2.0 * m.z));
+  return o;
+}
+
+// the position increment of a component: h6*((v + v4) + 2(v3 + v2))
+__device__ __forceinline__ double advance(double h6, double v, double r1, double r2, double r3) {
+  const double v2 = v + r1, v3_ = v + r2, v4 = v + r3;
+  return h6 * (v + v4 + 2.0 * (v3_ + v2));
+}
+
+// o[j] = the running sum before d[j] is added, for n (a multiple of 16) rounded additions in order; returns
+// the sum.  The next sixteen terms are loaded while the current ones are added, so a step costs the
+// latency of its addition; a 16-byte access covers two steps.
+__device__ __forceinline__ double add_in_order(double acc, const double *__restrict__ d, double *__restrict__ o, int n) {
+  double2 nx[8];
+  const double2 *const d2 = reinterpret_cast<const double2 *>(d);
+  double2 *const o2 = reinterpret_cast<double2 *>(o);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) nx[k] = d2[k];
+  for (int j = 0; j < n / 2; j += 8) {
+    double2 cu[8];
+    const int jn = j + 8 < n / 2 ? j + 8 : j;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      cu[k] = nx[k];
+      nx[k] = d2[jn + k];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      double2 v;
+      v.x = acc;
+      acc += cu[k].x;
+      v.y = acc;
+      acc += cu[k].y;
+      o2[j + k] = v;
+    }
+  }
+  return acc;
+}
+
+__global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ fields, int nfields) {
+  allow_next_grid();
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int items = J.nparticles * J.chains;
+  if (g < nfields) prepare(fields[g], W.prep[g]);
+  if (g == 0) {
+    *W.done = 0;
+    *W.all_ticket = 0;
+    *W.bad = 0;
+    *W.failed = 0;
+  }
+  if (g < items) W.ready[g] = kPasses;
+  if (g >= (int64_t)items * J.maxblk) return;
+  const int it = (int)(g / J.maxblk), s = (int)(g - (int64_t)it * J.maxblk);
+  const Item I = item_of(J, it);
+  const double t = I.h * (double)((int64_t)s * kStepsPerBlock);
+  for (int c = 0; c < 3; ++c) {  // straight flight (the first pass starts from T[1])
+    W.T[1][6 * g + c] = s == 0 ? I.s0[c] : I.s0[c] + I.s0[3 + c] * t;
+    W.T[1][6 * g + 3 + c] = I.s0[3 + c];
+  }
+}
+
+// The mismatches that pass k left between the blocks of an item, summed over the blocks before block s:
+// shift[0..2] of its start position, shift[3..5] of its start velocity (a velocity shift moves the
+// positions of all later blocks).  Every thread gets them; returns whether the item has settled: the
+// transverse mismatches at the rounding of the speed and none in a component that carries the flight
+// (its bits decide the phases); lost: the mismatches are far above that.
+__device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I, int it, int s, int k,
+                                  double (*red)[kStepsPerBlock / 32], double shift[6], bool *lost) {
+  const double *const T = W.T[k & 1] + 6 * (int64_t)it * J.maxblk, *const E = W.E[k & 1] + 6 * (int64_t)it * J.maxblk;
+  const double v2 = mag2(ld3(I.s0 + 3)), hb = I.h * (double)kStepsPerBlock;
+  double sum[6] = {0, 0, 0, 0, 0, 0}, big2 = 0.0;
+  int open = 0;
+  for (int q = threadIdx.x; q < I.nblk - 1; q += kStepsPerBlock) {
+    double t6[6], e6[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      e6[c] = E[6 * q + c];
+      t6[c] = T[6 * (q + 1) + c];
+    }
+    const double left = hb * (double)(s - 1 - q);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double dx = e6[c] - t6[c], dv = e6[3 + c] - t6[3 + c];
+      if (q < s) {
+        sum[c] += dx + dv * left;
+        sum[3 + c] += dv;
+      }
+      big2 = fmax(big2, dv * dv);
+      if ((t6[3 + c] * t6[3 + c] > 0.00390625 * v2 && (dv != 0.0 || dx != 0.0)) || !(dv == dv) || !(dx == dx)) open = 1;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+  if ((threadIdx.x & 31) == 0)
+    for (int c = 0; c < 6; ++c) red[c][threadIdx.x >> 5] = sum[c];
+  open = __syncthreads_or((open || big2 > 1e-32 * v2 ? 1 : 0) | (big2 < 1e-8 * v2 ? 0 : 2));
+  for (int c = 0; c < 6; ++c) {
+    shift[c] = 0.0;
+    for (int w = 0; w < kStepsPerBlock / 32; ++w) shift[c] += red[c][w];
+  }
+  *lost = (open & 2) != 0;
+  return open == 0;
+}
+
+// Picard iteration number `pass` (see the file comment); in the first the states are straight flight.
+__global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_field *__restrict__ gfields, int nfields,
+                                                                  Job J, Scratch W, int pass) {
+  __shared__ srs_field sf[kMaxFieldsShared];
+  __shared__ Prepared sp[kMaxFieldsShared];
+  __shared__ __align__(16) double sd[3][kStepsPerBlock], sv[3][kStepsPerBlock];
+  __shared__ double red[6][kStepsPerBlock / 32];
+  wait_for_previous_grid();
+  allow_next_grid();
+  const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
+  const bool settled = W.ready[it] < pass || *W.failed;
+  const Item I = item_of(J, it);
+  const int64_t blk = (int64_t)it * J.maxblk + s, i = (int64_t)s * kStepsPerBlock + t;
+  copy_fields(sf, sp, gfields, W.prep, nfields);
+  double *const S = W.S + (int64_t)it * 6 * J.stride;
+  double *const T = W.T[pass & 1] + 6 * blk, *const E = W.E[pass & 1] + 6 * blk;
+  const double h = I.h, h6 = h / 6.0;
+  const bool active = i < I.m;
+  V3 vel = ld3(I.s0 + 3), pos = ld3(I.s0) + vel * (h * (double)i);
+  if (pass > 0 && active) {
+    vel = v3(S[3 * J.stride + i], S[4 * J.stride + i], S[5 * J.stride + i]);
+    pos = v3(S[i], S[J.stride + i], S[2 * J.stride + i]);
+  }
+  double start[6];
+  for (int c = 0; c < 6; ++c) start[c] = s < I.nblk ? W.T[(pass + 1) & 1][6 * blk + c] : 0.0;
+  if (settled || s >= I.nblk) return;
+  if (pass > 0) {
+    double shift[6];
+    bool lost;
+    const bool ready = mismatches(J, W, I, it, s, pass - 1, red, shift, &lost);
+    if (lost && pass > kContracted) {
+      if (t == 0) *W.failed = 1;
+      return;
+    }
+    if (ready) {
+      if (t == 0) W.ready[it] = pass - 1;
+      return;
+    }
+    const V3 dv = ld3(shift + 3);
+    vel = vel + dv;
+    pos = pos + ld3(shift) + dv * (h * (double)t);
+    for (int c = 0; c < 6; ++c) start[c] += shift[c];
+  }
+  if (t < 6) T[t] = start[t];
+  __syncthreads();
+  Increments o;
+  o.d = v3(0, 0, 0);
+  if (active) o = increments(sp, sf, nfields, I.qomg, h, pos, vel);
+  sd[0][t] = o.d.x;
+  sd[1][t] = o.d.y;
+  sd[2][t] = o.d.z;
+  __syncthreads();
+  // the block's steps in order from its start state: velocities, then positions (three lanes)
+  if (t < 3) E[3 + t] = add_in_order(t == 0 ? start[3] : t == 1 ? start[4] : start[5], sd[t], sv[t], kStepsPerBlock);
+  __syncthreads();
+  vel = v3(sv[0][t], sv[1][t], sv[2][t]);
+  sd[0][t] = active ? advance(h6, vel.x, o.r1.x, o.r2.x, o.r3.x) : 0.0;
+  sd[1][t] = active ? advance(h6, vel.y, o.r1.y, o.r2.y, o.r3.y) : 0.0;
+  sd[2][t] = active ? advance(h6, vel.z, o.r1.z, o.r2.z, o.r3.z) : 0.0;
+  __syncthreads();
+  if (t < 3) E[t] = add_in_order(t == 0 ? start[0] : t == 1 ? start[1] : start[2], sd[t], sv[t], kStepsPerBlock);
+  __syncthreads();
+  if (active) {
+    S[i] = sv[0][t];
+    S[J.stride + i] = sv[1][t];
+    S[2 * J.stride + i] = sv[2][t];
+    S[3 * J.stride + i] = vel.x;
+    S[4 * J.stride + i] = vel.y;
+    S[5 * J.stride + i] = vel.z;
+  }
+}
+
+// Every step's increments from the current states, the check, and the trajectory arrays (see the file
+// comment).  from_passes: the states still have to be moved by the last pass's shifts.
+__global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_field *__restrict__ gfields, int nfields,
+                                                                   Job J, Scratch W, int from_passes) {
+  __shared__ srs_field sf[kMaxFieldsShared];
+  __shared__ Prepared sp[kMaxFieldsShared];
+  __shared__ double red[6][kStepsPerBlock / 32];
+  wait_for_previous_grid();
+  allow_next_grid();
+  if (*W.done || *W.failed) return;
+  const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
+  const Item I = item_of(J, it);
+  copy_fields(sf, sp, gfields, W.prep, nfields);
+  double shift[6];
+  if (from_passes && s < I.nblk) {
+    bool lost;  // the passes return at once after the one that found the item settled
+    mismatches(J, W, I, it, s, min(W.ready[it], kPasses - 1), red, shift, &lost);
+  }
+  __syncthreads();
+  const int64_t i = (int64_t)s * kStepsPerBlock + t;
+  const double *const S = W.S + (int64_t)it * 6 * J.stride;
+  const double rC = 1.0 / kC;
+  auto store = [&](int64_t k, V3 p, V3 v, V3 a) {
+    I.x[k] = p.x; I.x[I.n + k] = p.y; I.x[2 * I.n + k] = p.z;
+    I.b[k] = div_rn(v.x, kC, rC); I.b[I.n + k] = div_rn(v.y, kC, rC); I.b[2 * I.n + k] = div_rn(v.z, kC, rC);
+    I.a[k] = div_rn(a.x, kC, rC); I.a[I.n + k] = div_rn(a.y, kC, rC); I.a[2 * I.n + k] = div_rn(a.z, kC, rC);
+  };
+  int bad = 0;
+  if (i == 0 && I.dir > 0 && I.n > I.first) store(I.first, ld3(I.s0), ld3(I.s0 + 3), v3(0, 0, 0));
+  if (i < I.m) {
+    auto state = [&](int64_t k, V3 &p, V3 &v) {
+      p = v3(S[k], S[J.stride + k], S[2 * J.stride + k]);
+      v = v3(S[3 * J.stride + k], S[4 * J.stride + k], S[5 * J.stride + k]);
+    };
+    V3 pos, vel;
+    state(i, pos, vel);
+    if (from_passes) {
+      const V3 dv = ld3(shift + 3);
+      vel = vel + dv;
+      pos = pos + ld3(shift) + dv * (I.h * (double)t);
+    }
+    const Increments o = increments(sp, sf, nfields, I.qomg, I.h, pos, vel);
+    double *const R = W.R + (int64_t)it * 12 * J.stride + i;
+    const V3 *const part[4] = {&o.r1, &o.r2, &o.r3, &o.d};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      R[(3 * q) * J.stride] = part[q]->x;
+      R[(3 * q + 1) * J.stride] = part[q]->y;
+      R[(3 * q + 2) * J.stride] = part[q]->z;
+    }
+    if (from_passes) {
+      bad = 1;  // moved by approximate shifts: to be re-added in order first
+    } else {
+      V3 np_, nv;
+      state(i + 1, np_, nv);
+      const double h6 = I.h / 6.0;
+      auto same = [](double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); };
+      bad = !(same(nv.x, vel.x + o.d.x) && same(nv.y, vel.y + o.d.y) && same(nv.z, vel.z + o.d.z) &&
+              same(np_.x, pos.x + advance(h6, vel.x, o.r1.x, o.r2.x, o.r3.x)) &&
+              same(np_.y, pos.y + advance(h6, vel.y, o.r1.y, o.r2.y, o.r3.y)) &&
+              same(np_.z, pos.z + advance(h6, vel.z, o.r1.z, o.r2.z, o.r3.z)));
+      store(I.first + I.dir * (I.dir > 0 ? i + 1 : i), np_, nv, o.a1);
+    }
+  }
+  bad = __syncthreads_count(bad);
+  if (t == 0) {
+    if (bad) atomicAdd(W.bad, (unsigned long long)bad);
+    __threadfence();
+    if (atomicAdd(W.all_ticket, 1) == (int)(gridDim.x * gridDim.y) - 1) {
+      __threadfence();
+      const unsigned long long total = atomicAdd(W.bad, 0ull);
+      *W.bad = 0;
+      *W.all_ticket = 0;
+      *W.done = total == 0;
+    }
+  }
+}
+
+// The additions of one chain in order, tile after tile: warp 0 (three lanes) the velocities of tile k,
+// warp 1 the positions of tile k - 2, the other warps the position increments of tile k - 1, the loads
+// of tile k + 1 and the stores.  Bound by the latency of one FP64 addition (8 cycles) per step.
+__global__ void __launch_bounds__(kChainThreads) pit_chain_kernel(Job J, Scratch W) {
+  __shared__ __align__(16) double sd[2][3][kChainTile], sv[2][3][kChainTile], se[2][3][kChainTile],
+      sx[2][3][kChainTile];
+  wait_for_previous_grid();
+  allow_next_grid();
+  if (*W.done || *W.failed) return;
+  const int it = blockIdx.x, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const Item I = item_of(J, it);
+  if (I.m == 0) return;
+  double *const S = W.S + (int64_t)it * 6 * J.stride;
+  const double *const R = W.R + (int64_t)it * 12 * J.stride;
+  const int64_t tiles = I.m / kChainTile + 1;  // of the m + 1 states
+  const double h6 = I.h / 6.0;
+  // the feeding warps are those of the two schedulers that the adding warps 0 and 1 are not on
+  const bool feeds = (warp & 2) != 0;
+  constexpr int kFeeders = kChainThreads / 2, kEach = 3 * kChainTile / kFeeders;
+  static_assert(kEach * kFeeders == 3 * kChainTile, "the feeders share a tile evenly");
+  const int ft = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
+  auto load = [&](int64_t k) {  // the increments d of tile k (none after the last state)
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+      const int e = ft + q * kFeeders, c = e / kChainTile, j = e % kChainTile;
+      const int64_t g = k * kChainTile + j;
+      sd[k & 1][c][j] = g < I.m ? R[(9 + c) * J.stride + g] : 0.0;
+    }
+  };
+  if (feeds) load(0);
+  double acc = lane < 3 ? (warp == 0 ? I.s0[3 + lane] : I.s0[lane]) : 0.0;
+  __syncthreads();
+  for (int64_t k = 0; k < tiles + 3; ++k) {
+    if (warp == 0) {
+      if (k < tiles && lane < 3) acc = add_in_order(acc, sd[k & 1][lane], sv[k & 1][lane], kChainTile);
+    } else if (warp == 1) {
+      const int64_t kk = k - 2;
+      if (kk >= 0 && kk < tiles && lane < 3) acc = add_in_order(acc, se[kk & 1][lane], sx[kk & 1][lane], kChainTile);
+    } else if (feeds) {
+      const int64_t kv = k - 1, kx = k - 3;
+      if (kv >= 0 && kv < tiles) {
+        double r[kEach][3];
+#pragma unroll
+        for (int q = 0; q < kEach; ++q) {
+          const int e = ft + q * kFeeders, c = e / kChainTile;
+          const int64_t g = kv * kChainTile + e % kChainTile;
+          for (int u = 0; u < 3; ++u) r[q][u] = g < I.m ? R[(3 * u + c) * J.stride + g] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kEach; ++q) {
+          const int e = ft + q * kFeeders, c = e / kChainTile, j = e % kChainTile;
+          const int64_t g = kv * kChainTile + j;
+          const double v = sv[kv & 1][c][j];
+          se[kv & 1][c][j] = g < I.m ? advance(h6, v, r[q][0], r[q][1], r[q][2]) : 0.0;
+          if (g <= I.m) S[(3 + c) * J.stride + g] = v;
+        }
+      }
+      if (k + 1 < tiles) load(k + 1);
+      if (kx >= 0 && kx < tiles) {
+#pragma unroll
+        for (int q = 0; q < kEach; ++q) {
+          const int e = ft + q * kFeeders, c = e / kChainTile, j = e % kChainTile;
+          const int64_t g = kx * kChainTile + j;
+          if (g <= I.m) S[c * J.stride + g] = sx[kx & 1][c][j];
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const TrajSpec *h_specs, int nparticles, double dt,
+             int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a) {
+  Job J;
+  J.particles = d_particles;
+  J.specs = d_specs;
+  J.dt = dt;
+  J.nfwd = nfwd;
+  J.nbwd = nbwd;
+  J.x = d_x;
+  J.b = d_b;
+  J.a = d_a;
+  J.nparticles = nparticles;
+  int64_t mf = nfwd - 1, mb = nbwd;
+  if (h_specs) {
+    mf = mb = 0;
+    for (int p = 0; p < nparticles; ++p) {
+      mf = std::max(mf, h_specs[p].nfwd - 1);
+      mb = std::max(mb, h_specs[p].nbwd);
+    }
+  }
+  J.chains = mb > 0 ? 2 : 1;
+  const int64_t m = std::max<int64_t>(std::max(mf, mb), 0);
+  J.stride = (m + 2) / 2 * 2;
+  J.maxblk = (int)((m + kStepsPerBlock - 1) / kStepsPerBlock);
+  return J;
+}
+
+size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
+  const size_t items = (size_t)J.nparticles * J.chains, blocks = items * (size_t)std::max(1, J.maxblk);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += (bytes + 15) / 16 * 16;
+    return static_cast<char *>(base) + o;
+  };
+  Scratch s;
+  s.S = (double *)take(sizeof(double) * 6 * items * J.stride);
+  s.R = (double *)take(sizeof(double) * 12 * items * J.stride);
+  for (int k = 0; k < 2; ++k) {
+    s.T[k] = (double *)take(sizeof(double) * 6 * blocks);
+    s.E[k] = (double *)take(sizeof(double) * 6 * blocks);
+  }
+  s.ready = (int *)take(sizeof(int) * items);
+  s.done = (int *)take(sizeof(int));
+  s.all_ticket = (int *)take(sizeof(int));
+  s.failed = (int *)take(sizeof(int));
+  s.bad = (unsigned long long *)take(sizeof(unsigned long long));
+  s.prep = (Prepared *)take(sizeof(Prepared) * (size_t)std::max(1, nfields));
+  if (W) *W = s;
+  return off;
+}
+
+}  // namespace
+
+// When the parallel iteration is used: trajectories long enough to pay for its ~30 launches, and few
+// enough of them (the serial kernels integrate up to 592 particles in the time of one, while this one
+// costs ~2.4 ns per step and particle).
+constexpr int64_t kExactMinSteps = 256;
+constexpr int kExactMaxParticles = 128;
+// And only where the iteration contracts: the angle by which the fields could turn a particle over the
+// whole trajectory, |q/(m gamma)| sum |B| T (grids not counted: their samples are on the device).  3 GeV
+// electrons in 1 T over 2 m: 0.2; at 12 (50 MeV) the passes diverge, which costs 0.1-0.2 ms before the
+// serial kernel takes over.
+constexpr double kExactMaxTurn = 3.0;
+
+static double turn_bound(const srs_field *fields, int nfields, const srs_particle *particles, int nparticles, double time) {
+  double b = 0.0, q = 0.0;
+  for (int f = 0; f < nfields; ++f)
+    if (field_shape(fields[f].kind) != SRS_FIELD_GRID) b += mag(ld3(fields[f].field));
+  for (int p = 0; p < nparticles; ++p) q = std::max(q, fabs(particles[p].qomg));
+  return q * b * time;
+}
+
+cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
+                                double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
+                                const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,
+                                const srs_field *host_fields, const srs_particle *host_particles) {
+  if (nparticles <= 0) return cudaSuccess;
+  if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
+  const int64_t stage_doubles = nfields > 0 ? grid_stage_doubles(host_fields, nfields) : 0;
+  const bool electric = has_electric(host_fields, nfields);
+  auto serial = [&](const int *d_skip) {
+    return launch_rk4(d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles,
+                      electric, d_specs, d_skip);
+  };
+  const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
+  const int64_t items = (int64_t)nparticles * J.chains;
+  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles)
+    return serial(nullptr);
+  double time = dt * (double)(nfwd + nbwd);
+  if (host_specs)
+    for (int p = 0; p < nparticles; ++p)
+      time = std::max(time, host_specs[p].dt * (double)(host_specs[p].nfwd + host_specs[p].nbwd));
+  if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) < kExactMaxTurn)) return serial(nullptr);
+  DeviceBuffer scratch;
+  if (scratch.alloc(carve(J, nfields, nullptr, nullptr), s) != cudaSuccess) {
+    cudaGetLastError();  // no room for the states: the serial kernels need none
+    return serial(nullptr);
+  }
+  Scratch W;
+  carve(J, nfields, scratch.ptr, &W);
+  const dim3 grid((unsigned)std::max(1, J.maxblk), (unsigned)items), block(kStepsPerBlock);
+  const int64_t init = std::max<int64_t>(items * std::max(1, J.maxblk), nfields);
+  pit_init_kernel<<<(unsigned)((init + 127) / 128), 128, 0, s>>>(J, W, d_fields, nfields);
+  for (int k = 0; k < kPasses; ++k)
+    if (cudaError_t e = launch_after(pit_pass_kernel, grid, block, 0, s, d_fields, nfields, J, W, k)) return e;
+  for (int k = 0; k <= kSweeps; ++k) {
+    if (cudaError_t e = launch_after(pit_steps_kernel, grid, block, 0, s, d_fields, nfields, J, W, k == 0 ? 1 : 0))
+      return e;
+    if (k == kSweeps) break;
+    if (cudaError_t e = launch_after(pit_chain_kernel, dim3((unsigned)items), dim3(kChainThreads), 0, s, J, W)) return e;
+  }
+  if (cudaError_t e = cudaGetLastError()) return e;
+  return serial(W.done);  // returns at once when the check held
+}
+
+}  // namespace srs

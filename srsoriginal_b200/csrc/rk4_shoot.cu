@@ -620,7 +620,8 @@ cudaError_t launch_rk4_shoot(const srs_field *d_fields, int nfields, const srs_p
   if (d_stats) shoot_stats_kernel<<<1, 1, 0, s>>>(W.flags, W.diag, d_stats);
   if (cudaError_t e = cudaGetLastError()) return e;
   // the serial kernel, which returns at once when the iteration converged
-  return launch_rk4_unless(d_fields, nfields, d_particle, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles, W.flags);
+  return launch_rk4(d_fields, nfields, d_particle, 1, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles, false, nullptr,
+                    W.flags);
 }
 
 }  // namespace srs

@@ -346,8 +346,9 @@ struct srs_sim {
                                 dp.as<srs_particle>(), hp[0], dt, nf, nb, X, B, A, stream, stage, 0, 0, scratch.ptr,
                                 nullptr));
     } else {
-      SRS_CUDA(launch_rk4(reinterpret_cast<const srs_field *>(d_fields), (int)fields.size(), dp.as<srs_particle>(), np,
-                          dt, nf, nb, X, B, A, stream, stage, electric));
+      SRS_CUDA(launch_trajectories(reinterpret_cast<const srs_field *>(d_fields), (int)fields.size(),
+                                   dp.as<srs_particle>(), np, dt, nf, nb, X, B, A, nullptr, nullptr, stream,
+                                   fields.data(), hp.data()));
     }
     view.x = X;
     view.beta = B;

@@ -108,16 +108,18 @@ cudaError_t efield_time(const srs_traj_view &t, double charge, const double obs[
 int64_t grid_stage_doubles(const srs_field *host_fields, int nfields);
 // electric: some of the fields are electric (SRS_FIELD_ELECTRIC); has_electric tells from a HOST array
 bool has_electric(const srs_field *host_fields, int nfields);
+// d_specs: per-particle settings and outputs instead of the common ones; d_skip: return at once when
+// *d_skip != 0.
 cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                        double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
-                       cudaStream_t s, int64_t stage_doubles, bool electric = false);
-cudaError_t launch_rk4_specs(const srs_field *d_fields, int nfields, const srs_particle *d_particles,
-                             const TrajSpec *d_specs, int nparticles, cudaStream_t s, int64_t stage_doubles,
-                             bool electric = false);
-// One particle with the serial warp kernel, which returns at once when *d_skip != 0.
-cudaError_t launch_rk4_unless(const srs_field *d_fields, int nfields, const srs_particle *d_particles, double dt,
-                              int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a, cudaStream_t s,
-                              int64_t stage_doubles, const int *d_skip);
+                       cudaStream_t s, int64_t stage_doubles, bool electric = false, const TrajSpec *d_specs = nullptr,
+                       const int *d_skip = nullptr);
+// The same trajectories bit for bit, parallel in time where that is faster (rk4_exact.cu); host_*: the
+// host copies of the device arrays.
+cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
+                                double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
+                                const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,
+                                const srs_field *host_fields, const srs_particle *host_particles);
 // One particle parallel in time (rk4_shoot.cu); scratch of shoot_scratch_bytes bytes.
 int shoot_default_steps(int64_t nsteps);
 size_t shoot_scratch_bytes(int64_t nfwd, int64_t nbwd, int steps_per_segment, int nfields);

@@ -1,0 +1,80 @@
+"""The parallel-in-time integration of the serial trajectory (srs_trajectory of few particles): every
+point equals the serial kernel's bit for bit.  The serial kernel is reached by integrating more than
+128 copies of the particle at once."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MANY = 129
+
+
+def _fields(name):
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+
+    def shape(kind, b, c, s, rot=(0, 0, 0)):
+        f = _lib.Field()
+        f.kind = kind
+        f.field, f.center, f.sigma_or_width, f.rotations = _lib.v3(b), _lib.v3(c), _lib.v3(s), _lib.v3(rot)
+        return f
+
+    und = D.undulator([0, 1.0, 0], [0, 0, 0.049], 31)
+    if name == "undulator":
+        return [und], None
+    if name == "epu":
+        return [und, D.undulator([0.6, 0, 0], [0, 0, 0.049], 31, phase=math.pi / 2, taper=0.01)], None
+    if name == "none":
+        return [], None
+    if name == "grid":
+        z = np.linspace(-1.05, 1.05, 701)
+        by = np.sin(2 * np.pi * z / 0.049) * (np.abs(z) < 0.8)
+        data = torch.tensor(np.column_stack([0 * by, by, 0 * by]), device="cuda")
+        return [D.grid_z(z[0], z[1] - z[0], by, data)], data
+    return [shape(_lib.GAUSSIAN, (0, 1, 0), (0, 0, 0), (0, 0, 0.05)),
+            shape(_lib.GAUSSIAN, (0.3, 0.4, 0.2), (0, 0, 0.3), (0.01, 0.02, 0.05), (0.1, 0.2, 0.3)),
+            shape(_lib.UNIFORM_BOX, (0, 0.2, 0.1), (0, 0, -0.5), (0, 0, 0.3))], None
+
+
+# The sizes sit at the edges of the blocks (128 steps), of the chain's tiles (256 states) and of the rule
+# (more than 256 steps); "two chains" starts in the middle; 0.05 GeV does not contract and ends in the
+# serial kernel.
+@pytest.mark.parametrize("field,npoints,energy,start", [
+    ("undulator", 257, 3.0, 0.0), ("undulator", 258, 3.0, 0.0), ("undulator", 385, 3.0, 0.0),
+    ("undulator", 512, 3.0, 0.0), ("undulator", 513, 3.0, 0.0), ("undulator", 20001, 2.997, 0.0),
+    ("undulator", 4097, 3.0, -1.0), ("undulator", 3001, 0.05, 0.0), ("undulator", 16641, 0.5, 0.0),
+    ("epu", 9999, 3.0, 0.0), ("epu", 40001, 3.0, 0.0), ("grid", 2049, 3.0, -1.0), ("none", 1025, 3.0, 0.0),
+    ("mixed", 5003, 3.0, -0.7),
+])
+def test_single_trajectory_equals_the_serial_kernel_bitwise(field, npoints, energy, start):
+    import torch
+
+    from srsoriginal_b200 import device as D
+
+    fields, keep = _fields(field)
+    x0 = [1e-5, -2e-5, -1.0 if start == 0.0 else 0.0]
+    part, _ = D.ideal_particle(energy, x0, [3e-6, -5e-6, 1])
+    one = D.trajectory(fields, [part], start, start + 2.0, 0.0, npoints)
+    many = D.trajectory(fields, [part] * MANY, start, start + 2.0, 0.0, npoints)
+    torch.cuda.synchronize()
+    for a in ("x", "beta", "aoc"):
+        assert torch.equal(getattr(one, a)[0], getattr(many, a)[MANY - 1]), a
+
+
+def test_few_particles_together_equal_the_serial_kernel_bitwise():
+    import torch
+
+    from srsoriginal_b200 import device as D
+
+    fields, _ = _fields("undulator")
+    rng = np.random.default_rng(5)
+    parts = [D.ideal_particle(3.0 * (1 + 1e-3 * rng.normal()), [3e-5 * rng.normal(), 1e-5 * rng.normal(), 0.0],
+                              [2e-5 * rng.normal(), 1e-5 * rng.normal(), 1])[0] for _ in range(7)]
+    few = D.trajectory(fields, parts, -1.0, 1.0, 0.0, 3001)
+    many = D.trajectory(fields, parts * 19, -1.0, 1.0, 0.0, 3001)
+    torch.cuda.synchronize()
+    for a in ("x", "beta", "aoc"):
+        assert torch.equal(getattr(few, a), getattr(many, a)[:7]), a
