@@ -7,10 +7,8 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <map>
-#include <mutex>
-#include <utility>
 
+#include "splits.h"
 #include "srs_device.cuh"
 
 namespace srs {
@@ -72,30 +70,6 @@ inline int splits_for(int64_t ctas, int64_t n, int64_t min_chunk, int64_t slots)
     }
   }
   return best_s;
-}
-
-// Resident CTAs of `kernel` (kThreads threads, no dynamic shared memory) on the current device,
-// queried once per (kernel, device): the launchers ask on every call.
-template <typename K>
-inline int64_t wave_slots(K kernel) {
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, int64_t> cache;
-  int dev = 0, sms = 148, occ = 1;
-  const bool have_dev = cudaGetDevice(&dev) == cudaSuccess;
-  const auto key = std::make_pair(reinterpret_cast<const void *>(kernel), dev);
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-  }
-  if (have_dev) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, 0) != cudaSuccess || occ < 1) occ = 1;
-  const int64_t slots = (int64_t)sms * occ;
-  if (have_dev) {
-    std::lock_guard<std::mutex> lk(mu);
-    cache[key] = slots;
-  }
-  return slots;
 }
 
 // Observation-grid tiles.  The u2 axis is cut into strips of balanced width (8 to 16 points when the

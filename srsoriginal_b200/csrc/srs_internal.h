@@ -169,10 +169,11 @@ cudaError_t mixed_power_density(const srs_traj_view &t, const srs_beam_consts &b
                                 int directional, double *d_out, void *scratch, cudaStream_t s);
 
 // Finishing kernels shared by both precisions: add the S per-chunk partial sums in chunk order and
-// apply the reference's final scaling.
+// apply the reference's final scaling.  Angular frequencies per output from energies (eV) or omegas when
+// given, else omega0.
 cudaError_t finish_flux_partials(const double *partial, int S, int64_t nout, int nparticles, const double *omegas,
                                  double omega0, double dt, double C0, double C2, double *out, cudaStream_t s,
-                                 double *e6 = nullptr);
+                                 double *e6 = nullptr, const double *energies = nullptr);
 cudaError_t finish_pd_partials(const double *partial, int S, int64_t np, int nparticles, double cdt, int directional,
                                double *out, cudaStream_t s);
 

@@ -1,5 +1,5 @@
-// Plain FP64 radiation sums: the drop-in for the reference's GPU/CPU sums, in the reference's
-// IEEE-double operation order (this file is compiled with -fmad=false).
+// Plain FP64 radiation sums: the drop-in for the reference's GPU/CPU sums (this file is compiled with
+// -fmad=false; fused operations are written out).
 //
 //   spectrum  : OSCARSSR::CalculateSpectrum   src/OSCARSSR.cc:1154-1251 (energy loop :1202-1246)
 //   flux      : OSCARSSR::CalculateFlux2      src/OSCARSSR.cc:1989-2099 (point loop :2054-2096)
@@ -7,16 +7,21 @@
 //   total pow : OSCARSSR::CalculateTotalPower src/OSCARSSR.cc:1939-1978
 //
 // Per term the flux/spectrum integrand is (beta - n (1 + i c/(w D)))/D exp(i w (i dt + D/c)), summed
-// over trajectory points; the phase w*(i*dt + D/c) is formed exactly as the reference forms it and
-// reduced modulo 2*pi (Cody-Waite, three-part 2*pi, FMA) before the FP64 sincos, which is then
-// evaluated on |r| <= pi.
-//
-// Divisions: every division of a term by the same distance D (or D^2, or (1 - n.beta)^5) is formed
-// from one correctly rounded reciprocal (__drcp_rn) by Markstein's correction (div_rn), which gives
-// the correctly rounded quotient, i.e. the IEEE division's result bit for bit, in three instructions
-// instead of a division sequence each (normal operands: D, 1/D and the quotients of these sums are far
-// from overflow and underflow).  The power density's (1 - n.beta)^5 is formed by multiplications
-// (x^2 x^2 x, within two ulps of the reference's std::pow(x, 5)).
+// over trajectory points.  What decides the result's bits is kept in the reference's IEEE operation
+// order: D = RN(sqrt(|R|^2)) and the phase w*(i*dt + D/c) (~1e11 rad: one rounding of it moves a
+// term by ~1e-5 rad), and for the power density n = R/D and 1 - n.beta (~1e-8, raised to the fifth
+// power).  Everything after them only carries relative errors of ~1e-16 into the term, so it is
+// arranged for the FP64 pipe, which bounds these kernels (a fused multiply-add is one operation):
+//  * D, 1/D and the quotients by D from one reciprocal square root (sqrt_both, div_rn): no division
+//    sequence;
+//  * the phase reduced to |r| <= pi/4 in four operations and its sine and cosine from two polynomials
+//    (sincos_reduced): 20 operations per term;
+//  * the near-field term i c/(w D) n/D and the factor 1/D applied to the phasor instead of to the six
+//    amplitude components, the sums as fused multiply-adds;
+//  * the power density's |V|^2 as the sum of V's squared components (V is perpendicular to n, so the
+//    reference's two projections on a basis normal to n add up to it).
+// Operations per term: flux 63, spectrum 33, power density 63 (127, ~75 and ~165 when every step was in
+// the reference's order).
 //
 // Parallel layout (B200: 148 SMs): one thread per output (energy or observation point), 128 outputs
 // per CTA, and the trajectory axis split into S contiguous chunks across CTAs so that small outputs
@@ -28,7 +33,9 @@
 #include <cuda_pipeline.h>
 
 #include <algorithm>
+#include <cstdint>
 
+#include "splits.h"
 #include "srs_device.cuh"
 #include "srs_internal.h"
 
@@ -38,22 +45,73 @@ namespace {
 
 constexpr int kTile = 128;     // outputs per CTA and trajectory points per shared-memory tile
 
-// a / b for the three components, from rb = RN(1/b)
-__device__ __forceinline__ V3 div3_rn(V3 a, double b, double rb) {
-  return v3(div_rn(a.x, b, rb), div_rn(a.y, b, rb), div_rn(a.z, b, rb));
+// m = RN(sqrt(a)) and y = 1/sqrt(a) to about an ulp, for normal positive a: the hardware's approximation
+// (rsqrt.approx.ftz.f64, ~20 bits), one third-order Newton step, and the correctly rounded root from the
+// exact remainder a - g^2 (P. Markstein, IBM J. Res. Dev. 34(1), 1990).
+__device__ __forceinline__ void sqrt_both(double a, double &m, double &y) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+  const double e = __fma_rn(-(a * y0), y0, 1.0);
+  y = __fma_rn(y0 * e, __fma_rn(0.375, e, 0.5), y0);
+  const double g = a * y, r = __fma_rn(-g, g, a);
+  m = __fma_rn(r, 0.5 * y, g);
 }
-// a / |a| (TVector3D::UnitVector), the three divisions from one reciprocal
-__device__ __forceinline__ V3 unit_rn(V3 a) {
-  const double m = mag(a);
-  return div3_rn(a, m, __drcp_rn(m));
-}
-constexpr int kTargetCtas = 148 * 8;
 
-int choose_splits(int64_t ctas_without_split, int64_t n) {
-  int64_t s = (kTargetCtas + ctas_without_split - 1) / std::max<int64_t>(1, ctas_without_split);
-  int64_t max_s = std::max<int64_t>(1, (n + 255) / 256);
-  s = std::min<int64_t>(std::max<int64_t>(s, 1), std::min<int64_t>(max_s, 65535));
-  return (int)s;
+// 1/a to about an ulp, for normal a: the hardware's approximation and two Newton steps.
+__device__ __forceinline__ double reciprocal(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  x = __fma_rn(x, __fma_rn(-a, x, 1.0), x);
+  return __fma_rn(x, __fma_rn(-a, x, 1.0), x);
+}
+
+// sin and cos of x for |x| < 2^46: x = k pi/2 + r by Cody & Waite's steps (k from the 1.5 * 2^52 shift; a
+// third part of pi/2, below |k| * 2e-33, would not be seen), then sin r = r + r^3 S(r^2) and cos r = 1 -
+// r^2/2 + r^4 C(r^2) with S and C the degree-5 interpolants at the Chebyshev nodes of [0, (pi/4)^2] of
+// (sin(r)/r - 1)/r^2 and (cos(r) - 1 + r^2/2)/r^4: 1e-17 and 5e-19 from the functions.
+__device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs) {
+  const double shift = 6755399441055744.0;
+  const double kd = __fma_rn(x, 0.6366197723675814, shift);
+  const int k = __double2loint(kd);
+  const double kf = kd - shift;
+  double r = __fma_rn(-kf, 1.5707963267948966, x);
+  r = __fma_rn(-kf, 6.123233995736766e-17, r);
+  const double w = r * r;
+  double s = __fma_rn(w, 1.5918129266803394e-10, -2.5051131844614108e-08);
+  double c = __fma_rn(w, -1.1382632407965617e-11, 2.087614626815952e-09);
+  s = __fma_rn(w, s, 2.755731610255057e-06);
+  c = __fma_rn(w, c, -2.7557317271728623e-07);
+  s = __fma_rn(w, s, -0.0001984126983675857);
+  c = __fma_rn(w, c, 2.4801587298765686e-05);
+  s = __fma_rn(w, s, 0.008333333333330948);
+  c = __fma_rn(w, c, -0.0013888888888887398);
+  s = __fma_rn(w, s, -0.16666666666666666);
+  c = __fma_rn(w, c, 0.041666666666666664);
+  s = __fma_rn(r * w, s, r);
+  c = __fma_rn(w * w, c, __fma_rn(-0.5, w, 1.0));
+  const double a = (k & 1) ? c : s, b = (k & 1) ? s : c;
+  sn = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(k & 2) << 30), __double2loint(a));
+  cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((k + 1) & 2) << 30), __double2loint(b));
+}
+
+// Trajectory points per CTA for `ctas` tiles of outputs: the split of least waves * (points + overhead)
+// over the launches of up to six full waves, in multiples of 32 points (a small output then still
+// spreads over the GPU).
+int64_t chunk_for(int64_t ctas, int64_t n, int64_t slots) {
+  constexpr int64_t kGranule = 32, kOverhead = 24;
+  int64_t best = n, best_cost = INT64_MAX;
+  for (int64_t w = 1; w <= 6; ++w) {
+    const int64_t s = std::min<int64_t>(std::max<int64_t>(1, w * slots / std::max<int64_t>(1, ctas)), 65535);
+    int64_t chunk = ((n + s - 1) / s + kGranule - 1) / kGranule * kGranule;
+    chunk = std::max(chunk, (n + 65534) / 65535);
+    const int64_t used = (n + chunk - 1) / chunk, waves = (ctas * used + slots - 1) / slots;
+    const int64_t cost = waves * (chunk + kOverhead);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = chunk;
+    }
+  }
+  return best;
 }
 
 // ---------------------------------------------------------------- flux at observation points
@@ -62,7 +120,9 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
                                                           int64_t n, double dt, const double *__restrict__ pts,
                                                           int64_t np, double omega, int64_t chunk,
                                                           double *__restrict__ partial) {
-  __shared__ double sx[3][kTile], sb[3][kTile];
+  __shared__ double2 tile[4][kTile];  // (x, y), (z, i dt), (beta_x, beta_y), (beta_z, -)
+  wait_for_previous_grid();  // (launched with launch_after)
+  allow_next_grid();
   const int tid = threadIdx.x;
   const int64_t j = (int64_t)blockIdx.x * kTile + tid;
   const int s = blockIdx.y, S = gridDim.y, p = blockIdx.z;
@@ -76,30 +136,31 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
     const int cnt = (int)imin64(kTile, i1 - base);
     __syncthreads();
     if (tid < cnt) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sx[c][tid] = xp[c * n + base + tid];
-        sb[c][tid] = bp[c * n + base + tid];
-      }
+      const int64_t i = base + tid;
+      tile[0][tid] = make_double2(xp[i], xp[n + i]);
+      tile[1][tid] = make_double2(xp[2 * n + i], dt * (double)(int)i);
+      tile[2][tid] = make_double2(bp[i], bp[n + i]);
+      tile[3][tid] = make_double2(bp[2 * n + i], 0.0);
     }
     __syncthreads();
     if (!active) continue;
+#pragma unroll 2
     for (int k = 0; k < cnt; ++k) {
-      V3 R = obs - v3(sx[0][k], sx[1][k], sx[2][k]);
-      double m = mag(R);
-      const double rm = __drcp_rn(m);
-      V3 N = div3_rn(R, m, rm);
-      double ph = omega * (dt * (double)(int)(base + k) + div_rn(m, kC, rc));
-      double sn, cs;
-      sincos(reduce_2pi(ph), &sn, &cs);
-      double f = div_rn(icow, m, rm);
-      double ar, ai;
-      ar = div_rn(sb[0][k] - N.x, m, rm); ai = div_rn(-(N.x * f), m, rm);
-      axr += ar * cs - ai * sn; axi += ar * sn + ai * cs;
-      ar = div_rn(sb[1][k] - N.y, m, rm); ai = div_rn(-(N.y * f), m, rm);
-      ayr += ar * cs - ai * sn; ayi += ar * sn + ai * cs;
-      ar = div_rn(sb[2][k] - N.z, m, rm); ai = div_rn(-(N.z * f), m, rm);
-      azr += ar * cs - ai * sn; azi += ar * sn + ai * cs;
+      const double2 q0 = tile[0][k], q1 = tile[1][k], q2 = tile[2][k];
+      const double bz = tile[3][k].x;
+      const V3 R = obs - v3(q0.x, q0.y, q1.x);
+      double m, y, sn, cs;
+      sqrt_both(mag2(R), m, y);
+      sincos_reduced(omega * (q1.y + div_rn(m, kC, rc)), sn, cs);
+      // (beta - n)/D e^{i phi} - i (c/w) n/D^2 e^{i phi}, with e^{i phi}/D = (cr, ci)
+      const double cr = y * cs, ci = y * sn, f = icow * y * y, fr = f * cr, fi = f * ci;
+      const double dx = __fma_rn(-R.x, y, q2.x), dy = __fma_rn(-R.y, y, q2.y), dz = __fma_rn(-R.z, y, bz);
+      axr = __fma_rn(dx, cr, __fma_rn(R.x, fi, axr));
+      axi = __fma_rn(dx, ci, __fma_rn(-R.x, fr, axi));
+      ayr = __fma_rn(dy, cr, __fma_rn(R.y, fi, ayr));
+      ayi = __fma_rn(dy, ci, __fma_rn(-R.y, fr, ayi));
+      azr = __fma_rn(dz, cr, __fma_rn(R.z, fi, azr));
+      azi = __fma_rn(dz, ci, __fma_rn(-R.z, fr, azi));
     }
   }
   if (active) {
@@ -118,7 +179,8 @@ constexpr int kRedPoints = 32;
 constexpr int kRedBatch = 24;
 __global__ void __launch_bounds__(6 * kRedPoints) flux_fp64_reduce(const double *__restrict__ partial, int S,
                                                                    int64_t np, int nparticles,
-                                                                   const double *__restrict__ omegas, double omega0,
+                                                                   const double *__restrict__ omegas,
+                                                                   const double *__restrict__ energies, double omega0,
                                                                    double dt, double C0, double C2,
                                                                    double *__restrict__ out, double *__restrict__ e6) {
   __shared__ double se[kRedPoints][7];
@@ -148,7 +210,7 @@ __global__ void __launch_bounds__(6 * kRedPoints) flux_fp64_reduce(const double 
     double e[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) e[q] = se[k][q];
-    const double omega = omegas ? omegas[idx % np] : omega0;
+    const double omega = energies ? ev_to_omega(energies[idx % np]) : omegas ? omegas[idx % np] : omega0;
     out[idx] = finish_flux(e, omega, dt, C0, C2);
     if (e6) {
 #pragma unroll
@@ -164,8 +226,12 @@ __global__ void __launch_bounds__(kTile) spectrum_fp64_kernel(const double *__re
                                                               V3 obs, const double *__restrict__ energies,
                                                               int64_t ne, int64_t chunk,
                                                               double *__restrict__ partial) {
-  // Per trajectory point (energy independent): n = R/|R|, D, tau = i*dt + D/c, (beta - n)/D.
-  __shared__ double sN[3][kTile], sD[kTile], sR[kTile], sT[kTile], sA[3][kTile];
+  // Per trajectory point (energy independent): tau = i*dt + D/c, a = (beta - n)/D, b = n/D^2, as
+  // (tau, a_x), (a_y, a_z), (b_x, b_y), (b_z, -).  The near-field part -i (c/w) sum b e^{i w tau} is summed
+  // without its factor, which is applied once per chunk.
+  __shared__ double2 tile[4][kTile];
+  wait_for_previous_grid();  // (launched with launch_after)
+  allow_next_grid();
   const int tid = threadIdx.x;
   const int64_t k = (int64_t)blockIdx.x * kTile + tid;
   const int s = blockIdx.y, S = gridDim.y, p = blockIdx.z;
@@ -174,49 +240,45 @@ __global__ void __launch_bounds__(kTile) spectrum_fp64_kernel(const double *__re
   const bool active = k < ne;
   const double omega = active ? ev_to_omega(energies[k]) : 1.0;
   const double icow = kC / omega;
-  double axr = 0, axi = 0, ayr = 0, ayi = 0, azr = 0, azi = 0;
+  double a[6] = {0, 0, 0, 0, 0, 0}, b[6] = {0, 0, 0, 0, 0, 0};
   for (int64_t base = i0; base < i1; base += kTile) {
     const int cnt = (int)imin64(kTile, i1 - base);
     __syncthreads();
     if (tid < cnt) {
       const int64_t i = base + tid;
-      V3 R = obs - v3(xp[i], xp[n + i], xp[2 * n + i]);
-      double m = mag(R);
-      const double rm = __drcp_rn(m);
-      V3 N = div3_rn(R, m, rm);
-      sN[0][tid] = N.x; sN[1][tid] = N.y; sN[2][tid] = N.z;
-      sD[tid] = m;
-      sR[tid] = rm;
-      sT[tid] = dt * (double)(int)i + div_rn(m, kC, 1.0 / kC);
-      sA[0][tid] = div_rn(bp[i] - N.x, m, rm);
-      sA[1][tid] = div_rn(bp[n + i] - N.y, m, rm);
-      sA[2][tid] = div_rn(bp[2 * n + i] - N.z, m, rm);
+      const V3 R = obs - v3(xp[i], xp[n + i], xp[2 * n + i]);
+      double m, y;
+      sqrt_both(mag2(R), m, y);
+      const double y2 = y * y, y3 = y2 * y;
+      tile[0][tid] = make_double2(dt * (double)(int)i + div_rn(m, kC, 1.0 / kC), __fma_rn(-R.x, y, bp[i]) * y);
+      tile[1][tid] = make_double2(__fma_rn(-R.y, y, bp[n + i]) * y, __fma_rn(-R.z, y, bp[2 * n + i]) * y);
+      tile[2][tid] = make_double2(R.x * y3, R.y * y3);
+      tile[3][tid] = make_double2(R.z * y3, 0.0);
     }
     __syncthreads();
     if (!active) continue;
+#pragma unroll 2
     for (int q = 0; q < cnt; ++q) {
-      const double m = sD[q], rm = sR[q];
+      const double2 q0 = tile[0][q], q1 = tile[1][q], q2 = tile[2][q];
+      const double bz = tile[3][q].x;
       double sn, cs;
-      sincos(reduce_2pi(omega * sT[q]), &sn, &cs);
-      const double f = div_rn(icow, m, rm);
-      double ar, ai;
-      ar = sA[0][q]; ai = div_rn(-(sN[0][q] * f), m, rm);
-      axr += ar * cs - ai * sn; axi += ar * sn + ai * cs;
-      ar = sA[1][q]; ai = div_rn(-(sN[1][q] * f), m, rm);
-      ayr += ar * cs - ai * sn; ayi += ar * sn + ai * cs;
-      ar = sA[2][q]; ai = div_rn(-(sN[2][q] * f), m, rm);
-      azr += ar * cs - ai * sn; azi += ar * sn + ai * cs;
+      sincos_reduced(omega * q0.x, sn, cs);
+      a[0] = __fma_rn(q0.y, cs, a[0]); a[1] = __fma_rn(q0.y, sn, a[1]);
+      a[2] = __fma_rn(q1.x, cs, a[2]); a[3] = __fma_rn(q1.x, sn, a[3]);
+      a[4] = __fma_rn(q1.y, cs, a[4]); a[5] = __fma_rn(q1.y, sn, a[5]);
+      b[0] = __fma_rn(q2.x, cs, b[0]); b[1] = __fma_rn(q2.x, sn, b[1]);
+      b[2] = __fma_rn(q2.y, cs, b[2]); b[3] = __fma_rn(q2.y, sn, b[3]);
+      b[4] = __fma_rn(bz, cs, b[4]); b[5] = __fma_rn(bz, sn, b[5]);
     }
   }
   if (active) {
     double *o = partial + ((int64_t)p * S + s) * 6 * ne + k;
-    o[0] = axr; o[ne] = axi; o[2 * ne] = ayr; o[3 * ne] = ayi; o[4 * ne] = azr; o[5 * ne] = azi;
+#pragma unroll
+    for (int c = 0; c < 6; c += 2) {
+      o[c * ne] = __fma_rn(icow, b[c + 1], a[c]);
+      o[(c + 1) * ne] = __fma_rn(-icow, b[c], a[c + 1]);
+    }
   }
-}
-
-__global__ void omegas_kernel(const double *__restrict__ e, int64_t ne, double *__restrict__ w) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ne) w[i] = ev_to_omega(e[i]);
 }
 
 // ---------------------------------------------------------------- power density
@@ -227,46 +289,52 @@ __global__ void __launch_bounds__(kTile) pd_fp64_kernel(const double *__restrict
                                                         const double *__restrict__ nrms, int64_t np,
                                                         int directional, int64_t chunk,
                                                         double *__restrict__ partial) {
-  __shared__ double sx[3][kTile], sb[3][kTile], sa[3][kTile];
+  __shared__ double2 tile[5][kTile];  // (x, y), (z, beta_x), (beta_y, beta_z), (a_x, a_y), (a_z, -)
+  wait_for_previous_grid();  // (launched with launch_after)
+  allow_next_grid();
   const int tid = threadIdx.x;
   const int64_t j = (int64_t)blockIdx.x * kTile + tid;
   const int s = blockIdx.y, S = gridDim.y, p = blockIdx.z;
   const int64_t off = (int64_t)p * 3 * n;
+  const double *xp = X + off, *bp = Bt + off, *ap = A + off;
   const int64_t i0 = (int64_t)s * chunk, i1 = imin64(n, i0 + chunk);
   const bool active = j < np;
   V3 obs = active ? v3(pts[3 * j], pts[3 * j + 1], pts[3 * j + 2]) : v3(0, 0, 1);
   V3 nrm = active ? v3(nrms[3 * j], nrms[3 * j + 1], nrms[3 * j + 2]) : v3(0, 0, 1);
   double sum = 0;
+  // a x b with one rounding less per component
+  auto fcross = [](V3 a, V3 b) {
+    return v3(__fma_rn(a.y, b.z, -(b.y * a.z)), __fma_rn(a.z, b.x, -(b.z * a.x)), __fma_rn(a.x, b.y, -(b.x * a.y)));
+  };
   for (int64_t base = i0; base < i1; base += kTile) {
     const int cnt = (int)imin64(kTile, i1 - base);
     __syncthreads();
     if (tid < cnt) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sx[c][tid] = X[off + c * n + base + tid];
-        sb[c][tid] = Bt[off + c * n + base + tid];
-        sa[c][tid] = A[off + c * n + base + tid];
-      }
+      const int64_t i = base + tid;
+      tile[0][tid] = make_double2(xp[i], xp[n + i]);
+      tile[1][tid] = make_double2(xp[2 * n + i], bp[i]);
+      tile[2][tid] = make_double2(bp[n + i], bp[2 * n + i]);
+      tile[3][tid] = make_double2(ap[i], ap[n + i]);
+      tile[4][tid] = make_double2(ap[2 * n + i], 0.0);
     }
     __syncthreads();
     if (!active) continue;
+#pragma unroll 2
     for (int k = 0; k < cnt; ++k) {
-      const V3 Xk = v3(sx[0][k], sx[1][k], sx[2][k]);
-      const V3 B = v3(sb[0][k], sb[1][k], sb[2][k]);
-      const V3 AC = v3(sa[0][k], sa[1][k], sa[2][k]);
-      const V3 N1 = unit_rn(obs - Xk);
-      const V3 N2 = unit_rn(orthogonal(N1));
-      const V3 N3 = unit_rn(cross(N1, N2));
-      const double nd = dot(N1, nrm);
-      if (directional && nd <= 0) continue;
-      const V3 num = cross(N1, cross(N1 - B, AC));
-      const double omb = 1 - dot(B, N1), omb2 = omb * omb;
-      const double den = omb2 * omb2 * omb;
-      const double p2 = dot(num, N2), p3 = dot(num, N3);
-      const double m2 = mag2(obs - Xk);
-      const double rden = __drcp_rn(den), rm2 = __drcp_rn(m2);
-      sum += div_rn(div_rn(p2 * p2, den, rden), m2, rm2) * nd;
-      sum += div_rn(div_rn(p3 * p3, den, rden), m2, rm2) * nd;
+      const double2 q0 = tile[0][k], q1 = tile[1][k], q2 = tile[2][k], q3 = tile[3][k];
+      const V3 B = v3(q1.y, q2.x, q2.y), AC = v3(q3.x, q3.y, tile[4][k].x);
+      const V3 R = obs - v3(q0.x, q0.y, q1.x);
+      const double m2 = mag2(R);
+      double m, y;
+      sqrt_both(m2, m, y);
+      const V3 N = v3(div_rn(R.x, m, y), div_rn(R.y, m, y), div_rn(R.z, m, y));  // RN(R / D)
+      const double nd = __fma_rn(N.z, nrm.z, __fma_rn(N.y, nrm.y, N.x * nrm.x));
+      const V3 V = fcross(N, fcross(N - B, AC));
+      const double omb = 1 - dot(B, N), omb2 = omb * omb;
+      const double den = omb2 * omb2 * (omb * m2);
+      const double v2 = __fma_rn(V.z, V.z, __fma_rn(V.y, V.y, V.x * V.x));
+      const double with = __fma_rn(v2 * nd, reciprocal(den), sum);
+      sum = directional && nd <= 0 ? sum : with;
     }
   }
   if (active) partial[((int64_t)p * S + s) * np + j] = sum;
@@ -363,69 +431,72 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 
 // ---------------------------------------------------------------- launchers
 
-static int flux_splits(int64_t n, int64_t nout, int nparticles) {
-  return choose_splits(((nout + kTile - 1) / kTile) * nparticles, n);
+static int64_t tiles_of(int64_t nout, int nparticles) { return (nout + kTile - 1) / kTile * nparticles; }
+static int64_t splits(int64_t n, int64_t chunk) { return (n + chunk - 1) / chunk; }
+static int64_t flux_chunk(int64_t n, int64_t np, int nparticles) {
+  return chunk_for(tiles_of(np, nparticles), n, wave_slots(flux_fp64_kernel, kTile));
+}
+static int64_t spectrum_chunk(int64_t n, int64_t ne, int nparticles) {
+  return chunk_for(tiles_of(ne, nparticles), n, wave_slots(spectrum_fp64_kernel, kTile));
+}
+static int64_t pd_chunk(int64_t n, int64_t np, int nparticles) {
+  return chunk_for(tiles_of(np, nparticles), n, wave_slots(pd_fp64_kernel, kTile));
 }
 
 size_t fp64_flux_scratch_bytes(int64_t n, int64_t np, int nparticles) {
-  return sizeof(double) * 6 * (size_t)np * nparticles * flux_splits(n, np, nparticles);
+  return sizeof(double) * 6 * (size_t)np * nparticles * splits(n, flux_chunk(n, np, nparticles));
 }
 
 cudaError_t fp64_flux(const srs_traj_view &t, const srs_beam_consts &b, const double *d_points, int64_t np,
                       double energy_ev, double *d_out, void *scratch, cudaStream_t s) {
   if (np <= 0 || t.nparticles <= 0) return cudaSuccess;
-  const int S = flux_splits(t.n, np, t.nparticles);
-  const int64_t chunk = (t.n + S - 1) / S;
+  const int64_t chunk = flux_chunk(t.n, np, t.nparticles);
+  const int S = (int)splits(t.n, chunk);
   const double omega = ev_to_omega(energy_ev);
   double *partial = static_cast<double *>(scratch);
   dim3 grid((unsigned)((np + kTile - 1) / kTile), S, t.nparticles);
-  flux_fp64_kernel<<<grid, kTile, 0, s>>>(t.x, t.beta, t.n, t.dt, d_points, np, omega, chunk, partial);
-  flux_fp64_reduce<<<blocks_for(np * t.nparticles, kRedPoints), 6 * kRedPoints, 0, s>>>(partial, S, np, t.nparticles, nullptr, omega,
-                                                                      t.dt, flux_c0(b.charge),
-                                                                      flux_c2(b.charge, b.current), d_out, nullptr);
-  return cudaGetLastError();
+  if (cudaError_t e = launch_after(flux_fp64_kernel, grid, dim3(kTile), 0, s, t.x, t.beta, t.n, t.dt, d_points, np,
+                                   omega, chunk, partial))
+    return e;
+  return finish_flux_partials(partial, S, np, t.nparticles, nullptr, omega, t.dt, flux_c0(b.charge),
+                              flux_c2(b.charge, b.current), d_out, s);
 }
 
 size_t fp64_spectrum_scratch_bytes(int64_t n, int64_t ne, int nparticles) {
-  return sizeof(double) * ((size_t)6 * ne * nparticles * flux_splits(n, ne, nparticles) + (size_t)ne);
+  return sizeof(double) * 6 * (size_t)ne * nparticles * splits(n, spectrum_chunk(n, ne, nparticles));
 }
 
 cudaError_t fp64_spectrum(const srs_traj_view &t, const srs_beam_consts &b, const double obs[3],
                           const double *d_energies, int64_t ne, double *d_out, void *scratch, cudaStream_t s,
                           double *d_e6) {
   if (ne <= 0 || t.nparticles <= 0) return cudaSuccess;
-  const int S = flux_splits(t.n, ne, t.nparticles);
-  const int64_t chunk = (t.n + S - 1) / S;
+  const int64_t chunk = spectrum_chunk(t.n, ne, t.nparticles);
+  const int S = (int)splits(t.n, chunk);
   double *partial = static_cast<double *>(scratch);
-  double *omegas = partial + (size_t)6 * ne * t.nparticles * S;
   dim3 grid((unsigned)((ne + kTile - 1) / kTile), S, t.nparticles);
-  spectrum_fp64_kernel<<<grid, kTile, 0, s>>>(t.x, t.beta, t.n, t.dt, v3(obs[0], obs[1], obs[2]), d_energies, ne,
-                                              chunk, partial);
-  omegas_kernel<<<blocks_for(ne, 256), 256, 0, s>>>(d_energies, ne, omegas);
-  flux_fp64_reduce<<<blocks_for(ne * t.nparticles, kRedPoints), 6 * kRedPoints, 0, s>>>(partial, S, ne, t.nparticles, omegas, 0.0,
-                                                                      t.dt, flux_c0(b.charge),
-                                                                      flux_c2(b.charge, b.current), d_out, d_e6);
-  return cudaGetLastError();
+  if (cudaError_t e = launch_after(spectrum_fp64_kernel, grid, dim3(kTile), 0, s, t.x, t.beta, t.n, t.dt,
+                                   v3(obs[0], obs[1], obs[2]), d_energies, ne, chunk, partial))
+    return e;
+  return finish_flux_partials(partial, S, ne, t.nparticles, nullptr, 0.0, t.dt, flux_c0(b.charge),
+                              flux_c2(b.charge, b.current), d_out, s, d_e6, d_energies);
 }
 
 size_t fp64_pd_scratch_bytes(int64_t n, int64_t np, int nparticles) {
-  return sizeof(double) * (size_t)np * nparticles * flux_splits(n, np, nparticles);
+  return sizeof(double) * (size_t)np * nparticles * splits(n, pd_chunk(n, np, nparticles));
 }
 
 cudaError_t fp64_power_density(const srs_traj_view &t, const srs_beam_consts &b, const double *d_points,
                                const double *d_normals, int64_t np, int directional, double *d_out, void *scratch,
                                cudaStream_t s) {
   if (np <= 0 || t.nparticles <= 0) return cudaSuccess;
-  const int S = flux_splits(t.n, np, t.nparticles);
-  const int64_t chunk = (t.n + S - 1) / S;
+  const int64_t chunk = pd_chunk(t.n, np, t.nparticles);
+  const int S = (int)splits(t.n, chunk);
   double *partial = static_cast<double *>(scratch);
   dim3 grid((unsigned)((np + kTile - 1) / kTile), S, t.nparticles);
-  pd_fp64_kernel<<<grid, kTile, 0, s>>>(t.x, t.beta, t.aoc, t.n, d_points, d_normals, np, directional, chunk,
-                                        partial);
-  const double cdt = pd_const(b.charge, b.current) * t.dt;
-  pd_fp64_reduce<<<blocks_for(np * t.nparticles, 256), 256, 0, s>>>(partial, S, np, t.nparticles, cdt, directional,
-                                                                    d_out);
-  return cudaGetLastError();
+  if (cudaError_t e = launch_after(pd_fp64_kernel, grid, dim3(kTile), 0, s, t.x, t.beta, t.aoc, t.n, d_points,
+                                   d_normals, np, directional, chunk, partial))
+    return e;
+  return finish_pd_partials(partial, S, np, t.nparticles, pd_const(b.charge, b.current) * t.dt, directional, d_out, s);
 }
 
 cudaError_t total_power(const srs_traj_view &t, const srs_beam_consts &b, const double *d_gamma, double *d_out,
@@ -438,10 +509,10 @@ cudaError_t total_power(const srs_traj_view &t, const srs_beam_consts &b, const 
 
 cudaError_t finish_flux_partials(const double *partial, int S, int64_t nout, int nparticles, const double *omegas,
                                  double omega0, double dt, double C0, double C2, double *out, cudaStream_t s,
-                                 double *e6) {
+                                 double *e6, const double *energies) {
   // set up while the sums that wrote the partials finish (the kernel waits for their writes)
   return launch_after(flux_fp64_reduce, dim3((unsigned)blocks_for(nout * nparticles, kRedPoints)),
-                      dim3(6 * kRedPoints), 0, s, partial, S, nout, nparticles, omegas, omega0, dt, C0, C2, out, e6);
+                      dim3(6 * kRedPoints), 0, s, partial, S, nout, nparticles, omegas, energies, omega0, dt, C0, C2, out, e6);
 }
 
 cudaError_t finish_pd_partials(const double *partial, int S, int64_t np, int nparticles, double cdt, int directional,

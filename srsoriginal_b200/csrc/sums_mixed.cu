@@ -371,7 +371,7 @@ __global__ void omega_kernel(const double *__restrict__ e, int64_t ne, double *_
 // ---------------------------------------------------------------- launchers
 
 static int flux_mixed_splits(int64_t n, const srs_grid2d &g, int nparticles) {
-  return splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(flux_mixed_kernel));
+  return splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(flux_mixed_kernel, kThreads));
 }
 
 size_t mixed_flux_scratch_bytes(int64_t n, const srs_grid2d &g, int nparticles) {
@@ -400,7 +400,7 @@ cudaError_t mixed_flux(const srs_traj_view &t, const srs_beam_consts &b, const s
 }
 
 static int flux_points_splits(int64_t n, int64_t np, int nparticles) {
-  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(flux_points_mixed_kernel));
+  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(flux_points_mixed_kernel, kThreads));
 }
 
 size_t mixed_flux_points_scratch_bytes(int64_t n, int64_t np, int nparticles) {
@@ -488,14 +488,14 @@ namespace srs {
 
 size_t mixed_pd_scratch_bytes(int64_t n, const srs_grid2d &g, int nparticles) {
   return sizeof(double) * (size_t)g.n1 * g.n2 * nparticles *
-         splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(pd_mixed_kernel));
+         splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(pd_mixed_kernel, kThreads));
 }
 
 cudaError_t mixed_power_density(const srs_traj_view &t, const srs_beam_consts &b, const srs_grid2d &g,
                                 int directional, double *d_out, void *scratch, cudaStream_t s) {
   const StripTiles m = strip_tiles(g);
   const int64_t chunk =
-      aligned_chunk(t.n, splits_for((int64_t)m.tiles * t.nparticles, t.n, 256, wave_slots(pd_mixed_kernel)));
+      aligned_chunk(t.n, splits_for((int64_t)m.tiles * t.nparticles, t.n, 256, wave_slots(pd_mixed_kernel, kThreads)));
   const int S = used_chunks(t.n, chunk);
   double *partial = static_cast<double *>(scratch);
   dim3 grid((unsigned)m.tiles, S, t.nparticles);
@@ -508,7 +508,7 @@ cudaError_t mixed_power_density(const srs_traj_view &t, const srs_beam_consts &b
 }
 
 static int pd_points_splits(int64_t n, int64_t np, int nparticles) {
-  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(pd_points_mixed_kernel));
+  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(pd_points_mixed_kernel, kThreads));
 }
 
 size_t mixed_pd_points_scratch_bytes(int64_t n, int64_t np, int nparticles) {
@@ -542,7 +542,7 @@ struct SpecPlan {
 };
 static SpecPlan spectrum_plan(int64_t n, int64_t ne, int nparticles) {
   constexpr int K4 = kEnergiesPerThread;
-  const int64_t slots4 = wave_slots(spectrum_mixed_kernel<K4>);
+  const int64_t slots4 = wave_slots(spectrum_mixed_kernel<K4>, kThreads);
   const int64_t e4 = (ne + kThreads * K4 - 1) / (kThreads * K4);
   SpecPlan P;
   if (e4 * nparticles * std::max<int64_t>(1, n / 256) >= slots4) {
@@ -552,7 +552,7 @@ static SpecPlan spectrum_plan(int64_t n, int64_t ne, int nparticles) {
   } else {
     P.K = 2;
     P.etiles = (ne + kThreads * 2 - 1) / (kThreads * 2);
-    P.S_max = splits_for(P.etiles * nparticles, n, (int64_t)kSub, wave_slots(spectrum_mixed_kernel<2>));
+    P.S_max = splits_for(P.etiles * nparticles, n, (int64_t)kSub, wave_slots(spectrum_mixed_kernel<2>, kThreads));
   }
   return P;
 }
