@@ -30,8 +30,6 @@
 // adds the S partials in chunk order (deterministic) and applies the reference's final scaling.
 #include <cuda_runtime.h>
 
-#include <cuda_pipeline.h>
-
 #include <algorithm>
 #include <cstdint>
 
@@ -170,51 +168,56 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
 }
 
 
-// Block of kRedPoints x 6 threads: thread (c, k) adds component c of point j = block * kRedPoints + k
-// over the S chunks in chunk order, then one thread per point applies the final scaling.  The loads of
-// kRedBatch chunks are issued together as asynchronous copies into the thread's own shared-memory
-// slots, so that a launch of a few thousand threads waits for memory once per kRedBatch chunks; the
-// adds stay in chunk order (config 0's spectrum: 53 chunks, 6000 threads).
-constexpr int kRedPoints = 32;
-constexpr int kRedBatch = 24;
-__global__ void __launch_bounds__(6 * kRedPoints) flux_fp64_reduce(const double *__restrict__ partial, int S,
-                                                                   int64_t np, int nparticles,
-                                                                   const double *__restrict__ omegas,
-                                                                   const double *__restrict__ energies, double omega0,
-                                                                   double dt, double C0, double C2,
-                                                                   double *__restrict__ out, double *__restrict__ e6) {
-  __shared__ double se[kRedPoints][7];
-  __shared__ double sbuf[kRedBatch][6 * kRedPoints];  // [chunk in batch][thread]
+// Adds the S per-chunk partials of every output and applies the final scaling.  A block holds P outputs x 6
+// components x G groups of consecutive chunks: thread (g, c, k) adds its group's chunks of component c of
+// output k in chunk order, eight loads in flight, then the groups are added in order (a fixed order).  The
+// time is the latency of a thread's batches of loads, so few outputs take more groups: 101 energies in
+// 626 chunks 28 -> 5 us, 1000 in 157 9 -> 5 us, against one thread per component.
+template <int P, int G>
+__global__ void __launch_bounds__(6 * P * G) flux_reduce_kernel(const double *__restrict__ partial, int S, int64_t np,
+                                                                int nparticles, const double *__restrict__ omegas,
+                                                                const double *__restrict__ energies, double omega0,
+                                                                double dt, double C0, double C2,
+                                                                double *__restrict__ out, double *__restrict__ e6) {
+  __shared__ double se[G][6][P];
   wait_for_previous_grid();  // (launched with launch_after by finish_flux_partials)
-  const int k = threadIdx.x % kRedPoints, c = threadIdx.x / kRedPoints;
-  const int64_t idx = (int64_t)blockIdx.x * kRedPoints + k;
+  const int k = threadIdx.x % P, c = threadIdx.x / P % 6, g = threadIdx.x / (6 * P);
+  const int64_t idx = (int64_t)blockIdx.x * P + k;
   const bool valid = idx < np * nparticles;
+  double e = 0;
   if (valid) {
-    const int64_t p = idx / np, j = idx % np;
-    const double *o = partial + (int64_t)p * S * 6 * np + c * np + j;
-    const int64_t stride = 6 * np;
-    double e = 0;
-    int s = 0;
-    double *const mine = &sbuf[0][threadIdx.x];
-    for (; s < S; s += kRedBatch, o += kRedBatch * stride) {
-      const int m = S - s < kRedBatch ? S - s : kRedBatch;
-      for (int u = 0; u < m; ++u) __pipeline_memcpy_async(mine + u * 6 * kRedPoints, o + u * stride, sizeof(double));
-      __pipeline_commit();
-      __pipeline_wait_prior(0);
-      for (int u = 0; u < m; ++u) e += mine[u * 6 * kRedPoints];
-    }
-    se[k][c] = e;
-  }
-  __syncthreads();
-  if (c == 0 && valid) {
-    double e[6];
+    const int64_t p = idx / np, j = idx % np, stride = 6 * np;
+    const int per = (S + G - 1) / G, s0 = g * per, s1 = min(S, s0 + per);
+    const double *o = partial + ((p * S + s0) * 6 + c) * np + j;
+    int s = s0;
+    for (; s + 8 <= s1; s += 8, o += 8 * stride) {
+      double v[8];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) e[q] = se[k][q];
+      for (int u = 0; u < 8; ++u) v[u] = o[u * stride];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) e += v[u];
+    }
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = s + u < s1 ? o[u * stride] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e += v[u];
+  }
+  se[g][c][k] = e;
+  __syncthreads();
+  if (threadIdx.x < P && valid) {
+    double t[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      t[q] = se[0][q][k];
+#pragma unroll
+      for (int u = 1; u < G; ++u) t[q] += se[u][q][k];
+    }
     const double omega = energies ? ev_to_omega(energies[idx % np]) : omegas ? omegas[idx % np] : omega0;
-    out[idx] = finish_flux(e, omega, dt, C0, C2);
+    out[idx] = finish_flux(t, omega, dt, C0, C2);
     if (e6) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) e6[6 * idx + q] = e[q];
+      for (int q = 0; q < 6; ++q) e6[6 * idx + q] = t[q];
     }
   }
 }
@@ -340,22 +343,34 @@ __global__ void __launch_bounds__(kTile) pd_fp64_kernel(const double *__restrict
   if (active) partial[((int64_t)p * S + s) * np + j] = sum;
 }
 
-__global__ void pd_fp64_reduce(const double *__restrict__ partial, int S, int64_t np, int nparticles, double cdt,
-                               int directional, double *__restrict__ out) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= np * nparticles) return;
-  const int64_t p = idx / np, j = idx % np;
+// The same for the power density: P outputs x G groups of chunks.
+template <int P, int G>
+__global__ void __launch_bounds__(P * G) pd_reduce_kernel(const double *__restrict__ partial, int S, int64_t np,
+                                                          int nparticles, double cdt, int directional,
+                                                          double *__restrict__ out) {
+  __shared__ double se[G][P];
+  wait_for_previous_grid();  // (launched with launch_after by finish_pd_partials)
+  const int k = threadIdx.x % P, g = threadIdx.x / P;
+  const int64_t idx = (int64_t)blockIdx.x * P + k;
+  const bool valid = idx < np * nparticles;
   double sum = 0;
-  const double *o = partial + (int64_t)p * S * np + j;
-  int s = 0;
-  for (; s + 8 <= S; s += 8, o += 8 * np) {  // chunk order, eight chunks' loads in flight at a time
-    double v[8];
+  if (valid) {
+    const int64_t p = idx / np, j = idx % np;
+    const int per = (S + G - 1) / G, s0 = g * per, s1 = min(S, s0 + per);
+    const double *o = partial + (p * S + s0) * np + j;
+    for (int s = s0; s < s1; s += 8, o += 8 * np) {
+      double v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = o[u * np];
+      for (int u = 0; u < 8; ++u) v[u] = s + u < s1 ? o[u * np] : 0.0;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) sum += v[u];
+      for (int u = 0; u < 8; ++u) sum += v[u];
+    }
   }
-  for (; s < S; ++s, o += np) sum += *o;
+  se[g][k] = sum;
+  __syncthreads();
+  if (g != 0 || !valid) return;
+#pragma unroll
+  for (int u = 1; u < G; ++u) sum += se[u][k];
   sum *= cdt;
   sum /= 1e6;
   if (!directional && sum < 0) sum *= -1;
@@ -364,19 +379,30 @@ __global__ void pd_fp64_reduce(const double *__restrict__ partial, int S, int64_
 
 // ---------------------------------------------------------------- total power and accumulation
 
-__global__ void total_power_kernel(const double *__restrict__ Bt, const double *__restrict__ A, int64_t n,
-                                   int nparticles, double dt, double qi, const double *__restrict__ gamma,
-                                   double *__restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nparticles) return;
+// One block per particle; the terms (which cancel to 1/gamma^2) in the reference's operation order, their
+// sum over points strided over the threads and then over the block in a fixed order (one thread per
+// particle took 1.3 ms for 12001 points, this 8 us).
+constexpr int kPowerThreads = 512;
+__global__ void __launch_bounds__(kPowerThreads) total_power_kernel(const double *__restrict__ Bt,
+                                                                    const double *__restrict__ A, int64_t n, double dt,
+                                                                    double qi, const double *__restrict__ gamma,
+                                                                    double *__restrict__ out) {
+  __shared__ double sum[kPowerThreads];
+  const int p = blockIdx.x, t = threadIdx.x;
   const double *bp = Bt + (int64_t)p * 3 * n, *ap = A + (int64_t)p * 3 * n;
   double tp = 0;
-  for (int64_t i = 0; i < n; ++i) {
+#pragma unroll 4
+  for (int64_t i = t; i < n; i += kPowerThreads) {
     V3 B = v3(bp[i], bp[n + i], bp[2 * n + i]), AC = v3(ap[i], ap[n + i], ap[2 * n + i]);
     tp += (mag2(AC) - mag2(cross(B, AC))) * dt;
   }
-  tp *= fabs(qi) * pow(gamma[p], 6.0) / (6 * kPi * kEps0 * kC);
-  out[p] = tp;
+  sum[t] = tp;
+  __syncthreads();
+  for (int w = kPowerThreads / 2; w > 0; w >>= 1) {
+    if (t < w) sum[t] += sum[t + w];
+    __syncthreads();
+  }
+  if (t == 0) out[p] = sum[0] * (fabs(qi) * pow(gamma[p], 6.0) / (6 * kPi * kEps0 * kC));
 }
 
 // The Lienard-Wiechert field of the trajectory point i at the observer and its arrival time
@@ -502,23 +528,33 @@ cudaError_t fp64_power_density(const srs_traj_view &t, const srs_beam_consts &b,
 cudaError_t total_power(const srs_traj_view &t, const srs_beam_consts &b, const double *d_gamma, double *d_out,
                         cudaStream_t s) {
   if (t.nparticles <= 0) return cudaSuccess;
-  total_power_kernel<<<blocks_for(t.nparticles, 64), 64, 0, s>>>(t.beta, t.aoc, t.n, t.nparticles, t.dt,
-                                                                  b.charge * b.current, d_gamma, d_out);
+  total_power_kernel<<<(unsigned)t.nparticles, kPowerThreads, 0, s>>>(t.beta, t.aoc, t.n, t.dt, b.charge * b.current,
+                                                                      d_gamma, d_out);
   return cudaGetLastError();
 }
 
 cudaError_t finish_flux_partials(const double *partial, int S, int64_t nout, int nparticles, const double *omegas,
                                  double omega0, double dt, double C0, double C2, double *out, cudaStream_t s,
                                  double *e6, const double *energies) {
-  // set up while the sums that wrote the partials finish (the kernel waits for their writes)
-  return launch_after(flux_fp64_reduce, dim3((unsigned)blocks_for(nout * nparticles, kRedPoints)),
-                      dim3(6 * kRedPoints), 0, s, partial, S, nout, nparticles, omegas, energies, omega0, dt, C0, C2, out, e6);
+  // set up while the sums that wrote the partials finish (the kernel waits for their writes).  Up to 2048
+  // outputs 16 groups of chunks, above 4: by then 32 outputs per block fill the GPU, and rows of 32
+  // doubles are read in full lines.
+  const int64_t total = nout * nparticles;
+  if (total <= 2048)
+    return launch_after(flux_reduce_kernel<8, 16>, dim3((unsigned)blocks_for(total, 8)), dim3(768), 0, s, partial, S,
+                        nout, nparticles, omegas, energies, omega0, dt, C0, C2, out, e6);
+  return launch_after(flux_reduce_kernel<32, 4>, dim3((unsigned)blocks_for(total, 32)), dim3(768), 0, s, partial, S,
+                      nout, nparticles, omegas, energies, omega0, dt, C0, C2, out, e6);
 }
 
 cudaError_t finish_pd_partials(const double *partial, int S, int64_t np, int nparticles, double cdt, int directional,
                                double *out, cudaStream_t s) {
-  pd_fp64_reduce<<<blocks_for(np * nparticles, 128), 128, 0, s>>>(partial, S, np, nparticles, cdt, directional, out);
-  return cudaGetLastError();
+  const int64_t total = np * nparticles;
+  if (total <= 4096)
+    return launch_after(pd_reduce_kernel<8, 32>, dim3((unsigned)blocks_for(total, 8)), dim3(256), 0, s, partial, S, np,
+                        nparticles, cdt, directional, out);
+  return launch_after(pd_reduce_kernel<32, 8>, dim3((unsigned)blocks_for(total, 32)), dim3(256), 0, s, partial, S, np,
+                      nparticles, cdt, directional, out);
 }
 
 cudaError_t accumulate_particles(const double *d_vals, int nparticles, int64_t nout, double weight, double *d_out,
