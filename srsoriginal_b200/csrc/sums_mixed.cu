@@ -371,7 +371,7 @@ __global__ void omega_kernel(const double *__restrict__ e, int64_t ne, double *_
 // ---------------------------------------------------------------- launchers
 
 static int flux_mixed_splits(int64_t n, const srs_grid2d &g, int nparticles) {
-  return splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(flux_mixed_kernel, kThreads));
+  return splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, kSub, wave_slots(flux_mixed_kernel, kThreads));
 }
 
 size_t mixed_flux_scratch_bytes(int64_t n, const srs_grid2d &g, int nparticles) {
@@ -400,7 +400,7 @@ cudaError_t mixed_flux(const srs_traj_view &t, const srs_beam_consts &b, const s
 }
 
 static int flux_points_splits(int64_t n, int64_t np, int nparticles) {
-  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(flux_points_mixed_kernel, kThreads));
+  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, kSub, wave_slots(flux_points_mixed_kernel, kThreads));
 }
 
 size_t mixed_flux_points_scratch_bytes(int64_t n, int64_t np, int nparticles) {
@@ -488,14 +488,14 @@ namespace srs {
 
 size_t mixed_pd_scratch_bytes(int64_t n, const srs_grid2d &g, int nparticles) {
   return sizeof(double) * (size_t)g.n1 * g.n2 * nparticles *
-         splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, 256, wave_slots(pd_mixed_kernel, kThreads));
+         splits_for((int64_t)strip_tiles(g).tiles * nparticles, n, kSub, wave_slots(pd_mixed_kernel, kThreads));
 }
 
 cudaError_t mixed_power_density(const srs_traj_view &t, const srs_beam_consts &b, const srs_grid2d &g,
                                 int directional, double *d_out, void *scratch, cudaStream_t s) {
   const StripTiles m = strip_tiles(g);
   const int64_t chunk =
-      aligned_chunk(t.n, splits_for((int64_t)m.tiles * t.nparticles, t.n, 256, wave_slots(pd_mixed_kernel, kThreads)));
+      aligned_chunk(t.n, splits_for((int64_t)m.tiles * t.nparticles, t.n, kSub, wave_slots(pd_mixed_kernel, kThreads)));
   const int S = used_chunks(t.n, chunk);
   double *partial = static_cast<double *>(scratch);
   dim3 grid((unsigned)m.tiles, S, t.nparticles);
@@ -508,7 +508,7 @@ cudaError_t mixed_power_density(const srs_traj_view &t, const srs_beam_consts &b
 }
 
 static int pd_points_splits(int64_t n, int64_t np, int nparticles) {
-  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, 256, wave_slots(pd_points_mixed_kernel, kThreads));
+  return splits_for((np + kThreads - 1) / kThreads * nparticles, n, kSub, wave_slots(pd_points_mixed_kernel, kThreads));
 }
 
 size_t mixed_pd_points_scratch_bytes(int64_t n, int64_t np, int nparticles) {
