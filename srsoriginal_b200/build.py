@@ -27,6 +27,7 @@ SOURCES = [
     ("rk4.cu", True),
     ("rk4_shoot.cu", True),
     ("rk4_exact.cu", True),
+    ("rk4_lanes.cu", True),
     ("sums_fp64.cu", True),
     ("sums_mixed.cu", False),
     ("queue.cu", False),

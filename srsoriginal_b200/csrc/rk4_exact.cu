@@ -28,15 +28,16 @@
 // trajectory, bit for bit.  Both chains of the trajectory (forward from t0, backward) and several
 // particles are integrated side by side.
 //
-// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.28 ms, 40001
-// through two 39.0 -> 0.69 ms, 12001 through a field map in two chains 14.1 -> 0.17 ms, 24 particles of
-// 10001 points 9.1 -> 0.68 ms, 300 points 0.28 -> 0.12 ms.  A pass is bound by latency (~8 us: launch,
+// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.25 ms, 40001
+// through two 39.0 -> 0.64 ms, 12001 through a field map in two chains 14.1 -> 0.17 ms, 24 particles of
+// 10001 points 9.1 -> 0.55 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by latency (~7 us: launch,
 // loads, four field evaluations, 2 x 128 additions in order), the chain by its 20001 additions (~0.1 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "rk4_fields.cuh"
+#include "rk4_und.cuh"
 #include "srs_internal.h"
 
 namespace srs {
@@ -82,6 +83,7 @@ struct Scratch {
   unsigned long long *bad;    // steps that do not reproduce (reset by the last block)
   int *failed;                // an item whose passes did not converge
   Prepared *prep;
+  UndField *und;
 };
 
 __device__ inline Item item_of(const Job &J, int it) {
@@ -117,15 +119,6 @@ __device__ inline Item item_of(const Job &J, int it) {
   return I;
 }
 
-// The quantities of one serial RK4 step that depend on the state only weakly (OSCARSSR.cc:826-874; the
-// operations and their order are those of rk4.cu): r1 = hh*a1, r2 = hh*a2, r3 = h*a3,
-// d = h6*(a1 + a4 + 2(a3 + a2)).
-struct Increments {
-  V3 r1, r2, r3, d, a1;
-};
-
-__device__ inline V3 scaled(double s, V3 a) { return v3(s * a.x, s * a.y, s * a.z); }
-
 // One copy of the field code: a step evaluates it four times, and a cold instruction cache costs a pass
 // more than the calls.
 __device__ __noinline__ V3 field_total(const Prepared *sp, const srs_field *sf, int nfields, V3 x) {
@@ -144,19 +137,21 @@ __device__ __forceinline__ void copy_fields(srs_field *sf, Prepared *sp, const s
   for (int k = threadIdx.x; k < nfields * (int)(sizeof(Prepared) / 8); k += blockDim.x) d[k] = b[k];
 }
 
+// The increments of one serial RK4 step that depend on the state only weakly (OSCARSSR.cc:826-874; the
+// operations and their order are those of rk4.cu): r1 = hh*a1, r2 = hh*a2, r3 = h*a3,
+// d = h6*(a1 + a4 + 2(a3 + a2)).
 __device__ __forceinline__ Increments increments(const Prepared *sp, const srs_field *sf, int nfields, double qomg,
-                                                 double h, V3 pos, V3 vel) {
+                                                 double h, double hh, double h6, V3 pos, V3 vel) {
   auto B = [&](V3 x) { return field_total(sp, sf, nfields, x); };
-  const double hh = h * 0.5, h6 = h / 6.0;
   Increments o;
   o.a1 = force(qomg, vel, B(pos));
-  o.r1 = scaled(hh, o.a1);
+  o.r1 = scale3(hh, o.a1);
   const V3 v2 = vel + o.r1;
   const V3 a2 = force(qomg, v2, B(vadd_scaled(pos, hh, vel)));
-  o.r2 = scaled(hh, a2);
+  o.r2 = scale3(hh, a2);
   const V3 v3_ = vel + o.r2;
   const V3 a3 = force(qomg, v3_, B(vadd_scaled(pos, hh, v2)));
-  o.r3 = scaled(h, a3);
+  o.r3 = scale3(h, a3);
   const V3 v4 = vel + o.r3;
   const V3 a4 = force(qomg, v4, B(vadd_scaled(pos, h, v3_)));
   const V3 m = a3 + a2;
@@ -164,11 +159,31 @@ __device__ __forceinline__ Increments increments(const Prepared *sp, const srs_f
   return o;
 }
 
-// the position increment of a component: h6*((v + v4) + 2(v3 + v2))
-__device__ __forceinline__ double advance(double h6, double v, double r1, double r2, double r3) {
-  const double v2 = v + r1, v3_ = v + r2, v4 = v + r3;
-  return h6 * (v + v4 + 2.0 * (v3_ + v2));
-}
+// The fields of a job as the blocks' threads evaluate them: kN undulators along z, or any list (kN = 0).
+template <int kN>
+struct Fields {
+  UndField und[kMaxUndulators];
+  __device__ __forceinline__ void load(const srs_field *, const Scratch &W, int) {
+    const long long *a = reinterpret_cast<const long long *>(W.und);
+    long long *b = reinterpret_cast<long long *>(und);
+    for (int k = threadIdx.x; k < kN * (int)(sizeof(UndField) / 8); k += blockDim.x) b[k] = a[k];
+  }
+  __device__ __forceinline__ Increments step(int, double qomg, double h, double hh, double h6, V3 pos, V3 vel) const {
+    return und_increments<kN>(und, qomg, h, hh, h6, pos, vel);
+  }
+};
+template <>
+struct Fields<0> {
+  srs_field sf[kMaxFieldsShared];
+  Prepared sp[kMaxFieldsShared];
+  __device__ __forceinline__ void load(const srs_field *gf, const Scratch &W, int nfields) {
+    copy_fields(sf, sp, gf, W.prep, nfields);
+  }
+  __device__ __forceinline__ Increments step(int nfields, double qomg, double h, double hh, double h6, V3 pos,
+                                             V3 vel) const {
+    return increments(sp, sf, nfields, qomg, h, hh, h6, pos, vel);
+  }
+};
 
 // o[j] = the running sum before d[j] is added, for n (a multiple of 16) rounded additions in order; returns
 // the sum.  The next sixteen terms are loaded while the current ones are added, so a step costs the
@@ -200,11 +215,12 @@ __device__ __forceinline__ double add_in_order(double acc, const double *__restr
   return acc;
 }
 
-__global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ fields, int nfields) {
+__global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ fields, int nfields, int undulators) {
   allow_next_grid();
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int items = J.nparticles * J.chains;
-  if (g < nfields) prepare(fields[g], W.prep[g]);
+  if (g < nfields && undulators) prepare_undulator(fields[g], W.und[g]);
+  else if (g < nfields) prepare(fields[g], W.prep[g]);
   if (g == 0) {
     *W.done = 0;
     *W.all_ticket = 0;
@@ -268,10 +284,10 @@ __device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I,
 }
 
 // Picard iteration number `pass` (see the file comment); in the first the states are straight flight.
+template <int kN>
 __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_field *__restrict__ gfields, int nfields,
                                                                   Job J, Scratch W, int pass) {
-  __shared__ srs_field sf[kMaxFieldsShared];
-  __shared__ Prepared sp[kMaxFieldsShared];
+  __shared__ Fields<kN> fields;
   __shared__ __align__(16) double sd[3][kStepsPerBlock], sv[3][kStepsPerBlock];
   __shared__ double red[6][kStepsPerBlock / 32];
   wait_for_previous_grid();
@@ -280,10 +296,10 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   const bool settled = W.ready[it] < pass || *W.failed;
   const Item I = item_of(J, it);
   const int64_t blk = (int64_t)it * J.maxblk + s, i = (int64_t)s * kStepsPerBlock + t;
-  copy_fields(sf, sp, gfields, W.prep, nfields);
+  fields.load(gfields, W, nfields);
   double *const S = W.S + (int64_t)it * 6 * J.stride;
   double *const T = W.T[pass & 1] + 6 * blk, *const E = W.E[pass & 1] + 6 * blk;
-  const double h = I.h, h6 = h / 6.0;
+  const double h = I.h, hh = h * 0.5, h6 = h / 6.0;
   const bool active = i < I.m;
   V3 vel = ld3(I.s0 + 3), pos = ld3(I.s0) + vel * (h * (double)i);
   if (pass > 0 && active) {
@@ -314,7 +330,7 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   __syncthreads();
   Increments o;
   o.d = v3(0, 0, 0);
-  if (active) o = increments(sp, sf, nfields, I.qomg, h, pos, vel);
+  if (active) o = fields.step(nfields, I.qomg, h, hh, h6, pos, vel);
   sd[0][t] = o.d.x;
   sd[1][t] = o.d.y;
   sd[2][t] = o.d.z;
@@ -341,17 +357,17 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
 
 // Every step's increments from the current states, the check, and the trajectory arrays (see the file
 // comment).  from_passes: the states still have to be moved by the last pass's shifts.
+template <int kN>
 __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_field *__restrict__ gfields, int nfields,
                                                                    Job J, Scratch W, int from_passes) {
-  __shared__ srs_field sf[kMaxFieldsShared];
-  __shared__ Prepared sp[kMaxFieldsShared];
+  __shared__ Fields<kN> fields;
   __shared__ double red[6][kStepsPerBlock / 32];
   wait_for_previous_grid();
   allow_next_grid();
   if (*W.done || *W.failed) return;
   const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
   const Item I = item_of(J, it);
-  copy_fields(sf, sp, gfields, W.prep, nfields);
+  fields.load(gfields, W, nfields);
   double shift[6];
   if (from_passes && s < I.nblk) {
     bool lost;  // the passes return at once after the one that found the item settled
@@ -380,7 +396,8 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
       vel = vel + dv;
       pos = pos + ld3(shift) + dv * (I.h * (double)t);
     }
-    const Increments o = increments(sp, sf, nfields, I.qomg, I.h, pos, vel);
+    const double hh = I.h * 0.5, h6 = I.h / 6.0;
+    const Increments o = fields.step(nfields, I.qomg, I.h, hh, h6, pos, vel);
     double *const R = W.R + (int64_t)it * 12 * J.stride + i;
     const V3 *const part[4] = {&o.r1, &o.r2, &o.r3, &o.d};
 #pragma unroll
@@ -394,7 +411,6 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
     } else {
       V3 np_, nv;
       state(i + 1, np_, nv);
-      const double h6 = I.h / 6.0;
       auto same = [](double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); };
       bad = !(same(nv.x, vel.x + o.d.x) && same(nv.y, vel.y + o.d.y) && same(nv.z, vel.z + o.d.z) &&
               same(np_.x, pos.x + advance(h6, vel.x, o.r1.x, o.r2.x, o.r3.x)) &&
@@ -536,6 +552,7 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
   s.failed = (int *)take(sizeof(int));
   s.bad = (unsigned long long *)take(sizeof(unsigned long long));
   s.prep = (Prepared *)take(sizeof(Prepared) * (size_t)std::max(1, nfields));
+  s.und = (UndField *)take(sizeof(UndField) * kMaxUndulators);
   if (W) *W = s;
   return off;
 }
@@ -543,10 +560,11 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
 }  // namespace
 
 // When the parallel iteration is used: trajectories long enough to pay for its ~30 launches, and few
-// enough of them (the serial kernels integrate up to 592 particles in the time of one, while this one
-// costs ~2.4 ns per step and particle).
+// enough of them: it costs ~1.7 ns per step and particle, the serial kernels 0.78 us (rk4_lanes.cu) or
+// 0.87 us (rk4.cu) per step of up to 592 particles and more, so they meet near 500 particles; its 144
+// bytes of scratch per step and particle (0.7 GB for 256 of 20001 points) end it before.
 constexpr int64_t kExactMinSteps = 256;
-constexpr int kExactMaxParticles = 128;
+constexpr int kExactMaxParticles = 256;
 // And only where the iteration contracts: the angle by which the fields could turn a particle over the
 // whole trajectory, |q/(m gamma)| sum |B| T (grids not counted: their samples are on the device).  3 GeV
 // electrons in 1 T over 2 m: 0.2; at 12 (50 MeV) the passes diverge, which costs 0.1-0.2 ms before the
@@ -561,6 +579,21 @@ static double turn_bound(const srs_field *fields, int nfields, const srs_particl
   return q * b * time;
 }
 
+template <int kN>
+static cudaError_t launch_exact(const Job &J, const Scratch &W, const srs_field *d_fields, int nfields, dim3 grid,
+                                cudaStream_t s) {
+  const dim3 block(kStepsPerBlock);
+  for (int k = 0; k < kPasses; ++k)
+    if (cudaError_t e = launch_after(pit_pass_kernel<kN>, grid, block, 0, s, d_fields, nfields, J, W, k)) return e;
+  for (int k = 0; k <= kSweeps; ++k) {
+    if (cudaError_t e = launch_after(pit_steps_kernel<kN>, grid, block, 0, s, d_fields, nfields, J, W, k == 0 ? 1 : 0))
+      return e;
+    if (k == kSweeps) break;
+    if (cudaError_t e = launch_after(pit_chain_kernel, dim3(grid.y), dim3(kChainThreads), 0, s, J, W)) return e;
+  }
+  return cudaGetLastError();
+}
+
 cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                                 double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
                                 const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,
@@ -569,18 +602,22 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
   const int64_t stage_doubles = nfields > 0 ? grid_stage_doubles(host_fields, nfields) : 0;
   const bool electric = has_electric(host_fields, nfields);
-  auto serial = [&](const int *d_skip) {
-    return launch_rk4(d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles,
-                      electric, d_specs, d_skip);
-  };
-  const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
-  const int64_t items = (int64_t)nparticles * J.chains;
-  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles)
-    return serial(nullptr);
   double time = dt * (double)(nfwd + nbwd);
   if (host_specs)
     for (int p = 0; p < nparticles; ++p)
       time = std::max(time, host_specs[p].dt * (double)(host_specs[p].nfwd + host_specs[p].nbwd));
+  const int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time);
+  const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
+  if (undulators && nparticles > kExactMaxParticles)
+    return launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x, d_b, d_a,
+                            d_specs, s);
+  auto serial = [&](const int *d_skip) {
+    return launch_rk4(d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles,
+                      electric, d_specs, d_skip);
+  };
+  const int64_t items = (int64_t)nparticles * J.chains;
+  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles)
+    return serial(nullptr);
   if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) < kExactMaxTurn)) return serial(nullptr);
   DeviceBuffer scratch;
   if (scratch.alloc(carve(J, nfields, nullptr, nullptr), s) != cudaSuccess) {
@@ -589,17 +626,13 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   }
   Scratch W;
   carve(J, nfields, scratch.ptr, &W);
-  const dim3 grid((unsigned)std::max(1, J.maxblk), (unsigned)items), block(kStepsPerBlock);
+  const dim3 grid((unsigned)std::max(1, J.maxblk), (unsigned)items);
   const int64_t init = std::max<int64_t>(items * std::max(1, J.maxblk), nfields);
-  pit_init_kernel<<<(unsigned)((init + 127) / 128), 128, 0, s>>>(J, W, d_fields, nfields);
-  for (int k = 0; k < kPasses; ++k)
-    if (cudaError_t e = launch_after(pit_pass_kernel, grid, block, 0, s, d_fields, nfields, J, W, k)) return e;
-  for (int k = 0; k <= kSweeps; ++k) {
-    if (cudaError_t e = launch_after(pit_steps_kernel, grid, block, 0, s, d_fields, nfields, J, W, k == 0 ? 1 : 0))
-      return e;
-    if (k == kSweeps) break;
-    if (cudaError_t e = launch_after(pit_chain_kernel, dim3((unsigned)items), dim3(kChainThreads), 0, s, J, W)) return e;
-  }
+  pit_init_kernel<<<(unsigned)((init + 127) / 128), 128, 0, s>>>(J, W, d_fields, nfields, undulators);
+  const cudaError_t e = undulators == 1   ? launch_exact<1>(J, W, d_fields, nfields, grid, s)
+                        : undulators == 2 ? launch_exact<2>(J, W, d_fields, nfields, grid, s)
+                                          : launch_exact<0>(J, W, d_fields, nfields, grid, s);
+  if (e != cudaSuccess) return e;
   if (cudaError_t e = cudaGetLastError()) return e;
   return serial(W.done);  // returns at once when the check held
 }

@@ -114,8 +114,17 @@ cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particl
                        double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
                        cudaStream_t s, int64_t stage_doubles, bool electric = false, const TrajSpec *d_specs = nullptr,
                        const int *d_skip = nullptr);
-// The same trajectories bit for bit, parallel in time where that is faster (rk4_exact.cu); host_*: the
-// host copies of the device arrays.
+// The number of fields if all are undulators that rk4_und.cuh integrates (at most two, period along +z, no
+// taper, phases of the given particles below 1e5 rad over the time [s]), else 0.
+int undulators_along_z(const srs_field *host_fields, int nfields, const srs_particle *host_particles, int nparticles,
+                       double time);
+// Trajectories of many particles through them, bit for bit launch_rk4's; chains: 2 when some particle has points before t0.
+cudaError_t launch_rk4_lanes(int undulators, const srs_field *d_fields, int nfields, const srs_particle *d_particles,
+                             int nparticles, int chains, double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b,
+                             double *d_a, const TrajSpec *d_specs, cudaStream_t s);
+// launch_rk4's trajectories bit for bit by the fastest way: few particles parallel in time (rk4_exact.cu),
+// many through undulators one per lane (rk4_lanes.cu), the rest launch_rk4.  host_*: the host copies of the
+// device arrays.
 cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                                 double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
                                 const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,

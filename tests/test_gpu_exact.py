@@ -1,6 +1,7 @@
-"""The parallel-in-time integration of the serial trajectory (srs_trajectory of few particles): every
-point equals the serial kernel's bit for bit.  The serial kernel is reached by integrating more than
-128 copies of the particle at once."""
+"""The trajectory kernels of few and of many particles against the serial one, bit for bit: few are
+integrated parallel in time, many through undulators along z take one lane each.  The serial kernel is
+reached by integrating more than 256 particles at once with a field of no amplitude added to the list
+(x + 0 is exact)."""
 import math
 
 import numpy as np
@@ -8,7 +9,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-MANY = 129
+MANY = 257
 
 
 def _fields(name):
@@ -22,11 +23,14 @@ def _fields(name):
         f.field, f.center, f.sigma_or_width, f.rotations = _lib.v3(b), _lib.v3(c), _lib.v3(s), _lib.v3(rot)
         return f
 
+    if name == "nothing":
+        return [shape(_lib.GAUSSIAN, (0, 0, 0), (0, 0, 0), (0, 0, 1.0))], None
     und = D.undulator([0, 1.0, 0], [0, 0, 0.049], 31)
     if name == "undulator":
         return [und], None
-    if name == "epu":
-        return [und, D.undulator([0.6, 0, 0], [0, 0, 0.049], 31, phase=math.pi / 2, taper=0.01)], None
+    if name in ("epu", "taper"):
+        return [und, D.undulator([0.6, 0, 0], [0, 0, 0.049], 31, phase=math.pi / 2,
+                                 taper=0.01 if name == "taper" else 0.0)], None
     if name == "none":
         return [], None
     if name == "grid":
@@ -46,7 +50,7 @@ def _fields(name):
     ("undulator", 257, 3.0, 0.0), ("undulator", 258, 3.0, 0.0), ("undulator", 385, 3.0, 0.0),
     ("undulator", 512, 3.0, 0.0), ("undulator", 513, 3.0, 0.0), ("undulator", 20001, 2.997, 0.0),
     ("undulator", 4097, 3.0, -1.0), ("undulator", 3001, 0.05, 0.0), ("undulator", 16641, 0.5, 0.0),
-    ("epu", 9999, 3.0, 0.0), ("epu", 40001, 3.0, 0.0), ("grid", 2049, 3.0, -1.0), ("none", 1025, 3.0, 0.0),
+    ("taper", 9999, 3.0, 0.0), ("epu", 40001, 3.0, 0.0), ("grid", 2049, 3.0, -1.0), ("none", 1025, 3.0, 0.0),
     ("mixed", 5003, 3.0, -0.7),
 ])
 def test_single_trajectory_equals_the_serial_kernel_bitwise(field, npoints, energy, start):
@@ -58,7 +62,7 @@ def test_single_trajectory_equals_the_serial_kernel_bitwise(field, npoints, ener
     x0 = [1e-5, -2e-5, -1.0 if start == 0.0 else 0.0]
     part, _ = D.ideal_particle(energy, x0, [3e-6, -5e-6, 1])
     one = D.trajectory(fields, [part], start, start + 2.0, 0.0, npoints)
-    many = D.trajectory(fields, [part] * MANY, start, start + 2.0, 0.0, npoints)
+    many = D.trajectory(fields + _fields("nothing")[0], [part] * MANY, start, start + 2.0, 0.0, npoints)
     torch.cuda.synchronize()
     for a in ("x", "beta", "aoc"):
         assert torch.equal(getattr(one, a)[0], getattr(many, a)[MANY - 1]), a
@@ -74,7 +78,30 @@ def test_few_particles_together_equal_the_serial_kernel_bitwise():
     parts = [D.ideal_particle(3.0 * (1 + 1e-3 * rng.normal()), [3e-5 * rng.normal(), 1e-5 * rng.normal(), 0.0],
                               [2e-5 * rng.normal(), 1e-5 * rng.normal(), 1])[0] for _ in range(7)]
     few = D.trajectory(fields, parts, -1.0, 1.0, 0.0, 3001)
-    many = D.trajectory(fields, parts * 19, -1.0, 1.0, 0.0, 3001)
+    many = D.trajectory(fields + _fields("nothing")[0], parts * 37, -1.0, 1.0, 0.0, 3001)
     torch.cuda.synchronize()
     for a in ("x", "beta", "aoc"):
         assert torch.equal(getattr(few, a), getattr(many, a)[:7]), a
+
+
+# Sizes at the edges of the lane kernel: one, two and four particles per warp, the two chains, a last
+# block that is not full.
+@pytest.mark.parametrize("field,particles,npoints,start", [
+    ("undulator", 257, 2, 0.0), ("undulator", 257, 5001, 0.0), ("undulator", 601, 1025, -1.0),
+    ("epu", 1303, 2050, 0.0), ("undulator", 300, 401, 0.0), ("epu", 2500, 333, -1.0),
+])
+def test_many_particles_equal_the_serial_kernel_bitwise(field, particles, npoints, start):
+    import torch
+
+    from srsoriginal_b200 import device as D
+
+    fields, _ = _fields(field)
+    rng = np.random.default_rng(particles)
+    z0 = -1.0 if start == 0.0 else 0.0
+    parts = [D.ideal_particle(3.0 * (1 + 1e-3 * rng.normal()), [3e-5 * rng.normal(), 1e-5 * rng.normal(), z0],
+                              [2e-5 * rng.normal(), 1e-5 * rng.normal(), 1])[0] for _ in range(particles)]
+    got = D.trajectory(fields, parts, start, start + 2.0, 0.0, npoints)
+    ref = D.trajectory(fields + _fields("nothing")[0], parts, start, start + 2.0, 0.0, npoints)
+    torch.cuda.synchronize()
+    for a in ("x", "beta", "aoc"):
+        assert torch.equal(getattr(got, a), getattr(ref, a)), a
