@@ -406,7 +406,7 @@ class sr:  # noqa: N801  (the reference's type name)
                     f.write(f"{a:.6e} {b:.6e}\n")
         if bofile:
             np.column_stack([e, flux]).astype(np.float64).tofile(bofile)
-        return [[float(a), float(b)] for a, b in zip(e, flux)]
+        return [[a, b] for a, b in zip(e.tolist(), flux.tolist())]
 
     def spectrum_arrays(self, obs, npoints=0, energy_range_eV=None, points_eV=None, nparticles=0, nthreads=0,
                         gpu=0, precision=None):
@@ -515,6 +515,9 @@ class sr:  # noqa: N801  (the reference's type name)
         rot = _list3(rotations, "rotations") if rotations is not None and len(rotations) != 0 else [0.0, 0.0, 0.0]
         tr = _list3(translation, "translation") if translation is not None and len(translation) != 0 \
             else [0.0, 0.0, 0.0]
+        fast = sr._surface_arrays(points, rot, tr, invert_normal)
+        if fast is not None:
+            return fast
         xs, ns = [], []
         for item in points:
             if not hasattr(item, "__len__") or len(item) != 2:
@@ -532,6 +535,27 @@ class sr:  # noqa: N801  (the reference's type name)
             xs.append([X[0] + tr[0], X[1] + tr[1], X[2] + tr[2]])
             ns.append([N[0] / m, N[1] / m, N[2] / m])
         return np.array(xs, dtype=np.float64).reshape(-1, 3), np.array(ns, dtype=np.float64).reshape(-1, 3)
+
+    @staticmethod
+    def _surface_arrays(points, rot, tr, invert_normal):
+        """The same for a regular list of N pairs of three numbers, operation by operation on arrays (2347
+        points: 6.3 -> 1.1 ms); None for anything else, which the loop accepts or refuses item by item."""
+        try:
+            a = np.asarray(points)
+        except (TypeError, ValueError):
+            return None
+        if a.ndim != 3 or a.shape[0] < 1 or a.shape[1:] != (2, 3) or a.dtype.kind not in "fiub":
+            return None
+        a = a.astype(np.float64)
+        with np.errstate(all="ignore"):
+            x = np.column_stack(sr._rotate_xyz(a[:, 0].T, rot))
+            n = np.column_stack(sr._rotate_xyz(a[:, 1].T, rot))
+            if invert_normal:
+                n = -n
+            m = np.sqrt(n[:, 0] * n[:, 0] + n[:, 1] * n[:, 1] + n[:, 2] * n[:, 2])
+            if not m.all():
+                return None  # a normal of no length: the loop's division error
+            return x + np.array(tr), n / m[:, None]
 
     def _point_list(self, xyz, out, nparticles, nthreads, gpu, pd):
         """The reference's list for a point surface (dim = 3): the points, then the zero entries its
@@ -562,7 +586,7 @@ class sr:  # noqa: N801  (the reference's type name)
         C_, V = self._point_list(xyz, out, nparticles, nthreads, gpu, pd=False)
         if ofile:
             self._write_points(ofile, C_, V, 3)
-        return [[c, float(v)] for c, v in zip(C_.tolist(), V)]
+        return [[c, v] for c, v in zip(C_.tolist(), V.tolist())]
 
     def calculate_power_density(self, points, normal=0, rotations=None, translation=None, nparticles=0, gpu=0,
                                 nthreads=0, ofile="", precision=None):
@@ -586,7 +610,7 @@ class sr:  # noqa: N801  (the reference's type name)
         C_, V = self._point_list(xyz, out, nparticles, nthreads, gpu, pd=True)
         if ofile:
             self._write_points(ofile, C_, V, 3)
-        return [[c, float(v)] for c, v in zip(C_.tolist(), V)]
+        return [[c, v] for c, v in zip(C_.tolist(), V.tolist())]
 
     # ------------------------------------------------------------ flux
     def calculate_flux_rectangle(self, energy_eV, npoints, plane="", normal=0, dim=2, width=None, rotations=None,
@@ -626,7 +650,7 @@ class sr:  # noqa: N801  (the reference's type name)
         V = np.concatenate(vals)
         if ofile:
             self._write_points(ofile, C_, V, dim)
-        return [[c, float(v)] for c, v in zip(C_.tolist(), V)]
+        return [[c, v] for c, v in zip(C_.tolist(), V.tolist())]
 
     def flux_arrays(self, energy_eV, npoints, plane="", width=None, rotations=None, translation=None, x0x1x2=None,
                     nparticles=0, precision=None, normal=0):
@@ -693,7 +717,7 @@ class sr:  # noqa: N801  (the reference's type name)
         V = np.concatenate(vals)
         if ofile:
             self._write_points(ofile, C_, V, dim)
-        return [[c, float(v)] for c, v in zip(C_.tolist(), V)]
+        return [[c, v] for c, v in zip(C_.tolist(), V.tolist())]
 
     def power_density_arrays(self, npoints, plane="", width=None, rotations=None, translation=None, x0x1x2=None,
                              normal=0, nparticles=0, precision=None, weighted=False):
