@@ -23,15 +23,28 @@
 //                      tile, the other warps feeding them): one rounded addition, 8 cycles, per step
 //                      where the serial kernel needs ~1700.
 //
-// Steps and chain alternate until the check holds; the serial kernel runs if it never does (slow
+// On long chains (kRunsMinSteps) those additions are spread over the GPU too.  While the sum stays in one
+// binade, a rounded addition v + d is the exact addition of d rounded to that binade's grid, whatever v is
+// (ties aside), so a run of such steps is one exact addend.  The blocks, which know v nearly, find the runs
+// and leave a list of addends (run totals, and the d of the steps in between: a change of binade, a tie):
+// 2750 for the x of 20000 steps through an undulator, 625 (one per warp) for y and z.
+//
+//   pit_starts_kernel  adds a component's list in order, which gives every block's start state;
+//   pit_positions_kernel  re-adds the velocities of the blocks from there and lists the positions' runs;
+//   then the lists of the positions, and pit_steps_kernel re-adds those.
+//
+// The lists need no proof: a wrong one (the state known too badly) fails the check and costs a sweep.
+//
+// Steps and chains alternate until the check holds; the serial kernel runs if it never does (slow
 // particles in strong fields, where the iteration does not contract): the result is always the serial
 // trajectory, bit for bit.  Both chains of the trajectory (forward from t0, backward) and several
 // particles are integrated side by side.
 //
-// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.25 ms, 40001
-// through two 39.0 -> 0.64 ms, 12001 through a field map in two chains 14.1 -> 0.17 ms, 24 particles of
-// 10001 points 9.1 -> 0.55 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by latency (~7 us: launch,
-// loads, four field evaluations, 2 x 128 additions in order), the chain by its 20001 additions (~0.1 ms).
+// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.17 ms, 40001
+// through two 39.0 -> 0.35 ms, 12001 through a field map in two chains 14.1 -> 0.16 ms, 24 particles of
+// 10001 points 9.1 -> 0.56 ms, 2001 points 1.78 -> 0.13 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by
+// latency (~7 us: launch, loads, four field evaluations, 2 x 128 additions in order); a sweep takes 0.16 ms
+// by the chain kernel on 20001 points, 0.05 ms by runs (20 us per list, 10 us per kernel of blocks).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -46,9 +59,16 @@ namespace {
 constexpr int kStepsPerBlock = 128;  // steps (and threads) of a pass block
 constexpr int kChainTile = 256;      // steps per tile of the chain kernel
 constexpr int kChainThreads = 512;
+constexpr int kGroup = 12;           // blocks whose addends the starts kernel holds at a time, one feeding warp each
+constexpr int kStartsThreads = 32 * (kGroup + 1);
 constexpr int kPasses = 14;          // passes launched (they return at once when the item is ready)
 constexpr int kContracted = 4;       // by this pass a contracting iteration is far below 1e-4 of the speed
 constexpr int kSweeps = 4;           // exact sweeps before the serial kernel takes over
+// Chains by runs from this length: a sweep of the chain kernel takes 7.8 ns per step of the longest chain
+// (1 or 24 particles alike), one by runs ~40 us, 1.5 ns per step and ~20 ns per block of all particles.
+// Measured, chain kernel -> runs: 2001 points 128 -> 140 us, 2 x 6000 162 -> 149, 20001 253 -> 172, 40001
+// 645 -> 344, 24 particles of 20001 1102 -> 1031, of 10001 556 -> 575, 100 of 20001 3380 -> 3930.
+constexpr int64_t kRunsMinSteps = 4500, kRunsStepsPerBlock = 3;
 
 // One chain of one particle.
 struct Item {
@@ -72,12 +92,16 @@ struct Job {
   int nparticles, chains;  // chains per particle (2 when some particle has points before t0)
   int64_t stride;          // doubles per component of an item's states
   int maxblk;              // pass blocks of the longest chain
+  bool by_runs;            // the chains' additions by runs (kRunsMinSteps)
 };
 
 struct Scratch {
   double *S;      // [item][6][stride]: states
-  double *R;      // [item][12][stride]: increments hh*a1, hh*a2, h*a3, d (three components each)
-  double *T[2], *E[2];        // [item][maxblk][6]: start state of a block, state after its last step (pass k: k & 1)
+  double *R;      // [item][12][stride]: increments hh*a1, hh*a2, h*a3, d or those of the positions (3 components each)
+  double *L;      // [item][3][maxblk][kStepsPerBlock]: addends of a component's chain, block by block
+  int *count;     // [item][3][maxblk]: addends of a block
+  double *T[2], *E[2];        // [item][maxblk][6]: start state of a block, state after its last step (pass k: k & 1);
+                              // T[0] after the passes: the start states that the chains give
   int *ready;                 // per item: the pass that found nothing left to settle, or kPasses
   int *done, *all_ticket;     // the whole job verified; blocks of the steps kernel finished
   unsigned long long *bad;    // steps that do not reproduce (reset by the last block)
@@ -185,10 +209,10 @@ struct Fields<0> {
   }
 };
 
-// o[j] = the running sum before d[j] is added, for n (a multiple of 16) rounded additions in order; returns
+// o[j] (which may be d[j]) = the running sum before d[j] is added, for n (a multiple of 16) rounded additions in order; returns
 // the sum.  The next sixteen terms are loaded while the current ones are added, so a step costs the
 // latency of its addition; a 16-byte access covers two steps.
-__device__ __forceinline__ double add_in_order(double acc, const double *__restrict__ d, double *__restrict__ o, int n) {
+__device__ __forceinline__ double add_in_order(double acc, const double *d, double *o, int n) {
   double2 nx[8];
   const double2 *const d2 = reinterpret_cast<const double2 *>(d);
   double2 *const o2 = reinterpret_cast<double2 *>(o);
@@ -213,6 +237,71 @@ __device__ __forceinline__ double add_in_order(double acc, const double *__restr
     }
   }
   return acc;
+}
+
+// Whether the rounded addition a + d is the exact addition of r, for every a' in place of a that differs by
+// less than tol: a' and a' + d lie in one binade, so the sum is rounded on that binade's grid, which a' is
+// on (a tie goes to the even neighbour, which depends on a').
+__device__ __forceinline__ bool exact_addend(double a, double d, double tol, double &r) {
+  const double s = a + d;
+  r = s - a;
+  if (d == 0.0) {
+    r = d;
+    return true;
+  }
+  const double lo = __longlong_as_double(__double_as_longlong(a) & 0x7ff0000000000000ll), hi = 2.0 * lo;
+  const bool same_sign = (__double_as_longlong(a) ^ __double_as_longlong(s)) >= 0;
+  return same_sign && fabs(a) >= lo + tol && fabs(a) <= hi - tol && fabs(s) >= lo + tol && fabs(s) <= hi - tol &&
+         fabs(d - r) != lo * 0x1p-53;
+}
+
+// The addends of a block's additions a + d: a run of steps whose additions are exact on one grid is one
+// addend, their sum (exact in any order: the partial sums are differences of numbers of one binade).
+__device__ __forceinline__ void emit_addends(const Job &J, const Scratch &W, int it, int s, bool active, V3 a, V3 d,
+                                             double tol, int (*counts)[3]) {
+  constexpr int kWarps = kStepsPerBlock / 32;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const double av[3] = {a.x, a.y, a.z}, dv[3] = {d.x, d.y, d.z};
+  double val[3];
+  unsigned heads[3];
+  int first[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    double r;
+    const bool run = !active || exact_addend(av[c], dv[c], tol, r);
+    val[c] = !active ? -0.0 : run ? r : dv[c];  // x + -0.0 is x for every x
+    const unsigned runs = __ballot_sync(0xffffffffu, run);
+    heads[c] = ~(runs & (runs << 1));  // a step that no run continues into
+    first[c] = 31 - __clz(heads[c] & (0xffffffffu >> (31 - lane)));
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double y = __shfl_up_sync(0xffffffffu, val[c], o);
+      if (lane - o >= first[c]) val[c] += y;
+    }
+  if (lane < 3) counts[warp][lane] = __popc(lane == 0 ? heads[0] : lane == 1 ? heads[1] : heads[2]);
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int64_t row = ((int64_t)it * 3 + c) * J.maxblk + s;
+    int at = 0, all = 0;
+    for (int w = 0; w < kWarps; ++w) {
+      if (w < warp) at += counts[w][c];
+      all += counts[w][c];
+    }
+    if (t == 0) W.count[row] = all;
+    if (lane == 31 || (heads[c] >> (lane + 1) & 1))
+      W.L[row * kStepsPerBlock + at + __popc(heads[c] & (0xffffffffu >> (31 - lane))) - 1] = val[c];
+  }
+}
+
+// Bounds on the distance of an approximate state from the exact one, as exact_addend takes them: a wrong
+// one costs a sweep, the check decides.
+__device__ __forceinline__ double speed_tolerance(const Item &I) { return 0x1p-43 * sqrt(mag2(ld3(I.s0 + 3))); }
+__device__ __forceinline__ double position_tolerance(const Item &I) {
+  return speed_tolerance(I) * fabs(I.h) * (double)I.m;
 }
 
 __global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ fields, int nfields, int undulators) {
@@ -293,7 +382,9 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   wait_for_previous_grid();
   allow_next_grid();
   const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
-  const bool settled = W.ready[it] < pass || *W.failed;
+  // as the passes before this one left it (in this pass other blocks may be writing ready = pass - 1, and all
+  // threads of a block have to decide alike)
+  const bool settled = W.ready[it] + 1 < pass;
   const Item I = item_of(J, it);
   const int64_t blk = (int64_t)it * J.maxblk + s, i = (int64_t)s * kStepsPerBlock + t;
   fields.load(gfields, W, nfields);
@@ -314,7 +405,7 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
     bool lost;
     const bool ready = mismatches(J, W, I, it, s, pass - 1, red, shift, &lost);
     if (lost && pass > kContracted) {
-      if (t == 0) *W.failed = 1;
+      if (t == 0) W.ready[it] = pass - 1, *W.failed = 1;
       return;
     }
     if (ready) {
@@ -355,27 +446,52 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   }
 }
 
-// Every step's increments from the current states, the check, and the trajectory arrays (see the file
-// comment).  from_passes: the states still have to be moved by the last pass's shifts.
-template <int kN>
+// Every step's increments from the current states, the check, the trajectory arrays, and the addends of the
+// velocities' chain (see the file comment).  from_passes: the states are the last pass's and still have
+// to be moved by its shifts; otherwise the positions follow from their chain and their increments.
+template <int kN, bool kRuns>
 __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_field *__restrict__ gfields, int nfields,
                                                                    Job J, Scratch W, int from_passes) {
   __shared__ Fields<kN> fields;
+  __shared__ __align__(16) double sd[3][kRuns ? kStepsPerBlock : 2], sx[3][kRuns ? kStepsPerBlock + 2 : 2];
   __shared__ double red[6][kStepsPerBlock / 32];
+  __shared__ int counts[kStepsPerBlock / 32][3];
   wait_for_previous_grid();
   allow_next_grid();
   if (*W.done || *W.failed) return;
   const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
   const Item I = item_of(J, it);
   fields.load(gfields, W, nfields);
-  double shift[6];
-  if (from_passes && s < I.nblk) {
-    bool lost;  // the passes return at once after the one that found the item settled
-    mismatches(J, W, I, it, s, min(W.ready[it], kPasses - 1), red, shift, &lost);
+  const int64_t i = (int64_t)s * kStepsPerBlock + t;
+  double *const S = W.S + (int64_t)it * 6 * J.stride, *const R = W.R + (int64_t)it * 12 * J.stride + i;
+  V3 pos = v3(0, 0, 0), vel = v3(0, 0, 0), nv = v3(0, 0, 0);
+  if (i < I.m) {
+    vel = v3(S[3 * J.stride + i], S[4 * J.stride + i], S[5 * J.stride + i]);
+    if (from_passes || !kRuns) pos = v3(S[i], S[J.stride + i], S[2 * J.stride + i]);
+    if (kRuns && !from_passes) nv = v3(S[3 * J.stride + i + 1], S[4 * J.stride + i + 1], S[5 * J.stride + i + 1]);
+  }
+  if (s < I.nblk) {
+    if (from_passes) {
+      double shift[6];
+      bool lost;  // the passes return at once after the one that found the item settled
+      mismatches(J, W, I, it, s, min(W.ready[it], kPasses - 1), red, shift, &lost);
+      const V3 dv = ld3(shift + 3);
+      vel = vel + dv;
+      pos = pos + ld3(shift) + dv * (I.h * (double)t);
+    } else if constexpr (kRuns) {
+      const double *const at = W.T[0] + 6 * ((int64_t)it * J.maxblk + s);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) sd[c][t] = i < I.m ? R[(9 + c) * J.stride] : 0.0;
+      __syncthreads();
+      if (t < 3) {
+        const double end = add_in_order(at[t], sd[t], sx[t], kStepsPerBlock);
+        sx[t][kStepsPerBlock] = s + 1 < I.nblk ? at[6 + t] : end;
+      }
+      __syncthreads();
+      pos = v3(sx[0][t], sx[1][t], sx[2][t]);
+    }
   }
   __syncthreads();
-  const int64_t i = (int64_t)s * kStepsPerBlock + t;
-  const double *const S = W.S + (int64_t)it * 6 * J.stride;
   const double rC = 1.0 / kC;
   auto store = [&](int64_t k, V3 p, V3 v, V3 a) {
     I.x[k] = p.x; I.x[I.n + k] = p.y; I.x[2 * I.n + k] = p.z;
@@ -384,21 +500,16 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
   };
   int bad = 0;
   if (i == 0 && I.dir > 0 && I.n > I.first) store(I.first, ld3(I.s0), ld3(I.s0 + 3), v3(0, 0, 0));
+  Increments o;
+  o.d = v3(0, 0, 0);
   if (i < I.m) {
-    auto state = [&](int64_t k, V3 &p, V3 &v) {
-      p = v3(S[k], S[J.stride + k], S[2 * J.stride + k]);
-      v = v3(S[3 * J.stride + k], S[4 * J.stride + k], S[5 * J.stride + k]);
-    };
-    V3 pos, vel;
-    state(i, pos, vel);
-    if (from_passes) {
-      const V3 dv = ld3(shift + 3);
-      vel = vel + dv;
-      pos = pos + ld3(shift) + dv * (I.h * (double)t);
+    if (kRuns) {
+      S[i] = pos.x;
+      S[J.stride + i] = pos.y;
+      S[2 * J.stride + i] = pos.z;
     }
     const double hh = I.h * 0.5, h6 = I.h / 6.0;
-    const Increments o = fields.step(nfields, I.qomg, I.h, hh, h6, pos, vel);
-    double *const R = W.R + (int64_t)it * 12 * J.stride + i;
+    o = fields.step(nfields, I.qomg, I.h, hh, h6, pos, vel);
     const V3 *const part[4] = {&o.r1, &o.r2, &o.r3, &o.d};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -409,8 +520,9 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
     if (from_passes) {
       bad = 1;  // moved by approximate shifts: to be re-added in order first
     } else {
-      V3 np_, nv;
-      state(i + 1, np_, nv);
+      if (!kRuns) nv = v3(S[3 * J.stride + i + 1], S[4 * J.stride + i + 1], S[5 * J.stride + i + 1]);
+      const V3 np_ = kRuns ? v3(sx[0][t + 1], sx[1][t + 1], sx[2][t + 1])
+                               : v3(S[i + 1], S[J.stride + i + 1], S[2 * J.stride + i + 1]);
       auto same = [](double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); };
       bad = !(same(nv.x, vel.x + o.d.x) && same(nv.y, vel.y + o.d.y) && same(nv.z, vel.z + o.d.z) &&
               same(np_.x, pos.x + advance(h6, vel.x, o.r1.x, o.r2.x, o.r3.x)) &&
@@ -419,6 +531,8 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
       store(I.first + I.dir * (I.dir > 0 ? i + 1 : i), np_, nv, o.a1);
     }
   }
+  if constexpr (kRuns)
+    if (s < I.nblk) emit_addends(J, W, it, s, i < I.m, vel, o.d, speed_tolerance(I), counts);
   bad = __syncthreads_count(bad);
   if (t == 0) {
     if (bad) atomicAdd(W.bad, (unsigned long long)bad);
@@ -504,6 +618,111 @@ __global__ void __launch_bounds__(kChainThreads) pit_chain_kernel(Job J, Scratch
   }
 }
 
+// The start states of the blocks: the additions of one component of an item's velocities (first = 3) or
+// positions (first = 0) in order.  The last warp adds (one lane), the others feed it: warp w gathers the addends of
+// block w of a group and writes its start state when the group is added.
+__global__ void __launch_bounds__(kStartsThreads) pit_starts_kernel(Job J, Scratch W, int first) {
+  __shared__ __align__(16) double a[3][kGroup * kStepsPerBlock + 16];
+  __shared__ int total[3];
+  wait_for_previous_grid();
+  allow_next_grid();
+  if (*W.done || *W.failed) return;
+  const int it = blockIdx.y, c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Item I = item_of(J, it);
+  const int groups = (I.nblk + kGroup - 1) / kGroup;
+  const int64_t row = ((int64_t)it * 3 + c) * J.maxblk;
+  double acc = I.s0[first + c];
+  int cn = 0, off[3] = {0, 0, 0};  // counts of a group's blocks; this warp's first addend in the last three groups
+  double val[kStepsPerBlock / 32];
+  auto counts = [&](int k) { return lane < kGroup && k * kGroup + lane < I.nblk ? W.count[row + k * kGroup + lane] : 0; };
+  auto fetch = [&](int k, int n) {  // the n addends of this warp's block of group k
+    const double *const L = W.L + (row + (int64_t)k * kGroup + warp) * kStepsPerBlock;
+#pragma unroll
+    for (int q = 0; q < kStepsPerBlock / 32; ++q) val[q] = lane + 32 * q < n ? L[lane + 32 * q] : 0.0;
+  };
+  const bool feeds = warp < kGroup;
+  int next = 0;
+  if (feeds) {
+    cn = counts(0);
+    next = counts(1);
+    fetch(0, __shfl_sync(0xffffffffu, cn, warp));
+  }
+  for (int k = 0; k < groups + 2; ++k) {  // group k is gathered, group k - 1 added, group k - 2 written
+    if (feeds) {
+      int sum = cn;
+#pragma unroll
+      for (int o = 1; o < kGroup; o *= 2) {
+        const int y = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += y;
+      }
+      const int n = __shfl_sync(0xffffffffu, cn, warp), all = __shfl_sync(0xffffffffu, sum, kGroup - 1);
+      off[2] = off[1];
+      off[1] = off[0];
+      off[0] = __shfl_sync(0xffffffffu, sum, warp) - n;
+      if (k < groups) {
+#pragma unroll
+        for (int q = 0; q < kStepsPerBlock / 32; ++q)
+          if (lane + 32 * q < n) a[k % 3][off[0] + lane + 32 * q] = val[q];
+        if (warp == 0 && lane < 16) a[k % 3][all + lane] = -0.0;  // (adds nothing)
+        if (warp == 0 && lane == 0) total[k % 3] = all;
+      }
+      cn = next;
+      fetch(k + 1, __shfl_sync(0xffffffffu, cn, warp));
+      next = counts(k + 2);
+      const int b = (k - 2) * kGroup + warp;
+      if (k >= 2 && b < I.nblk && lane == 0) W.T[0][6 * ((int64_t)it * J.maxblk + b) + first + c] = a[(k - 2) % 3][off[2]];
+    } else if (k >= 1 && k <= groups && lane == 0) {
+      acc = add_in_order(acc, a[(k - 1) % 3], a[(k - 1) % 3], (total[(k - 1) % 3] + 15) / 16 * 16);
+    }
+    __syncthreads();
+  }
+}
+
+// The velocities from their blocks' start states, the increments of the positions, and the addends of
+// the positions' chain.
+__global__ void __launch_bounds__(kStepsPerBlock) pit_positions_kernel(Job J, Scratch W) {
+  __shared__ __align__(16) double sd[3][kStepsPerBlock], sv[3][kStepsPerBlock];
+  __shared__ int counts[kStepsPerBlock / 32][3];
+  wait_for_previous_grid();
+  allow_next_grid();
+  if (*W.done || *W.failed) return;
+  const int it = blockIdx.y, s = blockIdx.x, t = threadIdx.x;
+  const Item I = item_of(J, it);
+  if (s >= I.nblk) return;
+  const int64_t i = (int64_t)s * kStepsPerBlock + t;
+  const bool active = i < I.m;
+  double *const S = W.S + (int64_t)it * 6 * J.stride + i, *const R = W.R + (int64_t)it * 12 * J.stride + i;
+  V3 r[4], pos = v3(0, 0, 0);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    r[q] = active ? v3(R[3 * q * J.stride], R[(3 * q + 1) * J.stride], R[(3 * q + 2) * J.stride]) : v3(0, 0, 0);
+  if (active) pos = v3(S[0], S[J.stride], S[2 * J.stride]);
+  sd[0][t] = r[3].x;
+  sd[1][t] = r[3].y;
+  sd[2][t] = r[3].z;
+  __syncthreads();
+  if (t < 3) {
+    const double end = add_in_order(W.T[0][6 * ((int64_t)it * J.maxblk + s) + 3 + t], sd[t], sv[t], kStepsPerBlock);
+    if ((int64_t)(s + 1) * kStepsPerBlock == I.m) W.S[((int64_t)it * 6 + 3 + t) * J.stride + I.m] = end;
+  }
+  __syncthreads();
+  const V3 vel = v3(sv[0][t], sv[1][t], sv[2][t]);
+  if (i <= I.m) {
+    S[3 * J.stride] = vel.x;
+    S[4 * J.stride] = vel.y;
+    S[5 * J.stride] = vel.z;
+  }
+  const double h6 = I.h / 6.0;
+  const V3 d = v3(advance(h6, vel.x, r[0].x, r[1].x, r[2].x), advance(h6, vel.y, r[0].y, r[1].y, r[2].y),
+                  advance(h6, vel.z, r[0].z, r[1].z, r[2].z));
+  if (active) {
+    R[9 * J.stride] = d.x;
+    R[10 * J.stride] = d.y;
+    R[11 * J.stride] = d.z;
+  }
+  emit_addends(J, W, it, s, active, pos, d, position_tolerance(I), counts);
+}
+
 Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const TrajSpec *h_specs, int nparticles, double dt,
              int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a) {
   Job J;
@@ -528,6 +747,7 @@ Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const Tra
   const int64_t m = std::max<int64_t>(std::max(mf, mb), 0);
   J.stride = (m + 2) / 2 * 2;
   J.maxblk = (int)((m + kStepsPerBlock - 1) / kStepsPerBlock);
+  J.by_runs = m >= kRunsMinSteps + kRunsStepsPerBlock * J.nparticles * J.chains * J.maxblk;
   return J;
 }
 
@@ -542,6 +762,8 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
   Scratch s;
   s.S = (double *)take(sizeof(double) * 6 * items * J.stride);
   s.R = (double *)take(sizeof(double) * 12 * items * J.stride);
+  s.L = (double *)take(J.by_runs ? sizeof(double) * 3 * blocks * kStepsPerBlock : 0);
+  s.count = (int *)take(J.by_runs ? sizeof(int) * 3 * blocks : 0);
   for (int k = 0; k < 2; ++k) {
     s.T[k] = (double *)take(sizeof(double) * 6 * blocks);
     s.E[k] = (double *)take(sizeof(double) * 6 * blocks);
@@ -562,7 +784,7 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
 // When the parallel iteration is used: trajectories long enough to pay for its ~30 launches, and few
 // enough of them: it costs ~1.7 ns per step and particle, the serial kernels 0.78 us (rk4_lanes.cu) or
 // 0.87 us (rk4.cu) per step of up to 592 particles and more, so they meet near 500 particles; its 144
-// bytes of scratch per step and particle (0.7 GB for 256 of 20001 points) end it before.
+// bytes of scratch per step and particle (0.7 GB for 256 of 20001 points; 168 by runs) end it before.
 constexpr int64_t kExactMinSteps = 256;
 constexpr int kExactMaxParticles = 256;
 // And only where the iteration contracts: the angle by which the fields could turn a particle over the
@@ -585,11 +807,18 @@ static cudaError_t launch_exact(const Job &J, const Scratch &W, const srs_field 
   const dim3 block(kStepsPerBlock);
   for (int k = 0; k < kPasses; ++k)
     if (cudaError_t e = launch_after(pit_pass_kernel<kN>, grid, block, 0, s, d_fields, nfields, J, W, k)) return e;
+  const auto steps = J.by_runs ? pit_steps_kernel<kN, true> : pit_steps_kernel<kN, false>;
+  const dim3 starts(3, grid.y), starts_threads(kStartsThreads);
   for (int k = 0; k <= kSweeps; ++k) {
-    if (cudaError_t e = launch_after(pit_steps_kernel<kN>, grid, block, 0, s, d_fields, nfields, J, W, k == 0 ? 1 : 0))
-      return e;
+    if (cudaError_t e = launch_after(steps, grid, block, 0, s, d_fields, nfields, J, W, k == 0 ? 1 : 0)) return e;
     if (k == kSweeps) break;
-    if (cudaError_t e = launch_after(pit_chain_kernel, dim3(grid.y), dim3(kChainThreads), 0, s, J, W)) return e;
+    if (!J.by_runs) {
+      if (cudaError_t e = launch_after(pit_chain_kernel, dim3(grid.y), dim3(kChainThreads), 0, s, J, W)) return e;
+      continue;
+    }
+    if (cudaError_t e = launch_after(pit_starts_kernel, starts, starts_threads, 0, s, J, W, 3)) return e;
+    if (cudaError_t e = launch_after(pit_positions_kernel, grid, block, 0, s, J, W)) return e;
+    if (cudaError_t e = launch_after(pit_starts_kernel, starts, starts_threads, 0, s, J, W, 0)) return e;
   }
   return cudaGetLastError();
 }

@@ -84,6 +84,30 @@ def test_few_particles_together_equal_the_serial_kernel_bitwise():
         assert torch.equal(getattr(few, a), getattr(many, a)[:7]), a
 
 
+# Chains added by runs (from 4500 steps and 3 per block of 128): the first length that is, a full last block and
+# one step in it, full groups of 12 blocks and one block more, two particles whose positions cross many
+# binades (x0 = 0), several particles in two chains.
+@pytest.mark.parametrize("field,particles,npoints,start", [
+    ("undulator", 1, 4608, 0.0), ("undulator", 1, 4609, 0.0), ("undulator", 1, 4612, 0.0), ("epu", 1, 4738, 0.0),
+    ("undulator", 2, 6145, 0.0), ("undulator", 4, 12001, -1.0), ("mixed", 2, 12289, -0.5), ("none", 1, 6001, 0.0),
+    ("grid", 1, 18434, -1.0),
+])
+def test_chains_by_runs_equal_the_serial_kernel_bitwise(field, particles, npoints, start):
+    import torch
+
+    from srsoriginal_b200 import device as D
+
+    fields, keep = _fields(field)
+    rng = np.random.default_rng(npoints)
+    parts = [D.ideal_particle(3.0 - 0.3 * i, [1e-6 * i * rng.normal(), 0.0, -1.0 if start == 0.0 else 0.0],
+                              [3e-6 * i * rng.normal(), 1e-6 * i, 1])[0] for i in range(particles)]
+    few = D.trajectory(fields, parts, start, start + 2.0, 0.0, npoints)
+    many = D.trajectory(fields + _fields("nothing")[0], parts * MANY, start, start + 2.0, 0.0, npoints)
+    torch.cuda.synchronize()
+    for a in ("x", "beta", "aoc"):
+        assert torch.equal(getattr(few, a), getattr(many, a)[:particles]), a
+
+
 # Sizes at the edges of the lane kernel: one, two and four particles per warp, the two chains, a last
 # block that is not full.
 @pytest.mark.parametrize("field,particles,npoints,start", [
