@@ -539,7 +539,7 @@ class sr:  # noqa: N801  (the reference's type name)
     @staticmethod
     def _surface_arrays(points, rot, tr, invert_normal):
         """The same for a regular list of N pairs of three numbers, operation by operation on arrays (2347
-        points: 6.3 -> 1.1 ms); None for anything else, which the loop accepts or refuses item by item."""
+        points: 4.6 -> 1.0 ms); None for anything else, which the loop accepts or refuses item by item."""
         try:
             a = np.asarray(points)
         except (TypeError, ValueError):
