@@ -12,15 +12,14 @@
 //    the Jacobian of RK4 step j.  Instead of one serial sweep back through the N steps (the forward
 //    RK4 is a serial chain; its adjoint need not be), the affine recurrence is solved as a scan:
 //      (a) every step's 6 x 6 Jacobian is formed in parallel from the stored states, by forward-mode
-//          tangents pushed through the four stages (step_jacobian_kernel);
-//      (b) chunks of kAdjChunk steps are composed into one affine map lambda_j0 = M lambda_j1 + b
-//          (chunk_compose_kernel);
-//      (c) one warp carries lambda across the chunk maps from the last point back to the first
+//          tangents pushed through the four stages, and chunks of kAdjChunk steps, then the kAdjBlock steps of a block, are composed there into
+//          affine maps lambda_j0 = M lambda_j1 + b (step_maps_kernel);
+//      (b) one warp carries lambda across the block maps from the last point back to the first
 //          (carry_kernel);
-//      (d) each chunk re-walks its steps backwards from its known end value, running the
-//          reverse-mode step (VJP through the four stages, recomputed from the stored state) that
-//          yields both lambda_j and the field-parameter and q/(m gamma) contributions
-//          (chunk_finish_kernel).
+//      (c) each block carries its end value across its chunks and, chunk by chunk, across the steps with
+//          the stored Jacobians; then all steps run the reverse-mode step from their own lambda at once
+//          (VJP through the four stages, recomputed from the stored state), which yields the
+//          field-parameter and q/(m gamma) contributions (finish_kernel).
 //    The stored trajectory is itself the checkpoint set: the state at every step is in HBM (the sums
 //    need every point anyway), so each step's stages are recomputed from its own stored state and
 //    no sqrt(N) re-integration is needed.  The reverse pass does not re-run the forward integration.
@@ -31,8 +30,6 @@
 // arithmetic is FP64.  Grid-sample gradients are accumulated with FP64 atomics (sub-ulp
 // run-to-run differences); everything else is reduced in a fixed order.
 #include <cuda_runtime.h>
-
-#include <cuda_pipeline.h>
 
 #include <algorithm>
 #include <cstring>
@@ -46,6 +43,8 @@ namespace srs {
 namespace {
 
 constexpr int kAdjChunk = 16;     // steps per scan chunk
+constexpr int kAdjBlock = 128;    // steps (and threads) per block
+constexpr int kAdjChunks = kAdjBlock / kAdjChunk;
 constexpr int kAdjMaxFields = 16;
 
 __device__ inline void rot_matrix(const double r[3], double R[3][3]) {
@@ -320,15 +319,15 @@ struct Chain {
   double h;          // step
   int64_t base;      // stored index of state 0
   int dir;           // stored index of state j: base + dir * j
-  int64_t nch;       // chunks
-  int64_t chunk_off; // first global chunk index
+  int64_t nblk;      // blocks
+  int64_t blk_off;   // first global block index
   int64_t step_off;  // first global step index (Jacobian storage)
   int skip_g0;       // state 0's g belongs to the other chain
 };
 struct Chains {
   Chain c[2];
   int n;
-  int64_t total_chunks, total_steps;
+  int64_t total_blocks;
 };
 
 struct Traj {
@@ -353,184 +352,237 @@ __device__ inline void load_g(const Traj &T, const Chain &ch, int64_t j, double 
   }
 }
 
-__device__ inline int find_chain(const Chains &C, int64_t gidx, bool steps) {
-  return (C.n > 1 && gidx >= (steps ? C.c[1].step_off : C.c[1].chunk_off)) ? 1 : 0;
-}
+__device__ inline int find_chain(const Chains &C, int64_t block) { return C.n > 1 && block >= C.c[1].blk_off ? 1 : 0; }
 
-// (a) J~_j (6 x 6, row = output, column = input, in (x, beta) units) of every step.
-__global__ void __launch_bounds__(128) step_jacobian_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
-                                                            Chains C, double *__restrict__ jac) {
-  __shared__ srs_field F[kAdjMaxFields];
-  for (int i = threadIdx.x; i < nf; i += blockDim.x) F[i] = gF[i];
+// A block's Jacobians in shared memory: step t's 36 entries from jac_at(t).  The odd stride and the extra
+// double per chunk keep both the threads' own steps and the chunks' same steps on different banks.
+__device__ __forceinline__ int jac_at(int t) { return 37 * t + t / kAdjChunk; }
+constexpr int kJacDoubles = 37 * kAdjBlock + kAdjChunks;
+
+// (a) J~_j (6 x 6, row = output, column = input, in (x, beta) units) of every step, and the maps of the
+// block's chunks and of the block, composed backwards from M = I, b = 0: eight lanes per chunk, one per
+// column of M and one for b.  Bound by the latency of the four stages and six tangents of a step with one
+// warp per scheduler: 20001 points (157 blocks) 40 us, where the Jacobians (36 us) and then the maps of
+// the chunks by one thread each (41 us) took two kernels.
+__global__ void __launch_bounds__(kAdjBlock) step_maps_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
+                                                              Chains C, double *__restrict__ jac,
+                                                              double *__restrict__ chunk_maps,
+                                                              double *__restrict__ block_maps) {
+  __shared__ double sJ[kJacDoubles];
+  __shared__ union {
+    srs_field F[kAdjMaxFields];
+    struct {
+      double g[kAdjBlock][6], map[kAdjChunks][42];
+    };
+  } sh;
+  const int t = threadIdx.x;
+  for (int i = t; i < nf; i += kAdjBlock) sh.F[i] = gF[i];
   __syncthreads();
-  const int64_t gs = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gs >= C.total_steps) return;
-  const Chain &ch = C.c[find_chain(C, gs, true)];
-  const int64_t j = gs - ch.step_off;
-  V3 pos, vel;
-  load_state(T, ch.base + ch.dir * j, pos, vel);
-  Stages S;
-  make_stages(F, nf, q, pos, vel, ch.h, S);
-  double *Jo = jac + 36 * gs;
-  for (int col = 0; col < 6; ++col) {
-    V3 dp = v3(0, 0, 0), dv = v3(0, 0, 0);
-    if (col < 3) dp = v3(col == 0, col == 1, col == 2);
-    else dv = v3(col == 3, col == 4, col == 5) * kC;
-    V3 op, ov;
-    step_jvp(S, q, ch.h, dp, dv, 0.0, op, ov);
-    const double out[6] = {op.x, op.y, op.z, ov.x / kC, ov.y / kC, ov.z / kC};
-    for (int r = 0; r < 6; ++r) Jo[6 * r + col] = out[r];
+  const Chain &ch = C.c[find_chain(C, blockIdx.x)];
+  const int64_t j0 = (blockIdx.x - ch.blk_off) * kAdjBlock;
+  const int cnt = (int)imin64(kAdjBlock, ch.L - 1 - j0);
+  if (t < cnt) {
+    V3 pos, vel;
+    load_state(T, ch.base + ch.dir * (j0 + t), pos, vel);
+    Stages S;
+    make_stages(sh.F, nf, q, pos, vel, ch.h, S);
+    double *const Jo = sJ + jac_at(t);
+    for (int col = 0; col < 6; ++col) {
+      V3 dp = v3(0, 0, 0), dv = v3(0, 0, 0);
+      if (col < 3) dp = v3(col == 0, col == 1, col == 2);
+      else dv = v3(col == 3, col == 4, col == 5) * kC;
+      V3 op, ov;
+      step_jvp(S, q, ch.h, dp, dv, 0.0, op, ov);
+      const double out[6] = {op.x, op.y, op.z, ov.x / kC, ov.y / kC, ov.z / kC};
+      for (int r = 0; r < 6; ++r) Jo[6 * r + col] = out[r];
+    }
   }
-}
-
-// (b) per chunk [j0, j1): lambda_j0 = M lambda_j1 + b, composed backwards from M = I, b = 0.
-__global__ void chunk_compose_kernel(Traj T, Chains C, const double *__restrict__ jac, double *__restrict__ Mb) {
-  const int64_t gc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gc >= C.total_chunks) return;
-  const Chain &ch = C.c[find_chain(C, gc, false)];
-  const int64_t c = gc - ch.chunk_off;
-  const int64_t j0 = c * kAdjChunk, j1 = imin64(j0 + kAdjChunk, ch.L - 1);
-  double M[6][6], b[6];
-  for (int r = 0; r < 6; ++r) {
-    b[r] = 0.0;
-    for (int k = 0; k < 6; ++k) M[r][k] = r == k;
-  }
-  for (int64_t j = j1 - 1; j >= j0; --j) {
-    const double *Jj = jac + 36 * (ch.step_off + j);
-    double A[6][6];  // A = J^T
-    for (int r = 0; r < 6; ++r)
-      for (int k = 0; k < 6; ++k) A[r][k] = Jj[6 * k + r];
+  __syncthreads();
+  if (t < cnt) {
     double g[6];
-    load_g(T, ch, j, g);
-    double nb[6], nM[6][6];
-    for (int r = 0; r < 6; ++r) {
-      double s = g[r];
-      for (int k = 0; k < 6; ++k) s += A[r][k] * b[k];
-      nb[r] = s;
-      for (int col = 0; col < 6; ++col) {
-        double t = 0.0;
-        for (int k = 0; k < 6; ++k) t += A[r][k] * M[k][col];
-        nM[r][col] = t;
-      }
-    }
-    for (int r = 0; r < 6; ++r) {
-      b[r] = nb[r];
-      for (int col = 0; col < 6; ++col) M[r][col] = nM[r][col];
-    }
+    load_g(T, ch, j0 + t, g);
+    for (int r = 0; r < 6; ++r) sh.g[t][r] = g[r];
   }
-  double *o = Mb + 42 * gc;
-  for (int r = 0; r < 6; ++r) {
-    for (int col = 0; col < 6; ++col) o[6 * r + col] = M[r][col];
-    o[36 + r] = b[r];
+  for (int k = t; k < 36 * cnt; k += kAdjBlock) jac[36 * (ch.step_off + j0) + k] = sJ[jac_at(k / 36) + k % 36];
+  __syncthreads();
+  const int col = t % 8;
+  if (t < 8 * kAdjChunks && col < 7) {
+    const int c = t / 8;
+    double m[6];
+    for (int r = 0; r < 6; ++r) m[r] = r == col;
+    for (int j = min((c + 1) * kAdjChunk, cnt) - 1; j >= c * kAdjChunk; --j) {
+      const double *const J = sJ + jac_at(j);  // lambda_j = g_j + J^T lambda_{j+1}
+      double n[6];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        double s = col == 6 ? sh.g[j][r] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += J[6 * k + r] * m[k];
+        n[r] = s;
+      }
+#pragma unroll
+      for (int r = 0; r < 6; ++r) m[r] = n[r];
+    }
+    for (int r = 0; r < 6; ++r) sh.map[c][col < 6 ? 6 * r + col : 36 + r] = m[r];
+  }
+  __syncthreads();
+  for (int k = t; k < 42 * kAdjChunks; k += kAdjBlock) chunk_maps[42 * kAdjChunks * (int64_t)blockIdx.x + k] = sh.map[k / 42][k % 42];
+  if (t < 7) {
+    double m[6];
+    for (int r = 0; r < 6; ++r) m[r] = r == t;
+    for (int c = kAdjChunks - 1; c >= 0; --c) {  // (a chunk past the end is the identity)
+      const double *const o = sh.map[c];
+      double n[6];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        double s = t == 6 ? o[36 + r] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += o[6 * r + k] * m[k];
+        n[r] = s;
+      }
+#pragma unroll
+      for (int r = 0; r < 6; ++r) m[r] = n[r];
+    }
+    for (int r = 0; r < 6; ++r) block_maps[42 * (int64_t)blockIdx.x + (t < 6 ? 6 * r + t : 36 + r)] = m[r];
   }
 }
 
-// (c) one warp per chain, lanes 0..5 own one component: lambda at every chunk start.  The sweep is
-// sequential over the chunks, so the chunk maps come through shared memory in tiles of kCarryTile,
-// the next tile's asynchronous copies in flight while the current one is swept (a step then waits on
-// shared memory, not on a global load: 1250 chunks of config 4 took 0.63 ms with the maps read from
-// global memory step by step).
-constexpr int kCarryTile = 64;  // chunk maps per tile: 64 x 42 doubles = 21.5 KB, two buffers
-__global__ void __launch_bounds__(32) carry_kernel(Traj T, Chains C, const double *__restrict__ Mb,
-                                                   double *__restrict__ lam0) {
-  __shared__ __align__(16) double tile[2][kCarryTile * 42];
-  const int chain = blockIdx.x;
-  if (chain >= C.n) return;
-  const Chain &ch = C.c[chain];
-  const int r = threadIdx.x;
+// b + M lambda for row r of an affine map, as a tree (depth 4 instead of a chain of six multiply-adds);
+// the six lanes from `first` hold lambda
+__device__ __forceinline__ double apply_row(const double m[6], double b, double lam, int first) {
+  double l[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) l[k] = __shfl_sync(0xffffffffu, lam, first + k);
+  return b + (((m[0] * l[0] + m[1] * l[1]) + (m[2] * l[2] + m[3] * l[3])) + (m[4] * l[4] + m[5] * l[5]));
+}
+
+// (b) one warp per chain, lanes 0..5 own one component: lambda at every block's end.  Sequential over the
+// blocks, the rows of the next maps loaded while one is applied: 37 us for the 157 maps of 20001 points (155
+// for the maps of 1250 chunks).
+__global__ void __launch_bounds__(32) carry_kernel(Traj T, Chains C, const double *__restrict__ block_maps,
+                                                   double *__restrict__ lam_end) {
+  const Chain &ch = C.c[blockIdx.x];
+  const int r = threadIdx.x, rr = r < 6 ? r : 0;
+  if (ch.nblk == 0) return;
   double g[6];
   load_g(T, ch, ch.L - 1, g);
-  double lam = r < 6 ? g[r] : 0.0;  // lambda_{L-1} = g_{L-1}
-  const int64_t nch = ch.nch, ntiles = (nch + kCarryTile - 1) / kCarryTile;
-  // tile t: chunks [lo(t), hi(t)], hi(t) = nch - 1 - t * kCarryTile, swept from hi down to lo
-  auto lo_of = [&](int64_t t) {
-    const int64_t hi = nch - 1 - t * kCarryTile;
-    return hi - kCarryTile + 1 > 0 ? hi - kCarryTile + 1 : (int64_t)0;
-  };
-  auto fetch = [&](int64_t t, int buf) {  // 16-byte copies: a chunk map is 21 of them, 16-byte aligned
-    const int64_t hi = nch - 1 - t * kCarryTile, lo = lo_of(t);
-    const double *src = Mb + 42 * (ch.chunk_off + lo);
-    const int n16 = (int)(hi - lo + 1) * 21;
-    for (int k = r; k < n16; k += 32) __pipeline_memcpy_async(&tile[buf][2 * k], src + 2 * k, 16);
-    __pipeline_commit();
-  };
-  if (ntiles > 0) fetch(0, 0);
-  for (int64_t t = 0; t < ntiles; ++t) {
-    const int buf = (int)(t & 1);
-    if (t + 1 < ntiles) fetch(t + 1, buf ^ 1);
-    else __pipeline_commit();  // an empty group, so that "all but the newest" is always tile t
-    __pipeline_wait_prior(1);
-    __syncwarp();
-    const int64_t hi = nch - 1 - t * kCarryTile, lo = lo_of(t);
-    const int rr = r < 6 ? r : 0;
-    for (int64_t c = hi; c >= lo; --c) {
-      const double *o = &tile[buf][42 * (c - lo)];
-      double l[6];
+  double lam = 0.0;  // lambda_{L-1} = g_{L-1}
 #pragma unroll
-      for (int k = 0; k < 6; ++k) l[k] = __shfl_sync(0xffffffffu, lam, k);
-      // b + M lambda as a tree (depth 4 instead of a chain of six multiply-adds: the sweep is a chain
-      // of these, one per chunk)
-      const double *m = o + 6 * rr;
-      const double p0 = m[0] * l[0], p1 = m[1] * l[1], p2 = m[2] * l[2], p3 = m[3] * l[3], p4 = m[4] * l[4],
-                   p5 = m[5] * l[5];
-      lam = o[36 + rr] + (((p0 + p1) + (p2 + p3)) + (p4 + p5));
-      if (r < 6) lam0[6 * (ch.chunk_off + c) + r] = lam;
+  for (int k = 0; k < 6; ++k)
+    if (r == k) lam = g[k];
+  constexpr int kAhead = 4;  // maps in flight
+  double m[kAhead][7];
+  auto load = [&](int64_t c, double *o) {
+    const double *const p = block_maps + 42 * (ch.blk_off + (c > 0 ? c : 0));
+#pragma unroll
+    for (int k = 0; k < 6; ++k) o[k] = p[6 * rr + k];
+    o[6] = p[36 + rr];
+  };
+#pragma unroll
+  for (int a = 0; a < kAhead; ++a) load(ch.nblk - 1 - a, m[a]);
+  for (int64_t c = ch.nblk - 1; c >= 0; c -= kAhead) {
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) {
+      if (c - a < 0) break;
+      if (r < 6) lam_end[6 * (ch.blk_off + c - a) + r] = lam;
+      lam = apply_row(m[a], m[a][6], lam, 0);
+      load(c - a - kAhead, m[a]);
     }
-    __syncwarp();  // every lane is done with this buffer before the next iteration refills it
   }
 }
 
-// (d) per chunk: walk back from lambda_j1 with the reverse-mode step; field-parameter and q
-// contributions go to per-chunk partials (amplitudes, q) or atomics (grid samples).
-__global__ void __launch_bounds__(64) chunk_finish_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
-                                                          Chains C, const double *__restrict__ lam0,
-                                                          double *const *grid_grads, double *__restrict__ amp_part,
-                                                          double *__restrict__ q_part, double *__restrict__ lam_init) {
+// (c) per block: lambda at the chunks' ends, then at the steps' ends, then the reverse-mode step of every
+// step; the field-parameter and q contributions go to per-block partials (amplitudes, q; a fixed tree) or
+// atomics (grid samples).  Only the 6 x 6 products of 16 steps are serial; 20001 points 54 us (258 when a
+// thread ran the reverse-mode steps of its chunk one after another).
+__global__ void __launch_bounds__(kAdjBlock) finish_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
+                                                           Chains C, const double *__restrict__ jac,
+                                                           const double *__restrict__ chunk_maps,
+                                                           const double *__restrict__ lam_end,
+                                                           double *const *grid_grads, double *__restrict__ amp_part,
+                                                           double *__restrict__ q_part, double *__restrict__ lam_init) {
   __shared__ srs_field F[kAdjMaxFields];
-  for (int i = threadIdx.x; i < nf; i += blockDim.x) F[i] = gF[i];
-  __syncthreads();
-  const int64_t gc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gc >= C.total_chunks) return;
-  const int chain = find_chain(C, gc, false);
+  __shared__ double sJ[kJacDoubles];
+  __shared__ double lam_g[kAdjBlock][6];  // g_j, then lambda_{j+1}
+  __shared__ double chunk_lam[kAdjChunks][6];
+  const int t = threadIdx.x, lane = t & 31;
+  const int chain = find_chain(C, blockIdx.x);
   const Chain &ch = C.c[chain];
-  const int64_t c = gc - ch.chunk_off;
-  const int64_t j0 = c * kAdjChunk, j1 = imin64(j0 + kAdjChunk, ch.L - 1);
-  double lam[6];
-  if (c == ch.nch - 1) {
-    load_g(T, ch, ch.L - 1, lam);
-  } else {
-    for (int r = 0; r < 6; ++r) lam[r] = lam0[6 * (ch.chunk_off + c + 1) + r];
+  const int64_t b = blockIdx.x - ch.blk_off, j0 = b * kAdjBlock;
+  const int cnt = (int)imin64(kAdjBlock, ch.L - 1 - j0);
+  for (int i = t; i < nf; i += kAdjBlock) F[i] = gF[i];
+  for (int k = t; k < 36 * cnt; k += kAdjBlock) sJ[jac_at(k / 36) + k % 36] = jac[36 * (ch.step_off + j0) + k];
+  V3 pos = v3(0, 0, 0), vel = v3(0, 0, 0);
+  if (t < cnt) {
+    double g[6];
+    load_g(T, ch, j0 + t, g);
+    for (int r = 0; r < 6; ++r) lam_g[t][r] = g[r];
+    load_state(T, ch.base + ch.dir * (j0 + t), pos, vel);
   }
+  if (t < 32) {
+    const int rr = lane < 6 ? lane : 0;
+    double m[kAdjChunks][7], lam = lam_end[6 * (int64_t)blockIdx.x + rr];
+#pragma unroll
+    for (int c = 0; c < kAdjChunks; ++c) {
+      const double *const o = chunk_maps + 42 * (kAdjChunks * (int64_t)blockIdx.x + c);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) m[c][k] = o[6 * rr + k];
+      m[c][6] = o[36 + rr];
+    }
+#pragma unroll
+    for (int c = kAdjChunks - 1; c >= 0; --c) {
+      if (lane < 6) chunk_lam[c][lane] = lam;
+      lam = apply_row(m[c], m[c][6], lam, 0);
+    }
+  }
+  __syncthreads();
+  if (t < 8 * kAdjChunks) {  // (two whole warps: eight lanes per chunk, six of them one component each)
+    const int c = t / 8, r = t % 8 < 6 ? t % 8 : 0;
+    double lam = chunk_lam[c][r];
+    for (int j = (c + 1) * kAdjChunk - 1; j >= c * kAdjChunk; --j) {
+      const double *const J = sJ + jac_at(j);  // (past the end: not used)
+      double m[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) m[k] = J[6 * k + r];
+      const double g = lam_g[j][r];
+      __syncwarp();
+      if (j < cnt && t % 8 < 6) lam_g[j][r] = lam;
+      const double next = apply_row(m, g, lam, lane & 24);
+      if (j < cnt) lam = next;
+    }
+    if (t < 6 && b == 0) lam_init[6 * chain + t] = lam;
+  }
+  __syncthreads();
   double amp[3 * kAdjMaxFields];
   for (int i = 0; i < 3 * kAdjMaxFields; ++i) amp[i] = 0.0;
   double qb = 0.0;
-  for (int64_t j = j1 - 1; j >= j0; --j) {
-    V3 pos, vel;
-    load_state(T, ch.base + ch.dir * j, pos, vel);
+  if (t < cnt) {
+    const double *const lam = lam_g[t];
     Stages S;
     make_stages(F, nf, q, pos, vel, ch.h, S);
     V3 pb, vb;
     step_vjp(F, nf, S, q, ch.h, v3(lam[0], lam[1], lam[2]), v3(lam[3], lam[4], lam[5]) * (1.0 / kC), pb, vb, qb, amp,
              grid_grads);
-    double g[6];
-    load_g(T, ch, j, g);
-    lam[0] = g[0] + pb.x;
-    lam[1] = g[1] + pb.y;
-    lam[2] = g[2] + pb.z;
-    lam[3] = g[3] + vb.x * kC;
-    lam[4] = g[4] + vb.y * kC;
-    lam[5] = g[5] + vb.z * kC;
   }
-  for (int i = 0; i < 3 * nf && i < 3 * kAdjMaxFields; ++i) amp_part[(int64_t)3 * nf * gc + i] = amp[i];
-  q_part[gc] = qb;
-  if (c == 0)
-    for (int r = 0; r < 6; ++r) lam_init[6 * chain + r] = lam[r];
+  double *const red = sJ;  // (its last readers passed the barrier)
+  for (int i = -1; i < 3 * nf; ++i) {
+    double v = i < 0 ? qb : amp[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[(i + 1) * (kAdjBlock / 32) + t / 32] = v;
+  }
+  __syncthreads();
+  for (int i = t; i < 1 + 3 * nf; i += kAdjBlock) {
+    double v = 0.0;
+    for (int w = 0; w < kAdjBlock / 32; ++w) v += red[i * (kAdjBlock / 32) + w];
+    if (i == 0) q_part[blockIdx.x] = v;
+    else amp_part[(int64_t)3 * nf * blockIdx.x + i - 1] = v;
+  }
 }
 
 // Fixed-order totals: out[0..2] dL/dx0, out[3..5] dL/dbeta0, out[6] dL/dq, out[7..] amplitudes.  The
-// per-chunk partials of q and of each amplitude are added by the block: thread t adds a contiguous
-// run of chunks in order, then a fixed tree over the 128 runs (a deterministic order; one thread
-// adding all 1250 partials of config 4 one load after another took 0.12 ms).
+// per-block partials of q and of each amplitude are added by the block: thread t adds a contiguous
+// run of them in order, then a fixed tree over the 128 runs (a deterministic order).
 __global__ void __launch_bounds__(128) adjoint_total_kernel(Chains C, int nf, const double *__restrict__ lam_init,
                                                             const double *__restrict__ amp_part,
                                                             const double *__restrict__ q_part,
@@ -542,7 +594,7 @@ __global__ void __launch_bounds__(128) adjoint_total_kernel(Chains C, int nf, co
     for (int k = 0; k < C.n; ++k) s += lam_init[6 * k + t];
     out[t] = s;
   }
-  const int64_t total = C.total_chunks, per = (total + 127) / 128;
+  const int64_t total = C.total_blocks, per = (total + 127) / 128;
   const int64_t g0 = t * per, g1 = g0 + per < total ? g0 + per : total;
   for (int o = 0; o < 1 + 3 * nf; ++o) {  // o = 0: q; o = 1 + i: amplitude i
     double s = 0.0;
@@ -697,7 +749,7 @@ srs_status srs_trajectory_adjoint(const srs_field *fields, int32_t nfields, cons
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Chains C;
   std::memset(&C, 0, sizeof C);
-  int64_t chunks = 0, steps = 0;
+  int64_t blocks = 0, steps = 0;
   auto add = [&](int64_t L, double h, int64_t base, int dir, int skip) {
     Chain &ch = C.c[C.n++];
     ch.L = L;
@@ -705,21 +757,20 @@ srs_status srs_trajectory_adjoint(const srs_field *fields, int32_t nfields, cons
     ch.base = base;
     ch.dir = dir;
     ch.skip_g0 = skip;
-    ch.nch = L > 1 ? (L - 1 + kAdjChunk - 1) / kAdjChunk : 0;
-    ch.chunk_off = chunks;
+    ch.nblk = (L - 1 + kAdjBlock - 1) / kAdjBlock;
+    ch.blk_off = blocks;
     ch.step_off = steps;
-    chunks += ch.nch;
+    blocks += ch.nblk;
     steps += L - 1;
   };
   add(nf, dt, nb, +1, 0);
   if (nb > 0) add(nb + 1, -dt, nb, -1, 1);
-  C.total_chunks = chunks;
-  C.total_steps = steps;
+  C.total_blocks = blocks;
   const Traj T{d_x, d_beta, d_gx, d_gbeta, nf + nb};
   const double q = particle->qomg;
 
   // device copies: fields, grid-gradient pointer table
-  DeviceBuffer dF, dG, jac, Mb, lam0, amp, qp, laminit, out;
+  DeviceBuffer dF, dG, jac, Mb, lam, amp, qp, laminit, out;
   SRS_CUDA(dF.alloc(sizeof(srs_field) * std::max(1, nfields), s));
   SRS_CUDA(dG.alloc(sizeof(double *) * std::max(1, nfields), s));
   std::vector<double *> gg(std::max(1, nfields), nullptr);
@@ -727,25 +778,25 @@ srs_status srs_trajectory_adjoint(const srs_field *fields, int32_t nfields, cons
   if (nfields > 0)
     SRS_CUDA(cudaMemcpyAsync(dF.ptr, fields, sizeof(srs_field) * nfields, cudaMemcpyHostToDevice, s));
   SRS_CUDA(cudaMemcpyAsync(dG.ptr, gg.data(), sizeof(double *) * gg.size(), cudaMemcpyHostToDevice, s));
+  const int64_t nb1 = std::max<int64_t>(1, blocks);
   SRS_CUDA(jac.alloc(sizeof(double) * 36 * std::max<int64_t>(1, steps), s));
-  SRS_CUDA(Mb.alloc(sizeof(double) * 42 * std::max<int64_t>(1, chunks), s));
-  SRS_CUDA(lam0.alloc(sizeof(double) * 6 * std::max<int64_t>(1, chunks), s));
-  SRS_CUDA(amp.alloc(sizeof(double) * 3 * std::max(1, nfields) * std::max<int64_t>(1, chunks), s));
-  SRS_CUDA(qp.alloc(sizeof(double) * std::max<int64_t>(1, chunks), s));
+  SRS_CUDA(Mb.alloc(sizeof(double) * 42 * (kAdjChunks + 1) * nb1, s));
+  SRS_CUDA(lam.alloc(sizeof(double) * 6 * nb1, s));
+  SRS_CUDA(amp.alloc(sizeof(double) * 3 * std::max(1, nfields) * nb1, s));
+  SRS_CUDA(qp.alloc(sizeof(double) * nb1, s));
   SRS_CUDA(laminit.alloc(sizeof(double) * 12, s));
   SRS_CUDA(out.alloc(sizeof(double) * (7 + 3 * std::max(1, nfields)), s));
   SRS_CUDA(cudaMemsetAsync(laminit.ptr, 0, sizeof(double) * 12, s));
   const srs_field *Fd = dF.as<srs_field>();
   if (steps > 0) {
-    step_jacobian_kernel<<<(unsigned)((steps + 127) / 128), 128, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>());
+    double *const chunk_maps = Mb.as<double>(), *const block_maps = chunk_maps + 42 * kAdjChunks * blocks;
+    step_maps_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(), chunk_maps, block_maps);
     SRS_CUDA(cudaGetLastError());
-    chunk_compose_kernel<<<(unsigned)((chunks + 63) / 64), 64, 0, s>>>(T, C, jac.as<double>(), Mb.as<double>());
+    carry_kernel<<<C.n, 32, 0, s>>>(T, C, block_maps, lam.as<double>());
     SRS_CUDA(cudaGetLastError());
-    carry_kernel<<<C.n, 32, 0, s>>>(T, C, Mb.as<double>(), lam0.as<double>());
-    SRS_CUDA(cudaGetLastError());
-    chunk_finish_kernel<<<(unsigned)((chunks + 63) / 64), 64, 0, s>>>(
-        Fd, nfields, q, T, C, lam0.as<double>(), reinterpret_cast<double *const *>(dG.ptr), amp.as<double>(),
-        qp.as<double>(), laminit.as<double>());
+    finish_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(), chunk_maps,
+                                                         lam.as<double>(), reinterpret_cast<double *const *>(dG.ptr),
+                                                         amp.as<double>(), qp.as<double>(), laminit.as<double>());
     SRS_CUDA(cudaGetLastError());
   }
   // chains of a single state: lambda_0 = g_0
