@@ -5,8 +5,8 @@
 // |E_k|^2 (OSCARSSR.cc:1154-1251).  Given dL/dflux_k this file computes dL/d(field parameters),
 // dL/dx0, dL/dbeta0 and dL/d(q/(m gamma)).
 //
-// 1. Sum adjoint (spectrum_adjoint_kernel): one thread per trajectory point i, looping over the
-//    energies, gives g_i = dL/d(x_i, beta_i) in closed form (derivatives of the amplitude
+// 1. Sum adjoint (spectrum_adjoint_kernel): four lanes per trajectory point i, looping over the
+//    energies, give g_i = dL/d(x_i, beta_i) in closed form (derivatives of the amplitude
 //    (beta - n(1 + i c/(w D)))/D and of the phase w (i dt + D/c) with respect to x and beta).
 // 2. Trajectory adjoint: lambda_j = dL/ds_j obeys lambda_j = g_j + J_j^T lambda_{j+1}, where J_j is
 //    the Jacobian of RK4 step j.  Instead of one serial sweep back through the N steps (the forward
@@ -612,7 +612,8 @@ __global__ void __launch_bounds__(128) adjoint_total_kernel(Chains C, int nf, co
 
 // ---------------------------------------------------------------- sum adjoint
 
-// Per energy k: W_k = 2 w_k conj(E_k) with w_k = dL/dflux_k * C2 (C0 w_k dt)^2.
+// Per energy k, nine doubles: w_k, 2 w conj(E_k) with w = dL/dflux_k * C2 (C0 w_k dt)^2, c/w_k, w_k/c.
+constexpr int kWeightDoubles = 9;  // (odd: four energies side by side in shared memory are on different banks)
 __global__ void spectrum_weights_kernel(const double *__restrict__ energies, const double *__restrict__ e6,
                                         const double *__restrict__ gflux, int64_t ne, double dt, double C0, double C2,
                                         double *__restrict__ W) {
@@ -621,14 +622,21 @@ __global__ void spectrum_weights_kernel(const double *__restrict__ energies, con
   const double om = ev_to_omega(energies[k]);
   const double g = C0 * om * dt;
   const double w = 2.0 * gflux[k] * C2 * g * g;
-  W[8 * k + 0] = om;
+  W += kWeightDoubles * k;
+  W[0] = om;
+  W[7] = kC / om;
+  W[8] = om / kC;
   for (int c = 0; c < 3; ++c) {
-    W[8 * k + 1 + 2 * c] = w * e6[6 * k + 2 * c];
-    W[8 * k + 2 + 2 * c] = -w * e6[6 * k + 2 * c + 1];
+    W[1 + 2 * c] = w * e6[6 * k + 2 * c];
+    W[2 + 2 * c] = -w * e6[6 * k + 2 * c + 1];
   }
 }
 
-constexpr int kSumAdjThreads = 128, kSumAdjTile = 128;
+// kSumAdjLanes lanes share a point, each every kSumAdjLanes-th energy: a trajectory has too few points for one
+// thread each (20001: one warp per scheduler).  Only the three sums that the derivatives are linear in are
+// formed per energy: ~50 operations, where the derivatives themselves took ~220 with two divisions;
+// 20001 points x 200 energies 90 -> 28 us (12 at the FP64 pipe's rate).
+constexpr int kSumAdjThreads = 128, kSumAdjTile = 128, kSumAdjLanes = 4, kSumAdjPoints = kSumAdjThreads / kSumAdjLanes;
 
 __global__ void __launch_bounds__(kSumAdjThreads) spectrum_adjoint_kernel(const double *__restrict__ X,
                                                                           const double *__restrict__ Bt, int64_t n,
@@ -636,8 +644,8 @@ __global__ void __launch_bounds__(kSumAdjThreads) spectrum_adjoint_kernel(const 
                                                                           const double *__restrict__ W, int64_t ne,
                                                                           double *__restrict__ gx,
                                                                           double *__restrict__ gb) {
-  __shared__ double sW[kSumAdjTile][8];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double sW[kSumAdjTile * kWeightDoubles];
+  const int64_t i = (int64_t)blockIdx.x * kSumAdjPoints + threadIdx.x / kSumAdjLanes;
   const bool active = i < n;
   const int64_t ii = active ? i : n - 1;
   const V3 x = v3(X[ii], X[n + ii], X[2 * n + ii]);
@@ -651,34 +659,43 @@ __global__ void __launch_bounds__(kSumAdjThreads) spectrum_adjoint_kernel(const 
   const V3 nv = R / D;
   const double tau = dt * (double)(int)ii + D / kC;
   const double nn[3] = {nv.x, nv.y, nv.z}, bb[3] = {be.x, be.y, be.z};
-  double A[3] = {0, 0, 0}, Bc[3] = {0, 0, 0}, Tt = 0.0;
+  // With P = W e^{i w tau}: A = Sum Re P, Bc = Sum (c/w) Im P, Wc = Sum (w/c) Im P; the derivatives of the
+  // amplitude and of the phase are linear in them
+  double A[3] = {0, 0, 0}, Bc[3] = {0, 0, 0}, Wc[3] = {0, 0, 0};
   for (int64_t k0 = 0; k0 < ne; k0 += kSumAdjTile) {
     const int cnt = (int)imin64(kSumAdjTile, ne - k0);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * 8; t += blockDim.x) sW[t / 8][t % 8] = W[8 * k0 + t];
+    for (int t = threadIdx.x; t < cnt * kWeightDoubles; t += blockDim.x) sW[t] = W[kWeightDoubles * k0 + t];
     __syncthreads();
-    for (int k = 0; k < cnt; ++k) {
-      const double om = sW[k][0];
+    for (int k = threadIdx.x % kSumAdjLanes; k < cnt; k += kSumAdjLanes) {
+      const double *const w = sW + kWeightDoubles * k;
       double sn, cs;
-      sincos(reduce_2pi(om * tau), &sn, &cs);
-      const double cow = kC / om, woc = om / kC;
-      double s1r = 0.0, s2i = 0.0, s3i = 0.0;
+      sincos_reduced(w[0] * tau, sn, cs);
+      const double cow = w[7], woc = w[8];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double wr = sW[k][1 + 2 * c], wi = sW[k][2 + 2 * c];
-        const double pr = wr * cs - wi * sn, pi = wr * sn + wi * cs;  // P = W e^{i a}
-        A[c] += pr;
-        Bc[c] += cow * pi;
-        s1r += pr * (bb[c] - 2.0 * nn[c]);
-        s2i += pi * nn[c];
-        // (w/c) Im(P u) with u = (beta - n)/D - i (c/w) n / D^2
-        s3i += -pr * nn[c] * iD * iD + woc * pi * (bb[c] - nn[c]) * iD;
+        const double wr = w[1 + 2 * c], wi = w[2 + 2 * c];
+        const double pi = __fma_rn(wr, sn, wi * cs);
+        A[c] += __fma_rn(wr, cs, -(wi * sn));
+        Bc[c] = __fma_rn(cow, pi, Bc[c]);
+        Wc[c] = __fma_rn(woc, pi, Wc[c]);
       }
-      Tt += s1r * iD * iD + 3.0 * cow * s2i * iD * iD * iD + s3i;
     }
   }
-  if (!active) return;
+#pragma unroll
+  for (int o = 1; o < kSumAdjLanes; o *= 2) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      A[c] += __shfl_xor_sync(0xffffffffu, A[c], o);
+      Bc[c] += __shfl_xor_sync(0xffffffffu, Bc[c], o);
+      Wc[c] += __shfl_xor_sync(0xffffffffu, Wc[c], o);
+    }
+  }
+  if (!active || threadIdx.x % kSumAdjLanes != 0) return;
   const double iD2 = iD * iD, iD3 = iD2 * iD;
+  double Tt = 0.0;
+  for (int c = 0; c < 3; ++c)
+    Tt += A[c] * (bb[c] - 3.0 * nn[c]) * iD2 + 3.0 * Bc[c] * nn[c] * iD3 + Wc[c] * (bb[c] - nn[c]) * iD;
   for (int c = 0; c < 3; ++c) {
     gb[c * n + i] = A[c] * iD;
     gx[c * n + i] = A[c] * iD2 - Bc[c] * iD3 + nn[c] * Tt;
@@ -723,11 +740,11 @@ srs_status srs_spectrum_adjoint(srs_traj_view traj, srs_beam_consts beam, const 
     return fail(SRS_ERR_INVALID, "bad argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   DeviceBuffer W;
-  SRS_CUDA(W.alloc(sizeof(double) * 8 * ne, s));
+  SRS_CUDA(W.alloc(sizeof(double) * kWeightDoubles * ne, s));
   spectrum_weights_kernel<<<(unsigned)((ne + 127) / 128), 128, 0, s>>>(
       d_energies, d_e6, d_gflux, ne, traj.dt, flux_c0(beam.charge), flux_c2(beam.charge, beam.current), W.as<double>());
   SRS_CUDA(cudaGetLastError());
-  spectrum_adjoint_kernel<<<(unsigned)((traj.n + kSumAdjThreads - 1) / kSumAdjThreads), kSumAdjThreads, 0, s>>>(
+  spectrum_adjoint_kernel<<<(unsigned)((traj.n + kSumAdjPoints - 1) / kSumAdjPoints), kSumAdjThreads, 0, s>>>(
       traj.x, traj.beta, traj.n, traj.dt, v3(obs[0], obs[1], obs[2]), W.as<double>(), ne, d_gx, d_gbeta);
   SRS_CUDA(cudaGetLastError());
   return SRS_OK;

@@ -257,7 +257,36 @@ __device__ __forceinline__ double reduce_2pi(double x) {
   return r;
 }
 
-// The same reduction in FP32 arithmetic, for arguments of a few hundred radians at most.
+// sin and cos of x for |x| < 2^46: x = k pi/2 + r by Cody & Waite's steps (k from the 1.5 * 2^52 shift; a
+// third part of pi/2, below |k| * 2e-33, would not be seen), then sin r = r + r^3 S(r^2) and cos r = 1 -
+// r^2/2 + r^4 C(r^2) with S and C the degree-5 interpolants at the Chebyshev nodes of [0, (pi/4)^2] of
+// (sin(r)/r - 1)/r^2 and (cos(r) - 1 + r^2/2)/r^4: 1e-17 and 5e-19 from the functions.
+__device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs) {
+  const double shift = 6755399441055744.0;
+  const double kd = __fma_rn(x, 0.6366197723675814, shift);
+  const int k = __double2loint(kd);
+  const double kf = kd - shift;
+  double r = __fma_rn(-kf, 1.5707963267948966, x);
+  r = __fma_rn(-kf, 6.123233995736766e-17, r);
+  const double w = r * r;
+  double s = __fma_rn(w, 1.5918129266803394e-10, -2.5051131844614108e-08);
+  double c = __fma_rn(w, -1.1382632407965617e-11, 2.087614626815952e-09);
+  s = __fma_rn(w, s, 2.755731610255057e-06);
+  c = __fma_rn(w, c, -2.7557317271728623e-07);
+  s = __fma_rn(w, s, -0.0001984126983675857);
+  c = __fma_rn(w, c, 2.4801587298765686e-05);
+  s = __fma_rn(w, s, 0.008333333333330948);
+  c = __fma_rn(w, c, -0.0013888888888887398);
+  s = __fma_rn(w, s, -0.16666666666666666);
+  c = __fma_rn(w, c, 0.041666666666666664);
+  s = __fma_rn(r * w, s, r);
+  c = __fma_rn(w * w, c, __fma_rn(-0.5, w, 1.0));
+  const double a = (k & 1) ? c : s, b = (k & 1) ? s : c;
+  sn = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(k & 2) << 30), __double2loint(a));
+  cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((k + 1) & 2) << 30), __double2loint(b));
+}
+
+// reduce_2pi in FP32 arithmetic, for arguments of a few hundred radians at most.
 __device__ __forceinline__ float reduce_2pi_f(float x) {
   const float kInv2Pi = 0.159154943f;
   const float P1 = 6.2831855f, P2 = -1.7484555e-07f, P3 = -6.860498e-15f;

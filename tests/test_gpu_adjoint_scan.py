@@ -1,5 +1,5 @@
-"""The trajectory adjoint's scan at the edges of its chunks (16 steps) and blocks (128) against a serial
-long-double sweep over the same stored points."""
+"""The trajectory adjoint's scan at the edges of its chunks (16 steps) and blocks (128), and the sum adjoint
+at the edges of its groups of energies, against long-double sums over the same stored points."""
 import ctypes as C
 import math
 
@@ -104,3 +104,43 @@ def test_trajectory_adjoint_against_a_serial_sweep(npoints, start):
     sx = np.abs(gx.cpu().numpy()).sum() + turn * sbeta
     assert np.all(np.abs(np.array(ic[:3]) - ric[:3]) <= eps * sx)
     assert np.all(np.abs(np.array(ic[3:6]) - ric[3:]) <= eps * sbeta)
+
+
+# The adjoint is linear in the energies: all at once against one energy at a time, summed in long double. An
+# energy adds ~20 rounded operations and one addition to what is added up.
+@pytest.mark.parametrize("npoints,ne", [(2, 1), (31, 3), (32, 4), (33, 5), (65, 127), (64, 128), (100, 129), (40, 260)])
+def test_sum_adjoint_against_long_double(npoints, ne):
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+
+    part, _ = D.ideal_particle(3.0, [1e-5, -2e-5, -1.0], [1e-5, 2e-5, 1])
+    tr = D.trajectory([D.undulator(list(AMPLITUDE), [0, 0, PERIOD], NPERIODS)], [part], 0.0, 2.0, 0.0, npoints)
+    n = tr.x.shape[-1]
+    rng = np.random.default_rng(ne)
+    energies = np.linspace(100.0, 900.0, ne)
+    e = torch.tensor(energies, device="cuda")
+    e6, gf = torch.tensor(rng.normal(size=6 * ne), device="cuda"), torch.tensor(rng.normal(size=ne), device="cuda")
+    gx, gb = torch.empty(3 * n, dtype=torch.float64, device="cuda"), torch.empty(3 * n, dtype=torch.float64, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    args = (tr.view(), _lib.BeamConsts(-1.602176634e-19, 0.5), _lib.v3([0.0, 0.0, 30.0]), ptr(e))
+    _lib.check(_lib.lib.srs_spectrum_adjoint(*args, ne, ptr(e6), ptr(gf), ptr(gx), ptr(gb), D._stream()))
+    # linear in the energies; the terms of one energy are bounded by those of E's six real components
+    sx, sb, mx, mb = (np.zeros(3 * n, dtype=L) for _ in range(4))
+    hx, hb = torch.empty_like(gx), torch.empty_like(gb)
+    for k in range(ne):
+        for part in range(7):
+            ek, ck, gk = e[k:k + 1].clone(), e6[6 * k:6 * k + 6].clone(), gf[k:k + 1].clone()
+            if part:
+                ck *= torch.arange(6, device="cuda") == part - 1
+            _lib.check(_lib.lib.srs_spectrum_adjoint(*args[:3], ptr(ek), 1, ptr(ck), ptr(gk), ptr(hx), ptr(hb), D._stream()))
+            x, b = hx.cpu().numpy().astype(L), hb.cpu().numpy().astype(L)
+            if part:
+                mx, mb = mx + np.abs(x), mb + np.abs(b)
+            else:
+                sx, sb = sx + x, sb + b
+    eps = (20 + ne) * 2.0 ** -53
+    # of the magnitudes per point: the three components share their terms (n Tt)
+    top = lambda a: np.tile(a.reshape(3, n).sum(axis=0), 3)
+    assert np.all(np.abs(gx.cpu().numpy() - sx) <= eps * top(mx))
+    assert np.all(np.abs(gb.cpu().numpy() - sb) <= eps * top(mb))
