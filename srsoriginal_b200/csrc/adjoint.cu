@@ -12,12 +12,11 @@
 //    the Jacobian of RK4 step j.  Instead of one serial sweep back through the N steps (the forward
 //    RK4 is a serial chain; its adjoint need not be), the affine recurrence is solved as a scan:
 //      (a) every step's 6 x 6 Jacobian is formed in parallel from the stored states, by forward-mode
-//          tangents pushed through the four stages, and chunks of kAdjChunk steps, then the kAdjBlock steps of a block, are composed there into
-//          affine maps lambda_j0 = M lambda_j1 + b (step_maps_kernel);
-//      (b) one warp carries lambda across the block maps from the last point back to the first
+//          tangents pushed through the four stages, and chunks of kAdjChunk steps are composed there into affine maps
+//          lambda_j0 = M lambda_j1 + b (step_maps_kernel);
+//      (b) one warp carries lambda across the chunk maps from the last point back to the first
 //          (carry_kernel);
-//      (c) each block carries its end value across its chunks and, chunk by chunk, across the steps with
-//          the stored Jacobians; then all steps run the reverse-mode step from their own lambda at once
+//      (c) each chunk carries its end value across its steps with the stored Jacobians; then all steps run the reverse-mode step from their own lambda at once
 //          (VJP through the four stages, recomputed from the stored state), which yields the
 //          field-parameter and q/(m gamma) contributions (finish_kernel).
 //    The stored trajectory is itself the checkpoint set: the state at every step is in HBM (the sums
@@ -30,6 +29,8 @@
 // arithmetic is FP64.  Grid-sample gradients are accumulated with FP64 atomics (sub-ulp
 // run-to-run differences); everything else is reduced in a fixed order.
 #include <cuda_runtime.h>
+
+#include <cuda_pipeline.h>
 
 #include <algorithm>
 #include <cstring>
@@ -360,14 +361,13 @@ __device__ __forceinline__ int jac_at(int t) { return 37 * t + t / kAdjChunk; }
 constexpr int kJacDoubles = 37 * kAdjBlock + kAdjChunks;
 
 // (a) J~_j (6 x 6, row = output, column = input, in (x, beta) units) of every step, and the maps of the
-// block's chunks and of the block, composed backwards from M = I, b = 0: eight lanes per chunk, one per
+// block's chunks, composed backwards from M = I, b = 0: eight lanes per chunk, one per
 // column of M and one for b.  Bound by the latency of the four stages and six tangents of a step with one
-// warp per scheduler: 20001 points (157 blocks) 40 us, where the Jacobians (36 us) and then the maps of
+// warp per scheduler: 20001 points (157 blocks) 38 us, where the Jacobians (36 us) and then the maps of
 // the chunks by one thread each (41 us) took two kernels.
 __global__ void __launch_bounds__(kAdjBlock) step_maps_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
                                                               Chains C, double *__restrict__ jac,
-                                                              double *__restrict__ chunk_maps,
-                                                              double *__restrict__ block_maps) {
+                                                              double *__restrict__ chunk_maps) {
   __shared__ double sJ[kJacDoubles];
   __shared__ union {
     srs_field F[kAdjMaxFields];
@@ -427,24 +427,6 @@ __global__ void __launch_bounds__(kAdjBlock) step_maps_kernel(const srs_field *_
   }
   __syncthreads();
   for (int k = t; k < 42 * kAdjChunks; k += kAdjBlock) chunk_maps[42 * kAdjChunks * (int64_t)blockIdx.x + k] = sh.map[k / 42][k % 42];
-  if (t < 7) {
-    double m[6];
-    for (int r = 0; r < 6; ++r) m[r] = r == t;
-    for (int c = kAdjChunks - 1; c >= 0; --c) {  // (a chunk past the end is the identity)
-      const double *const o = sh.map[c];
-      double n[6];
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        double s = t == 6 ? o[36 + r] : 0.0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) s += o[6 * r + k] * m[k];
-        n[r] = s;
-      }
-#pragma unroll
-      for (int r = 0; r < 6; ++r) m[r] = n[r];
-    }
-    for (int r = 0; r < 6; ++r) block_maps[42 * (int64_t)blockIdx.x + (t < 6 ? 6 * r + t : 36 + r)] = m[r];
-  }
 }
 
 // b + M lambda for row r of an affine map, as a tree (depth 4 instead of a chain of six multiply-adds);
@@ -456,55 +438,84 @@ __device__ __forceinline__ double apply_row(const double m[6], double b, double 
   return b + (((m[0] * l[0] + m[1] * l[1]) + (m[2] * l[2] + m[3] * l[3])) + (m[4] * l[4] + m[5] * l[5]));
 }
 
-// (b) one warp per chain, lanes 0..5 own one component: lambda at every block's end.  Sequential over the
-// blocks, the rows of the next maps loaded while one is applied: 37 us for the 157 maps of 20001 points (155
-// for the maps of 1250 chunks).
-__global__ void __launch_bounds__(32) carry_kernel(Traj T, Chains C, const double *__restrict__ block_maps,
+// (b) one warp per chain, lanes 0..5 own one component: lambda at every chunk's end.  Sequential over the chunks;
+// the maps come through shared memory in tiles of kCarryTile, the next tile's asynchronous copies in flight
+// while the current one is applied, and a map's row is in registers before the map's turn: 95
+// us for the 1250 maps of 20001 points (155 when a row was loaded at its turn).  Carrying across maps of whole
+// blocks takes 37, but the longitudinal derivative, in which the terms cancel to ~1e-10, then moves by up
+// to 1e-9 of the gradient against the carry over these maps (by 3e-10 as it is).
+constexpr int kCarryTile = 64;  // chunk maps per tile: 64 x 42 doubles = 21.5 KB, two buffers
+__global__ void __launch_bounds__(32) carry_kernel(Traj T, Chains C, const double *__restrict__ chunk_maps,
                                                    double *__restrict__ lam_end) {
+  __shared__ __align__(16) double tile[2][kCarryTile * 42];
   const Chain &ch = C.c[blockIdx.x];
   const int r = threadIdx.x, rr = r < 6 ? r : 0;
   if (ch.nblk == 0) return;
+  const int64_t nch = (ch.L - 1 + kAdjChunk - 1) / kAdjChunk, off = ch.blk_off * kAdjChunks;
   double g[6];
   load_g(T, ch, ch.L - 1, g);
   double lam = 0.0;  // lambda_{L-1} = g_{L-1}
 #pragma unroll
   for (int k = 0; k < 6; ++k)
     if (r == k) lam = g[k];
-  constexpr int kAhead = 4;  // maps in flight
-  double m[kAhead][7];
-  auto load = [&](int64_t c, double *o) {
-    const double *const p = block_maps + 42 * (ch.blk_off + (c > 0 ? c : 0));
-#pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = p[6 * rr + k];
-    o[6] = p[36 + rr];
-  };
-#pragma unroll
-  for (int a = 0; a < kAhead; ++a) load(ch.nblk - 1 - a, m[a]);
-  for (int64_t c = ch.nblk - 1; c >= 0; c -= kAhead) {
-#pragma unroll
-    for (int a = 0; a < kAhead; ++a) {
-      if (c - a < 0) break;
-      if (r < 6) lam_end[6 * (ch.blk_off + c - a) + r] = lam;
-      lam = apply_row(m[a], m[a][6], lam, 0);
-      load(c - a - kAhead, m[a]);
+  const int64_t ntiles = (nch + kCarryTile - 1) / kCarryTile;
+  // tile t: the chunks from hi(t) = nch - 1 - t * kCarryTile down to lo(t)
+  auto lo_of = [&](int64_t t) { return nch - (t + 1) * kCarryTile > 0 ? nch - (t + 1) * kCarryTile : (int64_t)0; };
+  auto fetch = [&](int64_t t) {  // 16-byte copies: a chunk map is 21 of them, 16-byte aligned
+    if (t < ntiles) {
+      const int64_t lo = lo_of(t);
+      const double *const src = chunk_maps + 42 * (off + lo);
+      const int n16 = (int)(nch - t * kCarryTile - lo) * 21;
+      for (int k = r; k < n16; k += 32) __pipeline_memcpy_async(&tile[t & 1][2 * k], src + 2 * k, 16);
     }
+    __pipeline_commit();
+  };
+  fetch(0);
+  for (int64_t t = 0; t < ntiles; ++t) {
+    fetch(t + 1);
+    __pipeline_wait_prior(1);
+    __syncwarp();
+    const int64_t lo = lo_of(t);
+    int c = (int)(nch - t * kCarryTile - lo) - 1;
+    constexpr int kAhead = 4;
+    double m[kAhead][7];
+    auto load = [&](int k, double *o) {
+      const double *const p = tile[t & 1] + 42 * (k > 0 ? k : 0);
+#pragma unroll
+      for (int q = 0; q < 6; q += 2) {
+        const double2 v = *reinterpret_cast<const double2 *>(p + 6 * rr + q);
+        o[q] = v.x;
+        o[q + 1] = v.y;
+      }
+      o[6] = p[36 + rr];
+    };
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) load(c - a, m[a]);
+    double *out = lam_end + 6 * (off + lo) + rr;
+    for (; c >= 0; c -= kAhead) {
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        if (c - a < 0) break;
+        if (r < 6) out[6 * (c - a)] = lam;
+        lam = apply_row(m[a], m[a][6], lam, 0);
+        load(c - a - kAhead, m[a]);
+      }
+    }
+    __syncwarp();  // every lane is done with this buffer before the next iteration refills it
   }
 }
 
-// (c) per block: lambda at the chunks' ends, then at the steps' ends, then the reverse-mode step of every
-// step; the field-parameter and q contributions go to per-block partials (amplitudes, q; a fixed tree) or
-// atomics (grid samples).  Only the 6 x 6 products of 16 steps are serial; 20001 points 54 us (258 when a
+// (c) per block: lambda at the steps' ends, then the reverse-mode step of every step; the field-parameter and q contributions go to per-block partials (amplitudes, q; a fixed tree) or
+// atomics (grid samples).  Only the 6 x 6 products of 16 steps are serial; 20001 points 51 us (258 when a
 // thread ran the reverse-mode steps of its chunk one after another).
 __global__ void __launch_bounds__(kAdjBlock) finish_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
                                                            Chains C, const double *__restrict__ jac,
-                                                           const double *__restrict__ chunk_maps,
                                                            const double *__restrict__ lam_end,
                                                            double *const *grid_grads, double *__restrict__ amp_part,
                                                            double *__restrict__ q_part, double *__restrict__ lam_init) {
   __shared__ srs_field F[kAdjMaxFields];
   __shared__ double sJ[kJacDoubles];
   __shared__ double lam_g[kAdjBlock][6];  // g_j, then lambda_{j+1}
-  __shared__ double chunk_lam[kAdjChunks][6];
   const int t = threadIdx.x, lane = t & 31;
   const int chain = find_chain(C, blockIdx.x);
   const Chain &ch = C.c[chain];
@@ -519,26 +530,10 @@ __global__ void __launch_bounds__(kAdjBlock) finish_kernel(const srs_field *__re
     for (int r = 0; r < 6; ++r) lam_g[t][r] = g[r];
     load_state(T, ch.base + ch.dir * (j0 + t), pos, vel);
   }
-  if (t < 32) {
-    const int rr = lane < 6 ? lane : 0;
-    double m[kAdjChunks][7], lam = lam_end[6 * (int64_t)blockIdx.x + rr];
-#pragma unroll
-    for (int c = 0; c < kAdjChunks; ++c) {
-      const double *const o = chunk_maps + 42 * (kAdjChunks * (int64_t)blockIdx.x + c);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) m[c][k] = o[6 * rr + k];
-      m[c][6] = o[36 + rr];
-    }
-#pragma unroll
-    for (int c = kAdjChunks - 1; c >= 0; --c) {
-      if (lane < 6) chunk_lam[c][lane] = lam;
-      lam = apply_row(m[c], m[c][6], lam, 0);
-    }
-  }
   __syncthreads();
   if (t < 8 * kAdjChunks) {  // (two whole warps: eight lanes per chunk, six of them one component each)
     const int c = t / 8, r = t % 8 < 6 ? t % 8 : 0;
-    double lam = chunk_lam[c][r];
+    double lam = c * kAdjChunk < cnt ? lam_end[6 * (kAdjChunks * (int64_t)blockIdx.x + c) + r] : 0.0;
     for (int j = (c + 1) * kAdjChunk - 1; j >= c * kAdjChunk; --j) {
       const double *const J = sJ + jac_at(j);  // (past the end: not used)
       double m[6];
@@ -797,8 +792,8 @@ srs_status srs_trajectory_adjoint(const srs_field *fields, int32_t nfields, cons
   SRS_CUDA(cudaMemcpyAsync(dG.ptr, gg.data(), sizeof(double *) * gg.size(), cudaMemcpyHostToDevice, s));
   const int64_t nb1 = std::max<int64_t>(1, blocks);
   SRS_CUDA(jac.alloc(sizeof(double) * 36 * std::max<int64_t>(1, steps), s));
-  SRS_CUDA(Mb.alloc(sizeof(double) * 42 * (kAdjChunks + 1) * nb1, s));
-  SRS_CUDA(lam.alloc(sizeof(double) * 6 * nb1, s));
+  SRS_CUDA(Mb.alloc(sizeof(double) * 42 * kAdjChunks * nb1, s));
+  SRS_CUDA(lam.alloc(sizeof(double) * 6 * kAdjChunks * nb1, s));
   SRS_CUDA(amp.alloc(sizeof(double) * 3 * std::max(1, nfields) * nb1, s));
   SRS_CUDA(qp.alloc(sizeof(double) * nb1, s));
   SRS_CUDA(laminit.alloc(sizeof(double) * 12, s));
@@ -806,12 +801,11 @@ srs_status srs_trajectory_adjoint(const srs_field *fields, int32_t nfields, cons
   SRS_CUDA(cudaMemsetAsync(laminit.ptr, 0, sizeof(double) * 12, s));
   const srs_field *Fd = dF.as<srs_field>();
   if (steps > 0) {
-    double *const chunk_maps = Mb.as<double>(), *const block_maps = chunk_maps + 42 * kAdjChunks * blocks;
-    step_maps_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(), chunk_maps, block_maps);
+    step_maps_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(), Mb.as<double>());
     SRS_CUDA(cudaGetLastError());
-    carry_kernel<<<C.n, 32, 0, s>>>(T, C, block_maps, lam.as<double>());
+    carry_kernel<<<C.n, 32, 0, s>>>(T, C, Mb.as<double>(), lam.as<double>());
     SRS_CUDA(cudaGetLastError());
-    finish_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(), chunk_maps,
+    finish_kernel<<<(unsigned)blocks, kAdjBlock, 0, s>>>(Fd, nfields, q, T, C, jac.as<double>(),
                                                          lam.as<double>(), reinterpret_cast<double *const *>(dG.ptr),
                                                          amp.as<double>(), qp.as<double>(), laminit.as<double>());
     SRS_CUDA(cudaGetLastError());
