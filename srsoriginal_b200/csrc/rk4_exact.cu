@@ -147,18 +147,8 @@ __device__ inline Item item_of(const Job &J, int it) {
 // more than the calls.
 __device__ __noinline__ V3 field_total(const Prepared *sp, const srs_field *sf, int nfields, V3 x) {
   V3 s = v3(0, 0, 0);
-  for (int f = 0; f < nfields; ++f) s = s + field_one(sp[f], sf[f], x);
+  for (int f = 0; f < nfields; ++f) s = s + field_along(sp[f], sf[f], x);
   return s;
-}
-
-// The field list and its prepared constants into shared memory, word by word.
-__device__ __forceinline__ void copy_fields(srs_field *sf, Prepared *sp, const srs_field *gf, const Prepared *gp,
-                                            int nfields) {
-  static_assert(sizeof(srs_field) % 8 == 0 && sizeof(Prepared) % 8 == 0, "copied as 8-byte words");
-  const long long *a = reinterpret_cast<const long long *>(gf), *b = reinterpret_cast<const long long *>(gp);
-  long long *c = reinterpret_cast<long long *>(sf), *d = reinterpret_cast<long long *>(sp);
-  for (int k = threadIdx.x; k < nfields * (int)(sizeof(srs_field) / 8); k += blockDim.x) c[k] = a[k];
-  for (int k = threadIdx.x; k < nfields * (int)(sizeof(Prepared) / 8); k += blockDim.x) d[k] = b[k];
 }
 
 // The increments of one serial RK4 step that depend on the state only weakly (OSCARSSR.cc:826-874; the
@@ -309,7 +299,7 @@ __global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ 
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int items = J.nparticles * J.chains;
   if (g < nfields && undulators) prepare_undulator(fields[g], W.und[g]);
-  else if (g < nfields) prepare(fields[g], W.prep[g]);
+  else if (g < nfields) prepare(fields[g], W.prep[g], true);
   if (g == 0) {
     *W.done = 0;
     *W.all_ticket = 0;

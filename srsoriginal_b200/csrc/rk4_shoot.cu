@@ -34,8 +34,6 @@
 
 #include <algorithm>
 
-#include <cuda_pipeline.h>
-
 #include "rk4_fields.cuh"
 #include "srs_internal.h"
 
@@ -98,7 +96,7 @@ __global__ void shoot_init_kernel(Plan P, const srs_particle *__restrict__ part,
                                   const srs_field *__restrict__ fields, int nfields) {
   allow_next_grid();  // the first pass may be set up meanwhile (it waits for this grid's writes)
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < nfields) prepare(fields[g], W.prep[g]);  // once per integration, not once per pass and block
+  if (g < nfields) prepare(fields[g], W.prep[g], true);  // once per integration, not once per pass and block
   if (g == 0) {
     for (int k = 0; k < 5; ++k) W.flags[k] = 0;
     for (int k = 0; k < kMaxIters; ++k) W.diag[k] = 0.0;
@@ -123,6 +121,16 @@ __device__ __forceinline__ double dot6(const double *a, int stride, const double
   return ((p0 + p1) + (p2 + p3)) + (p4 + p5);
 }
 
+// a row of a 6 x 6 matrix, 16-byte aligned
+__device__ __forceinline__ void load_row(double o[6], const double *p) {
+#pragma unroll
+  for (int k = 0; k < 6; k += 2) {
+    const double2 v = *reinterpret_cast<const double2 *>(p + k);
+    o[k] = v.x;
+    o[k + 1] = v.y;
+  }
+}
+
 struct F3 {
   float x, y, z;
 };
@@ -143,7 +151,8 @@ template <int M>
 struct PassShared {
   srs_field sf[kMaxFieldsShared];
   Prepared sp[kMaxFieldsShared];
-  double sPhi[M][36], sR[M][6], sU[M + 1][6], sF[M][6], sM[2][36], sB[2][6];
+  __align__(16) double sPhi[M][36];
+  double sR[M][6], sU[M + 1][6], sF[M][6];
   double wred[kShootThreads / 32];
   int am_last, done;
 };
@@ -160,8 +169,6 @@ __device__ __forceinline__ void shoot_pass(PassShared<kShootThreads / G> &sh, co
   auto &sR = sh.sR;
   auto &sU = sh.sU;
   auto &sF = sh.sF;
-  auto &sM = sh.sM;
-  auto &sB = sh.sB;
   auto &wred = sh.wred;
   int &am_last = sh.am_last;
   int &done = sh.done;
@@ -169,10 +176,7 @@ __device__ __forceinline__ void shoot_pass(PassShared<kShootThreads / G> &sh, co
   const int c = blockIdx.x, g0 = c * M, g = g0 + grp;
   const int iter = W.flags[1];
   const unsigned full = 0xffffffffu;
-  for (int i = t; i < nfields; i += blockDim.x) {
-    sf[i] = gfields[i];
-    sp[i] = W.prep[i];
-  }
+  copy_fields(sf, sp, gfields, W.prep, nfields);
   // (1) this chunk's start states: the previous iteration's update, segment after segment (the first
   // segment's was set by the last block's sweep)
   for (int k = t; k < M * 6; k += blockDim.x) sU[k / 6][k % 6] = W.U[6 * g0 + k];
@@ -223,7 +227,7 @@ __device__ __forceinline__ void shoot_pass(PassShared<kShootThreads / G> &sh, co
     float jm[9];
     const V3 at = slot == 0 ? pa : pb;
     if (nfields > 0) {
-      mine = field_one(myp, ff, at);
+      mine = field_along(myp, ff, at);
       if (kTan) field_one_jac(myp, ff, at, jm);
     }
     Ba = v3(0, 0, 0);
@@ -338,29 +342,35 @@ __device__ __forceinline__ void shoot_pass(PassShared<kShootThreads / G> &sh, co
   if (!kTan)  // the Jacobians of the last pass with tangents
     for (int k = t; k < M * 36; k += blockDim.x) sPhi[k / 36][k % 36] = W.Phi[36 * g0 + k];
   __syncthreads();
-  // compose M <- Phi_n M, b <- r_n + Phi_n b over the chunk's segments in order (threads 0..35 own an
-  // entry of M, threads 36..41 an entry of b; M is unchanged without new Jacobians)
-  const int ti = t < 36 ? t / 6 : t - 36, tj = t % 6;
-  if (t < 36) sM[0][t] = ti == tj ? 1.0 : 0.0;
-  if (t >= 36 && t < 42) sB[0][ti] = 0.0;
-  __syncthreads();
-  int cur = 0;
-  for (int n = 0; n < M; ++n) {
-    if (kTan && t < 36) {
-      sM[cur ^ 1][t] = dot6(&sPhi[n][6 * ti], 1, &sM[cur][tj], 6);
+  // compose M <- Phi_n M, b <- r_n + Phi_n b over the chunk's segments in order: eight lanes per column (b is
+  // column 6), six of them a row each; M is unchanged without new Jacobians.  A segment's row is in
+  // registers before its turn, and a column goes through shuffles: 16 segments 2 us, without Jacobians 1
+  // (3.9 and 2.5 through shared memory with a barrier per segment).
+  if (t < 64 && (kTan || t >= 32)) {
+    const int col = t >> 3, i = (t & 7) < 6 ? t & 7 : 0, first = lane & 24;
+    const bool mine = (t & 7) < 6 && (col == 6 || (kTan && col < 6));
+    double *const out = rec + (col < 6 ? 6 * i + col : 36 + i);
+    double v = i == col ? 1.0 : 0.0, row[6], nrow[6];
+    double r = col == 6 ? sR[0][i] : 0.0, nr = r;
+    load_row(row, &sPhi[0][6 * i]);
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      if (n + 1 < M) {
+        load_row(nrow, &sPhi[n + 1][6 * i]);
+        nr = sR[n + 1][i];
+      }
+      double l[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) l[k] = __shfl_sync(full, v, first + k);
+      const double p = dot6(row, 1, l, 1);
+      v = col == 6 ? r + p : p;
+      if (n == M - 2 && mine) out[42] = v;  // the map up to the last segment's start
+#pragma unroll
+      for (int k = 0; k < 6; ++k) row[k] = nrow[k];
+      r = nr;
     }
-    if (t >= 36 && t < 42) {
-      sB[cur ^ 1][ti] = sR[n][ti] + dot6(&sPhi[n][6 * ti], 1, sB[cur], 1);
-    }
-    __syncthreads();
-    cur ^= 1;
-    if (n == M - 2) {  // the map up to the last segment's start
-      if (kTan && t < 36) rec[42 + t] = sM[cur][t];
-      if (t >= 36 && t < 42) rec[78 + ti] = sB[cur][ti];
-    }
+    if (mine) out[0] = v;
   }
-  if (kTan && t < 36) rec[t] = sM[cur][t];
-  if (t >= 36 && t < 42) rec[36 + ti] = sB[cur][ti];
   if (kTan && t >= 64 && t < 100) rec[84 + t - 64] = sPhi[M - 1][t - 64];
 
   // the last block to finish decides and sweeps (the others' writes are fenced before their ticket)
