@@ -16,7 +16,8 @@
 //          lambda_j0 = M lambda_j1 + b (step_maps_kernel);
 //      (b) one warp carries lambda across the chunk maps from the last point back to the first
 //          (carry_kernel);
-//      (c) each chunk carries its end value across its steps with the stored Jacobians; then all steps run the reverse-mode step from their own lambda at once
+//      (c) each chunk carries its end value across its steps with the stored Jacobians; then all steps run
+//          the reverse-mode step from their own lambda at once
 //          (VJP through the four stages, recomputed from the stored state), which yields the
 //          field-parameter and q/(m gamma) contributions (finish_kernel).
 //    The stored trajectory is itself the checkpoint set: the state at every step is in HBM (the sums
@@ -114,6 +115,40 @@ __device__ void grid_corners(const srs_field &f, V3 XIN, Corners &C) {
   }
 }
 
+// The same for a map along one axis without rotation, the usual one: cell k, the weights of its two samples and
+// the weights' derivatives, as grid_corners forms them, in registers (with its corners in local memory the maps
+// and finish kernels took 38 and 51 us for 20001 points, so 28 and 33).
+struct AxisCorners {
+  int axis;  // -1: not such a map
+  bool inside;
+  int64_t k;
+  double w[2], dw[2];
+};
+__device__ __forceinline__ AxisCorners axis_corners(const srs_field &f, V3 X) {
+  AxisCorners C;
+  C.axis = -1;
+  C.inside = false;
+  if (has_rotation(f.rotations)) return C;
+  if (f.n[0] == 1 && f.n[1] == 1 && f.n[2] > 1) C.axis = 2;
+  else if (f.n[0] == 1 && f.n[1] > 1 && f.n[2] == 1) C.axis = 1;
+  else if (f.n[0] > 1 && f.n[1] == 1 && f.n[2] == 1) C.axis = 0;
+  else return C;
+  const int a = C.axis;
+  const double x = (a == 0 ? X.x : a == 1 ? X.y : X.z) - f.translation[a], start = f.start[a], step = f.step[a];
+  const int64_t n = f.n[a];
+  if (x <= start || x >= start + (double)(n - 1) * step) return C;
+  uint64_t k = (uint64_t)((x - start) / step);
+  if (k > (uint64_t)(n - 2)) k = n - 2;
+  const double t = ((x - start) - (double)k * step) / step;
+  C.inside = true;
+  C.k = (int64_t)k;
+  C.w[0] = 1.0 - t;
+  C.w[1] = t;
+  C.dw[0] = -1.0 / step;
+  C.dw[1] = 1.0 / step;
+  return C;
+}
+
 // Scalar profile of an amplitude field (B = field * shape) and its gradient in X.
 __device__ double amp_shape(const srs_field &f, V3 X, V3 &grad) {
   grad = v3(0, 0, 0);
@@ -174,6 +209,21 @@ __device__ void field_jet(const srs_field *F, int nf, V3 X, V3 &B, double J[3][3
   for (int q = 0; q < nf; ++q) {
     const srs_field &f = F[q];
     if (f.kind == SRS_FIELD_GRID) {
+      const AxisCorners one = axis_corners(f, X);
+      if (one.axis >= 0) {
+        if (!one.inside) continue;
+        const V3 lo = ld3(f.data + 3 * one.k), hi = ld3(f.data + 3 * one.k + 3);
+        B = B + lo * one.w[0];
+        B = B + hi * one.w[1];
+        const double g[3] = {lo.x * one.dw[0] + hi.x * one.dw[1], lo.y * one.dw[0] + hi.y * one.dw[1],
+                             lo.z * one.dw[0] + hi.z * one.dw[1]};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j)
+            if (j == one.axis) J[i][j] += g[i];
+        continue;
+      }
       Corners C;
       grid_corners(f, X, C);
       if (C.nc == 0) continue;
@@ -216,6 +266,17 @@ __device__ void field_param_vjp(const srs_field *F, int nf, V3 X, V3 Bbar, doubl
     if (f.kind == SRS_FIELD_GRID) {
       double *gg = grid_grads ? grid_grads[q] : nullptr;
       if (!gg) continue;
+      const AxisCorners one = axis_corners(f, X);
+      if (one.axis >= 0) {
+        if (one.inside)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            atomicAdd(gg + 3 * (one.k + c) + 0, one.w[c] * Bbar.x);
+            atomicAdd(gg + 3 * (one.k + c) + 1, one.w[c] * Bbar.y);
+            atomicAdd(gg + 3 * (one.k + c) + 2, one.w[c] * Bbar.z);
+          }
+        continue;
+      }
       Corners C;
       grid_corners(f, X, C);
       for (int c = 0; c < C.nc; ++c) {
@@ -363,7 +424,7 @@ constexpr int kJacDoubles = 37 * kAdjBlock + kAdjChunks;
 // (a) J~_j (6 x 6, row = output, column = input, in (x, beta) units) of every step, and the maps of the
 // block's chunks, composed backwards from M = I, b = 0: eight lanes per chunk, one per
 // column of M and one for b.  Bound by the latency of the four stages and six tangents of a step with one
-// warp per scheduler: 20001 points (157 blocks) 38 us, where the Jacobians (36 us) and then the maps of
+// warp per scheduler: 20001 points (157 blocks) 28 us, where the Jacobians (36 us) and then the maps of
 // the chunks by one thread each (41 us) took two kernels.
 __global__ void __launch_bounds__(kAdjBlock) step_maps_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
                                                               Chains C, double *__restrict__ jac,
@@ -506,7 +567,7 @@ __global__ void __launch_bounds__(32) carry_kernel(Traj T, Chains C, const doubl
 }
 
 // (c) per block: lambda at the steps' ends, then the reverse-mode step of every step; the field-parameter and q contributions go to per-block partials (amplitudes, q; a fixed tree) or
-// atomics (grid samples).  Only the 6 x 6 products of 16 steps are serial; 20001 points 51 us (258 when a
+// atomics (grid samples).  Only the 6 x 6 products of 16 steps are serial; 20001 points 33 us (258 when a
 // thread ran the reverse-mode steps of its chunk one after another).
 __global__ void __launch_bounds__(kAdjBlock) finish_kernel(const srs_field *__restrict__ gF, int nf, double q, Traj T,
                                                            Chains C, const double *__restrict__ jac,
@@ -549,7 +610,7 @@ __global__ void __launch_bounds__(kAdjBlock) finish_kernel(const srs_field *__re
   }
   __syncthreads();
   double amp[3 * kAdjMaxFields];
-  for (int i = 0; i < 3 * kAdjMaxFields; ++i) amp[i] = 0.0;
+  for (int i = 0; i < 3 * nf; ++i) amp[i] = 0.0;
   double qb = 0.0;
   if (t < cnt) {
     const double *const lam = lam_g[t];
