@@ -420,9 +420,10 @@ srs_status srs_sim_calculate_efield_time(srs_sim *sim, const double obs[3], doub
  * trajectory.  No counterpart in the reference. */
 srs_status srs_sim_set_trajectory_cache(srs_sim *sim, int32_t enabled);
 /* How the object integrates single-particle trajectories: SRS_TRAJ_AUTO (default) parallel in time
- * (srs_trajectory_shoot) for the mixed-precision sums and serially (srs_trajectory, the reference's
- * roundings) for everything else; SRS_TRAJ_SERIAL always serially; SRS_TRAJ_PARALLEL always parallel
- * in time.  Trajectories shorter than 1024 points and multi-particle batches are always serial.
+ * (srs_trajectory_shoot) for the mixed-precision sums and with the serial chain's bits (srs_trajectory,
+ * the reference's roundings) for everything else; SRS_TRAJ_SERIAL always with the serial chain's bits;
+ * SRS_TRAJ_PARALLEL always parallel in time.  Trajectories shorter than 1024 points and multi-particle
+ * batches always have the serial chain's bits (which the library may form in parallel too).
  * No counterpart in the reference. */
 enum { SRS_TRAJ_AUTO = 0, SRS_TRAJ_SERIAL = 1, SRS_TRAJ_PARALLEL = 2 };
 srs_status srs_sim_set_trajectory_mode(srs_sim *sim, int32_t mode);

@@ -29,7 +29,8 @@
 // Initial guess: straight flight from the initial state.
 //
 // The stored trajectory equals the serial one up to the ulps by which a start state a few ulps away
-// rounds differently (~1e-15 m), not bit for bit; the FP64 drop-in path keeps the serial kernel.
+// rounds differently (~1e-15 m), not bit for bit; the FP64 drop-in path takes the serial bits
+// (rk4_exact.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -27,8 +27,8 @@
 namespace srs {
 namespace {
 
-// Shortest single-particle trajectory integrated parallel in time (below it the serial chain, at
-// ~0.9 us per step, costs about what the shooting iterations' launches do).
+// Shortest single-particle trajectory integrated by shooting (below it the serial chain's bits, ~0.1 ms in
+// parallel or ~0.9 us per step, cost about what the shooting iterations' launches do).
 constexpr int64_t kShootMinPoints = 1024;
 
 // ---------------------------------------------------------------- global random generator
@@ -319,7 +319,7 @@ struct srs_sim {
   }
 
   // RK4 trajectories of a batch of particles that share t0 into device arrays (layout of srs_trajectory).
-  // shoot: one particle, parallel in time (long trajectories only; short ones are cheaper serially).
+  // shoot: one particle, by multiple shooting (long trajectories only); otherwise the serial chain's bits.
   srs_status integrate(const Particle *ps, int np, double *X, double *B, double *A, srs_traj_view &view,
                        bool shoot = false) {
     double dt;

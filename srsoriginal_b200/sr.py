@@ -291,8 +291,8 @@ class sr:  # noqa: N801  (the reference's type name)
 
     def set_trajectory_mode(self, mode="auto"):
         """How single-particle trajectories are integrated: 'auto' (default) parallel in time for the
-        mixed-precision sums and serially, with the reference's roundings, for everything else;
-        'serial' always serially; 'parallel' always parallel in time (multiple shooting: equal to the
+        mixed-precision sums and with the serial chain's bits, the reference's roundings, for everything
+        else; 'serial' always with the serial chain's bits; 'parallel' always parallel in time (multiple shooting: equal to the
         serial trajectory to ~1e-16 m).  Not in the reference."""
         if mode not in self._TRAJ_MODES:
             raise ValueError("'mode' must be one of 'auto', 'serial', 'parallel'")
