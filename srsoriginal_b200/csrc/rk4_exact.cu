@@ -42,7 +42,7 @@
 //
 // Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.17 ms, 40001
 // through two 39.0 -> 0.35 ms, 12001 through a field map in two chains 14.1 -> 0.16 ms, 24 particles of
-// 10001 points 9.1 -> 0.56 ms, 2001 points 1.78 -> 0.13 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by
+// 10001 points 9.1 -> 0.54 ms, 2001 points 1.78 -> 0.13 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by
 // latency (~7 us: launch, loads, four field evaluations, 2 x 128 additions in order); a sweep takes 0.16 ms
 // by the chain kernel on 20001 points, 0.05 ms by runs (20 us per list, 10 us per kernel of blocks).
 #include <cuda_runtime.h>
@@ -57,6 +57,10 @@ namespace srs {
 namespace {
 
 constexpr int kStepsPerBlock = 128;  // steps (and threads) of a pass block
+// Doubles of a component's row in shared memory: the three lanes that add walk on different banks (a third of
+// the wavefronts of a pass were these rows' conflicts; 24 particles of 10001 points 560 -> 540 us, 100 of 20001
+// 3.46 -> 3.29 ms, where the blocks of several waves share an SM's memory pipe).
+constexpr int kRow = kStepsPerBlock + 2;
 constexpr int kChainTile = 256;      // steps per tile of the chain kernel
 constexpr int kChainThreads = 512;
 constexpr int kGroup = 12;           // blocks whose addends the starts kernel holds at a time, one feeding warp each
@@ -367,7 +371,7 @@ template <int kN>
 __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_field *__restrict__ gfields, int nfields,
                                                                   Job J, Scratch W, int pass) {
   __shared__ Fields<kN> fields;
-  __shared__ __align__(16) double sd[3][kStepsPerBlock], sv[3][kStepsPerBlock];
+  __shared__ __align__(16) double sd[3][kRow], sv[3][kRow];
   __shared__ double red[6][kStepsPerBlock / 32];
   wait_for_previous_grid();
   allow_next_grid();
@@ -407,7 +411,9 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
     pos = pos + ld3(shift) + dv * (h * (double)t);
     for (int c = 0; c < 6; ++c) start[c] += shift[c];
   }
-  if (t < 6) T[t] = start[t];
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+    if (t == c) T[c] = start[c];
   __syncthreads();
   Increments o;
   o.d = v3(0, 0, 0);
@@ -443,7 +449,7 @@ template <int kN, bool kRuns>
 __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_field *__restrict__ gfields, int nfields,
                                                                    Job J, Scratch W, int from_passes) {
   __shared__ Fields<kN> fields;
-  __shared__ __align__(16) double sd[3][kRuns ? kStepsPerBlock : 2], sx[3][kRuns ? kStepsPerBlock + 2 : 2];
+  __shared__ __align__(16) double sd[3][kRuns ? kRow : 2], sx[3][kRuns ? kRow : 2];
   __shared__ double red[6][kStepsPerBlock / 32];
   __shared__ int counts[kStepsPerBlock / 32][3];
   wait_for_previous_grid();
@@ -671,7 +677,7 @@ __global__ void __launch_bounds__(kStartsThreads) pit_starts_kernel(Job J, Scrat
 // The velocities from their blocks' start states, the increments of the positions, and the addends of
 // the positions' chain.
 __global__ void __launch_bounds__(kStepsPerBlock) pit_positions_kernel(Job J, Scratch W) {
-  __shared__ __align__(16) double sd[3][kStepsPerBlock], sv[3][kStepsPerBlock];
+  __shared__ __align__(16) double sd[3][kRow], sv[3][kRow];
   __shared__ int counts[kStepsPerBlock / 32][3];
   wait_for_previous_grid();
   allow_next_grid();
