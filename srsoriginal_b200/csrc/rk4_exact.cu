@@ -783,6 +783,12 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
 // bytes of scratch per step and particle (0.7 GB for 256 of 20001 points; 168 by runs) end it before.
 constexpr int64_t kExactMinSteps = 256;
 constexpr int kExactMaxParticles = 256;
+// Longer batches go half by half, so that the scratch kept in the library's pool stays bounded (4 GB: 64 particles of
+// 430000 points at a time; a pass fills the GPU long before).  One particle takes what it needs, up to 2^26
+// steps: every block sums all the mismatches before it, which costs as much as the serial kernel near 10^8
+// (4 million points 0.12 s, serially 3.5 s).
+constexpr size_t kExactMaxScratch = (size_t)4 << 30;
+constexpr int64_t kExactMaxSteps = (int64_t)1 << 26;
 // And only where the iteration contracts: the angle by which the fields could turn a particle over the
 // whole trajectory, |q/(m gamma)| sum |B| T (grids not counted: their samples are on the device).  3 GeV
 // electrons in 1 T over 2 m: 0.2; at 12 (50 MeV) the passes diverge, which costs 0.1-0.2 ms before the
@@ -841,11 +847,24 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
                       electric, d_specs, d_skip);
   };
   const int64_t items = (int64_t)nparticles * J.chains;
-  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles)
+  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles ||
+      (int64_t)J.maxblk * kStepsPerBlock > kExactMaxSteps)
     return serial(nullptr);
   if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) < kExactMaxTurn)) return serial(nullptr);
+  const size_t bytes = carve(J, nfields, nullptr, nullptr);
+  if (bytes > kExactMaxScratch && nparticles > 1) {
+    const int half = nparticles / 2;
+    auto part = [&](int p, int count) {
+      const int64_t at = d_specs ? 0 : (int64_t)p * 3 * (nfwd + nbwd);  // (specs carry their own arrays)
+      return launch_trajectories(d_fields, nfields, d_particles + p, count, dt, nfwd, nbwd, d_x + at, d_b + at, d_a + at,
+                                 d_specs ? d_specs + p : nullptr, host_specs ? host_specs + p : nullptr, s, host_fields,
+                                 host_particles + p);
+    };
+    if (cudaError_t e = part(0, half)) return e;
+    return part(half, nparticles - half);
+  }
   DeviceBuffer scratch;
-  if (scratch.alloc(carve(J, nfields, nullptr, nullptr), s) != cudaSuccess) {
+  if (scratch.alloc(bytes, s) != cudaSuccess) {
     cudaGetLastError();  // no room for the states: the serial kernels need none
     return serial(nullptr);
   }

@@ -108,6 +108,22 @@ def test_chains_by_runs_equal_the_serial_kernel_bitwise(field, particles, npoint
         assert torch.equal(getattr(few, a), getattr(many, a)[:particles]), a
 
 
+def test_batches_beyond_the_scratch_bound_go_half_by_half():
+    import torch
+
+    from srsoriginal_b200 import device as D
+
+    fields, _ = _fields("undulator")
+    parts = [D.ideal_particle(3.0 - 0.01 * i, [1e-6 * i, 0, -1.0], [1e-7 * i, 0, 1])[0] for i in range(5)]
+    n = 6000001  # 5 x 6e6 steps of 144 bytes: 4.3 GB, one particle's 0.9
+    all_ = D.trajectory(fields, parts, 0.0, 2.0, 0.0, n)
+    for i in (0, 2, 4):
+        one = D.trajectory(fields, [parts[i]], 0.0, 2.0, 0.0, n)
+        torch.cuda.synchronize()
+        for a in ("x", "beta", "aoc"):
+            assert torch.equal(getattr(one, a)[0], getattr(all_, a)[i]), (i, a)
+
+
 # Sizes at the edges of the lane kernel: one, two and four particles per warp, the two chains, a last
 # block that is not full.
 @pytest.mark.parametrize("field,particles,npoints,start", [
