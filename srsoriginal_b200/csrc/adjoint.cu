@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "srs_device.cuh"
@@ -718,15 +719,22 @@ __global__ void __launch_bounds__(kSumAdjThreads) spectrum_adjoint_kernel(const 
   // With P = W e^{i w tau}: A = Sum Re P, Bc = Sum (c/w) Im P, Wc = Sum (w/c) Im P; the derivatives of the
   // amplitude and of the phase are linear in them
   double A[3] = {0, 0, 0}, Bc[3] = {0, 0, 0}, Wc[3] = {0, 0, 0};
+  __shared__ BlockBound longest;  // the retarded times
+  longest.set(tau);
   for (int64_t k0 = 0; k0 < ne; k0 += kSumAdjTile) {
     const int cnt = (int)imin64(kSumAdjTile, ne - k0);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * kWeightDoubles; t += blockDim.x) sW[t] = W[kWeightDoubles * k0 + t];
-    __syncthreads();
-    for (int k = threadIdx.x % kSumAdjLanes; k < cnt; k += kSumAdjLanes) {
+    bool far = false;
+    for (int t = threadIdx.x; t < cnt * kWeightDoubles; t += blockDim.x) {
+      const double v = W[kWeightDoubles * k0 + t];
+      sW[t] = v;
+      if (t % kWeightDoubles == 0) far = far || phases_far(v, longest.get());
+    }
+    far = __syncthreads_or(far);
+    auto term = [&](int k, auto is_far) {
       const double *const w = sW + kWeightDoubles * k;
       double sn, cs;
-      sincos_reduced(w[0] * tau, sn, cs);
+      sincos_phase<is_far.value>(w[0] * tau, sn, cs);
       const double cow = w[7], woc = w[8];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -736,7 +744,11 @@ __global__ void __launch_bounds__(kSumAdjThreads) spectrum_adjoint_kernel(const 
         Bc[c] = __fma_rn(cow, pi, Bc[c]);
         Wc[c] = __fma_rn(woc, pi, Wc[c]);
       }
-    }
+    };
+    if (far)
+      for (int k = threadIdx.x % kSumAdjLanes; k < cnt; k += kSumAdjLanes) term(k, std::true_type{});
+    else
+      for (int k = threadIdx.x % kSumAdjLanes; k < cnt; k += kSumAdjLanes) term(k, std::false_type{});
   }
 #pragma unroll
   for (int o = 1; o < kSumAdjLanes; o *= 2) {

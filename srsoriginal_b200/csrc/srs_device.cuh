@@ -257,7 +257,22 @@ __device__ __forceinline__ double reduce_2pi(double x) {
   return r;
 }
 
-// sin and cos of x for |x| < 2^46: x = k pi/2 + r by Cody & Waite's steps (k from the 1.5 * 2^52 shift; a
+// Whether a phase may lie beyond the reduction of sincos_reduced (7.4 MeV at 30 m); NaN too.
+__device__ __forceinline__ bool phases_far(double omega, double tau) { return !(fabs(omega) * fabs(tau) < 0x1p50); }
+
+// An upper bound on the |v| of a block of four warps (from their high words), complete after the next barrier.
+struct BlockBound {
+  int high[4];
+  __device__ __forceinline__ void set(double v) {
+    const int m = __reduce_max_sync(0xffffffffu, __double2hiint(fabs(v)));
+    if ((threadIdx.x & 31) == 0) high[threadIdx.x >> 5] = m;
+  }
+  __device__ __forceinline__ double get() const {
+    return __hiloint2double(max(max(high[0], high[1]), max(high[2], high[3])), -1);
+  }
+};
+
+// sin and cos of x for |x| < 2^50: x = k pi/2 + r by Cody & Waite's steps (k from the 1.5 * 2^52 shift; a
 // third part of pi/2, below |k| * 2e-33, would not be seen), then sin r = r + r^3 S(r^2) and cos r = 1 -
 // r^2/2 + r^4 C(r^2) with S and C the degree-5 interpolants at the Chebyshev nodes of [0, (pi/4)^2] of
 // (sin(r)/r - 1)/r^2 and (cos(r) - 1 + r^2/2)/r^4: 1e-17 and 5e-19 from the functions.
@@ -284,6 +299,16 @@ __device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs)
   const double a = (k & 1) ? c : s, b = (k & 1) ? s : c;
   sn = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(k & 2) << 30), __double2loint(a));
   cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((k + 1) & 2) << 30), __double2loint(b));
+}
+
+// The same for any x: phases beyond 2^50 rad are accepted, though a double holds them to a quarter of a radian
+// only, and reduced first (beyond 2^103 more than once).  A tile is summed this way when a bound on its phases
+// (phases_far) says so: testing every phase cost the sums 5 %.
+template <bool kFar>
+__device__ __forceinline__ void sincos_phase(double x, double &sn, double &cs) {
+  if constexpr (kFar)
+    for (int k = 0; k < 20 && fabs(x) >= 0x1p50; ++k) x = reduce_2pi(x);
+  sincos_reduced(x, sn, cs);
 }
 
 // reduce_2pi in FP32 arithmetic, for arguments of a few hundred radians at most.

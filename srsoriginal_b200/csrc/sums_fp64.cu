@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "splits.h"
 #include "srs_device.cuh"
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
                                                           int64_t n, double dt, const double *__restrict__ pts,
                                                           int64_t np, double omega, int64_t chunk,
                                                           double *__restrict__ partial) {
+  static_assert(kTile == 128, "BlockBound's four warps");
   __shared__ double2 tile[4][kTile];  // (x, y), (z, i dt), (beta_x, beta_y), (beta_z, -)
   wait_for_previous_grid();  // (launched with launch_after)
   allow_next_grid();
@@ -100,27 +102,32 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
   const bool active = j < np;
   V3 obs = active ? v3(pts[3 * j], pts[3 * j + 1], pts[3 * j + 2]) : v3(0, 0, 1);
   const double icow = kC / omega, rc = 1.0 / kC;
+  __shared__ BlockBound reach;  // of the block's points (no distance exceeds |x| + |y| + |z| of both ends)
+  reach.set(fabs(obs.x) + fabs(obs.y) + fabs(obs.z));
   double axr = 0, axi = 0, ayr = 0, ayi = 0, azr = 0, azi = 0;
   for (int64_t base = i0; base < i1; base += kTile) {
     const int cnt = (int)imin64(kTile, i1 - base);
     __syncthreads();
+    bool far = false;
     if (tid < cnt) {
       const int64_t i = base + tid;
-      tile[0][tid] = make_double2(xp[i], xp[n + i]);
-      tile[1][tid] = make_double2(xp[2 * n + i], dt * (double)(int)i);
+      const V3 x = v3(xp[i], xp[n + i], xp[2 * n + i]);
+      const double t = dt * (double)(int)i;
+      tile[0][tid] = make_double2(x.x, x.y);
+      tile[1][tid] = make_double2(x.z, t);
       tile[2][tid] = make_double2(bp[i], bp[n + i]);
       tile[3][tid] = make_double2(bp[2 * n + i], 0.0);
+      far = phases_far(omega, fabs(t) + (fabs(x.x) + fabs(x.y) + fabs(x.z) + reach.get()) * rc);
     }
-    __syncthreads();
+    far = __syncthreads_or(far);
     if (!active) continue;
-#pragma unroll 2
-    for (int k = 0; k < cnt; ++k) {
+    auto term = [&](int k, auto is_far) {
       const double2 q0 = tile[0][k], q1 = tile[1][k], q2 = tile[2][k];
       const double bz = tile[3][k].x;
       const V3 R = obs - v3(q0.x, q0.y, q1.x);
       double m, y, sn, cs;
       sqrt_both(mag2(R), m, y);
-      sincos_reduced(omega * (q1.y + div_rn(m, kC, rc)), sn, cs);
+      sincos_phase<is_far.value>(omega * (q1.y + div_rn(m, kC, rc)), sn, cs);
       // (beta - n)/D e^{i phi} - i (c/w) n/D^2 e^{i phi}, with e^{i phi}/D = (cr, ci)
       const double cr = y * cs, ci = y * sn, f = icow * y * y, fr = f * cr, fi = f * ci;
       const double dx = __fma_rn(-R.x, y, q2.x), dy = __fma_rn(-R.y, y, q2.y), dz = __fma_rn(-R.z, y, bz);
@@ -130,6 +137,13 @@ __global__ void __launch_bounds__(kTile) flux_fp64_kernel(const double *__restri
       ayi = __fma_rn(dy, ci, __fma_rn(-R.y, fr, ayi));
       azr = __fma_rn(dz, cr, __fma_rn(R.z, fi, azr));
       azi = __fma_rn(dz, ci, __fma_rn(-R.z, fr, azi));
+    };
+    if (far) {
+#pragma unroll 1
+      for (int k = 0; k < cnt; ++k) term(k, std::true_type{});
+    } else {
+#pragma unroll 2
+      for (int k = 0; k < cnt; ++k) term(k, std::false_type{});
     }
   }
   if (active) {
@@ -214,35 +228,45 @@ __global__ void __launch_bounds__(kTile) spectrum_fp64_kernel(const double *__re
   const bool active = k < ne;
   const double omega = active ? ev_to_omega(energies[k]) : 1.0;
   const double icow = kC / omega;
+  __shared__ BlockBound top;  // the angular frequencies
+  top.set(omega);
   double a[6] = {0, 0, 0, 0, 0, 0}, b[6] = {0, 0, 0, 0, 0, 0};
   for (int64_t base = i0; base < i1; base += kTile) {
     const int cnt = (int)imin64(kTile, i1 - base);
     __syncthreads();
+    bool far = false;
     if (tid < cnt) {
       const int64_t i = base + tid;
       const V3 R = obs - v3(xp[i], xp[n + i], xp[2 * n + i]);
       double m, y;
       sqrt_both(mag2(R), m, y);
-      const double y2 = y * y, y3 = y2 * y;
-      tile[0][tid] = make_double2(dt * (double)(int)i + div_rn(m, kC, 1.0 / kC), __fma_rn(-R.x, y, bp[i]) * y);
+      const double y2 = y * y, y3 = y2 * y, tau = dt * (double)(int)i + div_rn(m, kC, 1.0 / kC);
+      far = phases_far(top.get(), tau);
+      tile[0][tid] = make_double2(tau, __fma_rn(-R.x, y, bp[i]) * y);
       tile[1][tid] = make_double2(__fma_rn(-R.y, y, bp[n + i]) * y, __fma_rn(-R.z, y, bp[2 * n + i]) * y);
       tile[2][tid] = make_double2(R.x * y3, R.y * y3);
       tile[3][tid] = make_double2(R.z * y3, 0.0);
     }
-    __syncthreads();
+    far = __syncthreads_or(far);
     if (!active) continue;
-#pragma unroll 2
-    for (int q = 0; q < cnt; ++q) {
+    auto term = [&](int q, auto is_far) {
       const double2 q0 = tile[0][q], q1 = tile[1][q], q2 = tile[2][q];
       const double bz = tile[3][q].x;
       double sn, cs;
-      sincos_reduced(omega * q0.x, sn, cs);
+      sincos_phase<is_far.value>(omega * q0.x, sn, cs);
       a[0] = __fma_rn(q0.y, cs, a[0]); a[1] = __fma_rn(q0.y, sn, a[1]);
       a[2] = __fma_rn(q1.x, cs, a[2]); a[3] = __fma_rn(q1.x, sn, a[3]);
       a[4] = __fma_rn(q1.y, cs, a[4]); a[5] = __fma_rn(q1.y, sn, a[5]);
       b[0] = __fma_rn(q2.x, cs, b[0]); b[1] = __fma_rn(q2.x, sn, b[1]);
       b[2] = __fma_rn(q2.y, cs, b[2]); b[3] = __fma_rn(q2.y, sn, b[3]);
       b[4] = __fma_rn(bz, cs, b[4]); b[5] = __fma_rn(bz, sn, b[5]);
+    };
+    if (far) {
+#pragma unroll 1
+      for (int q = 0; q < cnt; ++q) term(q, std::true_type{});
+    } else {
+#pragma unroll 2
+      for (int q = 0; q < cnt; ++q) term(q, std::false_type{});
     }
   }
   if (active) {

@@ -52,3 +52,28 @@ def test_fp64_sums_against_the_oracle(npoints, nout):
             ref = O.power_density(X, B, A, t.dt, pts, nrm, bool(directional), -O.QE, 0.5)
             got = out.cpu().numpy()
             assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+# Phases around the end of the fast reduction (2^50 rad is 7.4 MeV at 30 m) and far beyond it
+@pytest.mark.parametrize("energies", [[7.0e6, 7.3e6, 7.5e6, 9.0e6], [1.0e5, 3.0e7, 1.0e9], [1.0e15, 2.0e20]])
+def test_fp64_sums_at_extreme_phases(energies):
+    import oracle as O
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+
+    t, (X, B, _) = _trajectory(1000)
+    e = np.array(energies)
+    de = torch.tensor(e, device="cuda")
+    out = torch.empty(len(e), dtype=torch.float64, device="cuda")
+    D.spectrum(t, -D.QE, 0.5, [1e-3, 2e-3, 30.0], de, out, precision=_lib.FP64)
+    got = out.cpu().numpy()
+    assert np.all(np.isfinite(got))
+    if e.max() < 1e12:  # beyond, k of the reduction itself has no room in a double
+        assert _normwise(got, O.spectrum(X, B, t.dt, [1e-3, 2e-3, 30.0], e, -O.QE, 0.5)) < TOL
+    pts = np.array([[1e-3, -2e-3, 30.0], [0.0, 5e-3, 28.0]])
+    D.flux(t, -D.QE, 0.5, float(e[-1]), out[:2], points=torch.tensor(pts.reshape(-1), device="cuda"), precision=_lib.FP64)
+    got = out[:2].cpu().numpy()
+    assert np.all(np.isfinite(got))
+    if e.max() < 1e12:
+        assert _normwise(got, O.flux(X, B, t.dt, pts, float(e[-1]), -O.QE, 0.5)) < TOL
