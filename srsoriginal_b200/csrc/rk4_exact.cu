@@ -833,11 +833,16 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
   const int64_t stage_doubles = nfields > 0 ? grid_stage_doubles(host_fields, nfields) : 0;
   const bool electric = has_electric(host_fields, nfields);
-  double time = dt * (double)(nfwd + nbwd);
+  double time = dt * (double)(nfwd + nbwd), step = dt;
   if (host_specs)
-    for (int p = 0; p < nparticles; ++p)
+    for (int p = 0; p < nparticles; ++p) {
       time = std::max(time, host_specs[p].dt * (double)(host_specs[p].nfwd + host_specs[p].nbwd));
-  const int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time);
+      step = std::max(step, host_specs[p].dt);
+    }
+  // (the undulators' phases are bounded by the way light goes: a step that turns the velocity by less than a
+  // radian does not lengthen it; RK4 grows beyond 2.8)
+  int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time);
+  if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
   const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
   if (undulators && nparticles > kExactMaxParticles)
     return launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x, d_b, d_a,

@@ -145,3 +145,21 @@ def test_many_particles_equal_the_serial_kernel_bitwise(field, particles, npoint
     torch.cuda.synchronize()
     for a in ("x", "beta", "aoc"):
         assert torch.equal(getattr(got, a), getattr(ref, a)), a
+
+
+# What the lane kernel's phase bound does not cover takes the serial kernel: steps that turn the velocity by more
+# than a radian (RK4 grows without bound beyond 2.8), a particle faster than light
+@pytest.mark.parametrize("energy,npoints,faster", [(0.02, 60, 1.0), (0.005, 30, 1.0), (3.0, 500, 5.0)])
+def test_batches_beyond_the_phase_bound_equal_the_serial_kernel_bitwise(energy, npoints, faster):
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+
+    und = D.undulator([0, 3.0, 0], [0, 0, 0.049], 31)
+    part, _ = D.ideal_particle(energy, [0, 0, -1.0], [1e-4, 0, 1])
+    part.beta0 = _lib.v3([faster * b for b in part.beta0])
+    a = D.trajectory([und], [part] * MANY, 0.0, 2.0, 0.0, npoints)
+    b = D.trajectory([und] + _fields("nothing")[0], [part] * MANY, 0.0, 2.0, 0.0, npoints)
+    torch.cuda.synchronize()
+    for k in ("x", "beta", "aoc"):
+        assert torch.equal(torch.nan_to_num(getattr(a, k), nan=7.0), torch.nan_to_num(getattr(b, k), nan=7.0)), k
