@@ -94,6 +94,13 @@ __device__ __forceinline__ bool along_axis(const Prepared &p, V3 X, double &x) {
   return !(x <= p.b_lo || x >= p.b_hi);
 }
 
+// The cell (0 .. last) of the quotient q by the step, as grid_interp limits it.  A position that is not a number
+// passes along_axis (both of its comparisons are false); its q is in no cell and takes the last one, whose samples
+// it then only multiplies into a NaN.  (A conversion to int alone would give INT_MIN.)
+__host__ __device__ __forceinline__ int axis_cell(double q, int last) {
+  return !(q < (double)last) ? last : q > 0.0 ? (int)q : 0;
+}
+
 __device__ inline V3 field_one(const Prepared &p, const srs_field &f, V3 X) {
   switch (p.kind) {
     case SRS_FIELD_UNDULATOR: {
@@ -135,9 +142,9 @@ __device__ __forceinline__ V3 field_along(const Prepared &p, const srs_field &f,
   if (p.kind < kGridAlong) return field_one(p, f, X);
   double x;
   if (!along_axis(p, X, x)) return v3(0, 0, 0);
-  const int k = (int)div_rn(x - p.b_lo, p.plen, p.rplen);
-  const double d = (x - p.b_lo) - (double)k * p.plen;
-  const double *const at = p.gd + 3 * (int64_t)min(k, (int)p.taper);
+  const double q = div_rn(x - p.b_lo, p.plen, p.rplen);
+  const double d = (x - p.b_lo) - trunc(q) * p.plen;  // (grid_interp limits the cell after this)
+  const double *const at = p.gd + 3 * (int64_t)axis_cell(q, (int)p.taper);
   const V3 lo = ld3(at), t = (ld3(at + 3) - lo) * d;  // grid_lerp
   return lo + v3(div_rn(t.x, p.plen, p.rplen), div_rn(t.y, p.plen, p.rplen), div_rn(t.z, p.plen, p.rplen));
 }
@@ -308,7 +315,7 @@ __device__ inline void field_one_jac(const Prepared &p, const srs_field &f, V3 X
       double x;
       if (!along_axis(p, X, x)) return;
       const double r = p.rplen;
-      const double *const at = p.gd + 3 * (int64_t)min((int)((x - p.b_lo) * r), (int)p.taper);
+      const double *const at = p.gd + 3 * (int64_t)axis_cell((x - p.b_lo) * r, (int)p.taper);
       const V3 lo = ld3(at), hi = ld3(at + 3);
       const float g[3] = {(float)(lo.x * -r + hi.x * r), (float)(lo.y * -r + hi.y * r), (float)(lo.z * -r + hi.z * r)};
 #pragma unroll
