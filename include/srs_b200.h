@@ -113,6 +113,15 @@ srs_status srs_trajectory(const srs_field *fields, int32_t nfields, const srs_pa
                           int32_t nparticles, double ctstart, double ctstop, double t0, int64_t npoints,
                           double *d_x, double *d_beta, double *d_aoc, void *stream);
 
+/* The same, and how each particle was integrated (the results are the same bits on every way): d_route, a
+ * DEVICE array of nparticles int32, gets SERIAL (one chain), PARALLEL (in time, every step verified), GIVEN_UP
+ * (in time without getting there, then serially) or LANES (one particle per lane).  A check for tests and tuning;
+ * srs_trajectory takes the same ways. */
+enum { SRS_TRAJ_ROUTE_SERIAL = 0, SRS_TRAJ_ROUTE_PARALLEL = 1, SRS_TRAJ_ROUTE_GIVEN_UP = 2, SRS_TRAJ_ROUTE_LANES = 3 };
+srs_status srs_trajectory_route(const srs_field *fields, int32_t nfields, const srs_particle *particles,
+                                int32_t nparticles, double ctstart, double ctstop, double t0, int64_t npoints,
+                                double *d_x, double *d_beta, double *d_aoc, int32_t *d_route, void *stream);
+
 /* The trajectory of ONE particle, integrated parallel in time: the serial RK4 chain is cut into
  * segments of steps_per_segment steps (0 = automatic) whose start states are found by Newton
  * iterations of multiple shooting, every segment stepping with the same arithmetic as srs_trajectory.

@@ -15,6 +15,7 @@ SRS_OK, SRS_ERR_INVALID, SRS_ERR_RANGE, SRS_ERR_CUDA, SRS_ERR_NO_DEVICE, SRS_ERR
 UNDULATOR, GAUSSIAN, UNIFORM_BOX, GRID = 1, 2, 3, 4
 ELECTRIC = 0x100  # kind flag of an electric field
 FP64, MIXED = 0, 1
+ROUTE_SERIAL, ROUTE_PARALLEL, ROUTE_GIVEN_UP, ROUTE_LANES = range(4)  # srs_trajectory_route
 
 _D = C.POINTER(C.c_double)
 _V3 = C.c_double * 3
@@ -87,6 +88,8 @@ def _load():
                                       C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
         "srs_trajectory": (S, [C.POINTER(Field), C.c_int32, C.POINTER(Particle), C.c_int32, C.c_double,
                                C.c_double, C.c_double, C.c_int64, P, P, P, P]),
+        "srs_trajectory_route": (S, [C.POINTER(Field), C.c_int32, C.POINTER(Particle), C.c_int32, C.c_double,
+                                     C.c_double, C.c_double, C.c_int64, P, P, P, P, P]),
         "srs_trajectory_shoot": (S, [C.POINTER(Field), C.c_int32, C.POINTER(Particle), C.c_double, C.c_double,
                                      C.c_double, C.c_int64, C.c_int32, C.c_int32, P, P, P, P, P]),
         "srs_spectrum": (S, [TrajView, BeamConsts, _D, P, C.c_int64, C.c_int32, P, P]),
@@ -180,7 +183,7 @@ def _load():
 
 lib = _load()
 EXPORTED = (
-    "srs_last_error srs_version srs_device_count srs_trim_memory srs_trajectory_counts srs_trajectory srs_trajectory_shoot srs_spectrum "
+    "srs_last_error srs_version srs_device_count srs_trim_memory srs_trajectory_counts srs_trajectory srs_trajectory_route srs_trajectory_shoot srs_spectrum "
     "srs_flux srs_power_density srs_total_power srs_accumulate srs_sim_create srs_sim_destroy "
     "srs_sim_set_ctstartstop srs_sim_set_npoints_trajectory srs_sim_get_ctstartstop "
     "srs_sim_get_npoints_trajectory srs_sim_set_nthreads_global srs_sim_set_gpu_global "

@@ -106,6 +106,13 @@ srs_status srs_trajectory_counts(double ctstart, double ctstop, double t0, int64
 srs_status srs_trajectory(const srs_field *fields, int32_t nfields, const srs_particle *particles,
                           int32_t nparticles, double ctstart, double ctstop, double t0, int64_t npoints,
                           double *d_x, double *d_beta, double *d_aoc, void *stream) {
+  return srs_trajectory_route(fields, nfields, particles, nparticles, ctstart, ctstop, t0, npoints, d_x, d_beta, d_aoc,
+                              nullptr, stream);
+}
+
+srs_status srs_trajectory_route(const srs_field *fields, int32_t nfields, const srs_particle *particles,
+                                int32_t nparticles, double ctstart, double ctstop, double t0, int64_t npoints,
+                                double *d_x, double *d_beta, double *d_aoc, int32_t *d_route, void *stream) {
   clear_error();
   double dt;
   int64_t nf, nb;
@@ -124,7 +131,7 @@ srs_status srs_trajectory(const srs_field *fields, int32_t nfields, const srs_pa
   if (nfields > 0) SRS_CUDA(cudaMemcpyAsync(df.ptr, fields, sizeof(srs_field) * nfields, cudaMemcpyHostToDevice, s));
   SRS_CUDA(cudaMemcpyAsync(dp.ptr, particles, sizeof(srs_particle) * nparticles, cudaMemcpyHostToDevice, s));
   SRS_CUDA(launch_trajectories(df.as<srs_field>(), nfields, dp.as<srs_particle>(), nparticles, dt, nf, nb, d_x, d_beta,
-                               d_aoc, nullptr, nullptr, s, fields, particles));
+                               d_aoc, nullptr, nullptr, s, fields, particles, d_route));
   return SRS_OK;
 }
 

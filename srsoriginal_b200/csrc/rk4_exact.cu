@@ -66,7 +66,14 @@ constexpr int kChainThreads = 512;
 constexpr int kGroup = 12;           // blocks whose addends the starts kernel holds at a time, one feeding warp each
 constexpr int kStartsThreads = 32 * (kGroup + 1);
 constexpr int kPasses = 14;          // passes launched (they return at once when the item is ready)
-constexpr int kContracted = 4;       // by this pass a contracting iteration is far below 1e-4 of the speed
+// When an item is given up: the first pass adds up the turns that the fields give on straight flight, and beyond
+// kMaxTurn the iteration does not get to the exact bits within the passes and sweeps below; or, where straight
+// flight misses the fields, mismatches above kLostMismatch of the speed are left after pass kContracted or a later
+// one.  (Lists of undulators along z alone are not summed up: the host knows their strength.)  Measured
+// for 300, 2001 and 20001 points in an undulator, a map of one and a map of a dipole: all settle up to a turn of
+// 1.0, at 1.2 five of nine, at 1.5 none; after pass 4 at most 9e-3 is left of those that settle.
+constexpr double kMaxTurn = 1.3, kLostMismatch = 0.03;
+constexpr int kContracted = 4;
 constexpr int kSweeps = 4;           // exact sweeps before the serial kernel takes over
 // Chains by runs from this length: a sweep of the chain kernel takes 7.8 ns per step of the longest chain
 // (1 or 24 particles alike), one by runs ~40 us, 1.5 ns per step and ~20 ns per block of all particles.
@@ -109,7 +116,8 @@ struct Scratch {
   int *ready;                 // per item: the pass that found nothing left to settle, or kPasses
   int *done, *all_ticket;     // the whole job verified; blocks of the steps kernel finished
   unsigned long long *bad;    // steps that do not reproduce (reset by the last block)
-  int *failed;                // an item whose passes did not converge
+  int *failed;                // an item was given up
+  float *turn;                // per item: sum |d| of the first pass
   Prepared *prep;
   UndField *und;
   // of pass k.  Selected: an index puts the kernel's argument on the stack of every thread (120 bytes; 24 particles
@@ -314,7 +322,10 @@ __global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ 
     *W.bad = 0;
     *W.failed = 0;
   }
-  if (g < items) W.ready[g] = kPasses;
+  if (g < items) {
+    W.ready[g] = kPasses;
+    W.turn[g] = 0.0f;
+  }
   if (g >= (int64_t)items * J.maxblk) return;
   const int it = (int)(g / J.maxblk), s = (int)(g - (int64_t)it * J.maxblk);
   const Item I = item_of(J, it);
@@ -329,7 +340,7 @@ __global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ 
 // shift[0..2] of its start position, shift[3..5] of its start velocity (a velocity shift moves the
 // positions of all later blocks).  Every thread gets them; returns whether the item has settled: the
 // transverse mismatches at the rounding of the speed and none in a component that carries the flight
-// (its bits decide the phases); lost: the mismatches are far above that.
+// (its bits decide the phases); lost: some are above kLostMismatch.
 __device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I, int it, int s, int k,
                                   double (*red)[kStepsPerBlock / 32], double shift[6], bool *lost) {
   const double *const T = W.starts(k) + 6 * (int64_t)it * J.maxblk, *const E = W.ends(k) + 6 * (int64_t)it * J.maxblk;
@@ -361,13 +372,14 @@ __device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I,
     for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
   if ((threadIdx.x & 31) == 0)
     for (int c = 0; c < 6; ++c) red[c][threadIdx.x >> 5] = sum[c];
-  open = __syncthreads_or((open || big2 > 1e-32 * v2 ? 1 : 0) | (big2 < 1e-8 * v2 ? 0 : 2));
+  const int any = __syncthreads_or(open || big2 > 1e-32 * v2);
   for (int c = 0; c < 6; ++c) {
     shift[c] = 0.0;
     for (int w = 0; w < kStepsPerBlock / 32; ++w) shift[c] += red[c][w];
   }
-  *lost = (open & 2) != 0;
-  return open == 0;
+  // (a barrier of its own: __syncthreads_or returns whether any argument was not zero, not their bits)
+  *lost = k >= kContracted && __syncthreads_or(big2 > kLostMismatch * kLostMismatch * v2);
+  return !any;
 }
 
 // Picard iteration number `pass` (see the file comment); in the first the states are straight flight.
@@ -383,6 +395,7 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   // as the passes before this one left it (in this pass other blocks may be writing ready = pass - 1, and all
   // threads of a block have to decide alike)
   const bool settled = W.ready[it] + 1 < pass;
+  const float turn = kN == 0 && pass == 1 ? W.turn[it] : 0.0f;
   const Item I = item_of(J, it);
   const int64_t blk = (int64_t)it * J.maxblk + s, i = (int64_t)s * kStepsPerBlock + t;
   fields.load(gfields, W, nfields);
@@ -402,8 +415,12 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
     double shift[6];
     bool lost;
     const bool ready = mismatches(J, W, I, it, s, pass - 1, red, shift, &lost);
-    if (lost && pass > kContracted) {
-      if (t == 0) W.ready[it] = pass - 1, *W.failed = 1;
+    if (lost || (kN == 0 && turn > (float)kMaxTurn * sqrtf((float)mag2(ld3(I.s0 + 3))))) {
+      // all items go to the serial kernel: no further pass of any (one that has settled keeps its number, which
+      // its blocks are reading)
+      for (int q = t; q < (int)gridDim.y; q += kStepsPerBlock)
+        if (W.ready[q] == kPasses) W.ready[q] = pass - 1;
+      if (t == 0) *W.failed = 1;
       return;
     }
     if (ready) {
@@ -422,10 +439,18 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   Increments o;
   o.d = v3(0, 0, 0);
   if (active) o = fields.step(nfields, I.qomg, h, hh, h6, pos, vel);
+  if (kN == 0 && pass == 0) {  // (its order does not matter: it decides how the same bits are reached)
+    float turn = sqrtf((float)mag2(o.d));
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) turn += __shfl_xor_sync(0xffffffffu, turn, k);
+    if ((t & 31) == 0) red[0][t >> 5] = turn;
+  }
   sd[0][t] = o.d.x;
   sd[1][t] = o.d.y;
   sd[2][t] = o.d.z;
   __syncthreads();
+  if (kN == 0 && pass == 0 && t == kStepsPerBlock - 1)
+    atomicAdd(W.turn + it, (float)(red[0][0] + red[0][1] + red[0][2] + red[0][3]));
   // the block's steps in order from its start state: velocities, then positions (three lanes)
   if (t < 3) E[3 + t] = add_in_order(t == 0 ? start[3] : t == 1 ? start[4] : start[5], sd[t], sv[t], kStepsPerBlock);
   __syncthreads();
@@ -723,6 +748,11 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_positions_kernel(Job J, Sc
   emit_addends(J, W, it, s, active, pos, d, position_tolerance(I), counts);
 }
 
+__global__ void route_kernel(int32_t *route, int nparticles, const int *done) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < nparticles) route[p] = !done ? SRS_TRAJ_ROUTE_LANES : *done ? SRS_TRAJ_ROUTE_PARALLEL : SRS_TRAJ_ROUTE_GIVEN_UP;
+}
+
 Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const TrajSpec *h_specs, int nparticles, double dt,
              int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a) {
   Job J;
@@ -772,6 +802,7 @@ size_t carve(const Job &J, int nfields, void *base, Scratch *W) {
   s.done = (int *)take(sizeof(int));
   s.all_ticket = (int *)take(sizeof(int));
   s.failed = (int *)take(sizeof(int));
+  s.turn = (float *)take(sizeof(float) * items);
   s.bad = (unsigned long long *)take(sizeof(unsigned long long));
   s.prep = (Prepared *)take(sizeof(Prepared) * (size_t)std::max(1, nfields));
   s.und = (UndField *)take(sizeof(UndField) * kMaxUndulators);
@@ -795,9 +826,11 @@ constexpr size_t kExactMaxScratch = (size_t)4 << 30;
 constexpr int64_t kExactMaxSteps = (int64_t)1 << 26;
 // And only where the iteration contracts: the angle by which the fields could turn a particle over the
 // whole trajectory, |q/(m gamma)| sum |B| T (grids not counted: their samples are on the device).  3 GeV
-// electrons in 1 T over 2 m: 0.2; at 12 (50 MeV) the passes diverge, which costs 0.1-0.2 ms before the
-// serial kernel takes over.
-constexpr double kExactMaxTurn = 3.0;
+// electrons in 1 T over 2 m: 0.2.  Through an undulator at 2.0 300, 2001 and 20001 points settle, at 2.4 two of
+// the three do not; other shapes may fill a part of the way only.  What is given up after the first pass costs 45 to
+// 75 us before the serial kernel (0.1 GeV through a 1 T map: 300 points 375 -> 449 us, 2001 2317 -> 2380; when all
+// passes and sweeps ran for it, 537 and 2518).
+constexpr double kExactMaxTurn = 3.0, kExactMaxTurnUndulators = 2.2;
 
 static double turn_bound(const srs_field *fields, int nfields, const srs_particle *particles, int nparticles, double time) {
   double b = 0.0, q = 0.0;
@@ -832,9 +865,14 @@ static cudaError_t launch_exact(const Job &J, const Scratch &W, const srs_field 
 cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                                 double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
                                 const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,
-                                const srs_field *host_fields, const srs_particle *host_particles) {
+                                const srs_field *host_fields, const srs_particle *host_particles, int32_t *d_route) {
   if (nparticles <= 0) return cudaSuccess;
   if (nfields > kMaxFieldsShared) return cudaErrorInvalidValue;
+  auto routed = [&](cudaError_t e, const int *done) {  // (after the launches that it tells about)
+    if (e != cudaSuccess || !d_route) return e;
+    route_kernel<<<(unsigned)((nparticles + 127) / 128), 128, 0, s>>>(d_route, nparticles, done);
+    return cudaGetLastError();
+  };
   const int64_t stage_doubles = nfields > 0 ? grid_stage_doubles(host_fields, nfields) : 0;
   const bool electric = has_electric(host_fields, nfields);
   double time = dt * (double)(nfwd + nbwd), step = dt;
@@ -849,9 +887,12 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
   const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
   if (undulators && nparticles > kExactMaxParticles)
-    return launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x, d_b, d_a,
-                            d_specs, s);
+    return routed(launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x,
+                                   d_b, d_a, d_specs, s),
+                  nullptr);
   auto serial = [&](const int *d_skip) {
+    if (d_route && !d_skip)
+      if (cudaError_t e = cudaMemsetAsync(d_route, 0, sizeof(int32_t) * (size_t)nparticles, s)) return e;
     return launch_rk4(d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles,
                       electric, d_specs, d_skip);
   };
@@ -859,7 +900,9 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles ||
       (int64_t)J.maxblk * kStepsPerBlock > kExactMaxSteps)
     return serial(nullptr);
-  if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) < kExactMaxTurn)) return serial(nullptr);
+  if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) <
+        (undulators ? kExactMaxTurnUndulators : kExactMaxTurn)))
+    return serial(nullptr);
   const size_t bytes = carve(J, nfields, nullptr, nullptr);
   if (bytes > kExactMaxScratch && nparticles > 1) {
     const int half = nparticles / 2;
@@ -867,7 +910,7 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
       const int64_t at = d_specs ? 0 : (int64_t)p * 3 * (nfwd + nbwd);  // (specs carry their own arrays)
       return launch_trajectories(d_fields, nfields, d_particles + p, count, dt, nfwd, nbwd, d_x + at, d_b + at, d_a + at,
                                  d_specs ? d_specs + p : nullptr, host_specs ? host_specs + p : nullptr, s, host_fields,
-                                 host_particles + p);
+                                 host_particles + p, d_route ? d_route + p : nullptr);
     };
     if (cudaError_t e = part(0, half)) return e;
     return part(half, nparticles - half);
@@ -887,7 +930,7 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
                                           : launch_exact<0>(J, W, d_fields, nfields, grid, s);
   if (e != cudaSuccess) return e;
   if (cudaError_t e = cudaGetLastError()) return e;
-  return serial(W.done);  // returns at once when the check held
+  return routed(serial(W.done), W.done);  // the serial kernel returns at once when the check held
 }
 
 }  // namespace srs

@@ -124,11 +124,12 @@ cudaError_t launch_rk4_lanes(int undulators, const srs_field *d_fields, int nfie
                              double *d_a, const TrajSpec *d_specs, cudaStream_t s);
 // launch_rk4's trajectories bit for bit by the fastest way: few particles parallel in time (rk4_exact.cu),
 // many through undulators one per lane (rk4_lanes.cu), the rest launch_rk4.  host_*: the host copies of the
-// device arrays.
+// device arrays; d_route (optional): per particle the SRS_TRAJ_ROUTE_* that it took.
 cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
                                 double dt, int64_t nfwd, int64_t nbwd, double *d_x, double *d_b, double *d_a,
                                 const TrajSpec *d_specs, const TrajSpec *host_specs, cudaStream_t s,
-                                const srs_field *host_fields, const srs_particle *host_particles);
+                                const srs_field *host_fields, const srs_particle *host_particles,
+                                int32_t *d_route = nullptr);
 // One particle parallel in time (rk4_shoot.cu); scratch of shoot_scratch_bytes bytes.
 int shoot_default_steps(int64_t nsteps);
 size_t shoot_scratch_bytes(int64_t nfwd, int64_t nbwd, int steps_per_segment, int nfields);
