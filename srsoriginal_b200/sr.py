@@ -540,9 +540,11 @@ class sr:  # noqa: N801  (the reference's type name)
     def _surface_arrays(points, rot, tr, invert_normal):
         """The same for a regular list of N pairs of three numbers, operation by operation on arrays (2347
         points: 4.6 -> 1.0 ms); None for anything else, which the loop accepts or refuses item by item."""
+        if isinstance(points, np.ma.MaskedArray):
+            return None
         try:
             a = np.asarray(points)
-        except (TypeError, ValueError):
+        except Exception:  # noqa: BLE001  (ragged lists, tensors that require a gradient, ...: the loop decides)
             return None
         if a.ndim != 3 or a.shape[0] < 1 or a.shape[1:] != (2, 3) or a.dtype.kind not in "fiub":
             return None
