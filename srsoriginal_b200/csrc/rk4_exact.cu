@@ -48,6 +48,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "rk4_fields.cuh"
 #include "rk4_und.cuh"
@@ -836,7 +837,10 @@ static double turn_bound(const srs_field *fields, int nfields, const srs_particl
   double b = 0.0, q = 0.0;
   for (int f = 0; f < nfields; ++f)
     if (field_shape(fields[f].kind) != SRS_FIELD_GRID) b += mag(ld3(fields[f].field));
-  for (int p = 0; p < nparticles; ++p) q = std::max(q, fabs(particles[p].qomg));
+  for (int p = 0; p < nparticles; ++p) {
+    if (std::isnan(particles[p].qomg)) return particles[p].qomg;  // (no bound: std::max would drop it)
+    q = std::max(q, fabs(particles[p].qomg));
+  }
   return q * b * time;
 }
 

@@ -154,7 +154,7 @@ int undulators_along_z(const srs_field *f, int nfields, const srs_particle *part
   double far = kC * time;  // |z| stays below
   for (int p = 0; p < nparticles; ++p) {
     const double *const b = particles[p].beta0;
-    if (!(b[0] * b[0] + b[1] * b[1] + b[2] * b[2] <= 1.0 + 1e-9)) return 0;
+    if (!(b[0] * b[0] + b[1] * b[1] + b[2] * b[2] <= 1.0 + 1e-9) || !std::isfinite(particles[p].x0[2])) return 0;
     far = std::max(far, kC * time + std::fabs(particles[p].x0[2]));
   }
   for (int i = 0; i < nfields; ++i) {

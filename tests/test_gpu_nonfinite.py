@@ -48,3 +48,27 @@ def test_maps_with_a_sample_that_is_no_number(axis, value, npoints, start):
         assert _same(getattr(exact, a)[0], getattr(many, a)[MANY - 1]), a
     for a in ("x", "beta"):  # (a segment's first a/c is formed from the segment before it, NaN or not)
         assert torch.equal(getattr(shoot, a)[0].isnan(), getattr(many, a)[MANY - 1].isnan()), a
+
+
+# A start height or a charge that is no number, alone and in a batch: the undulator kernels' sines take both for
+# finite, so such calls take the serial kernel.
+@pytest.mark.parametrize("field", ["undulator", "epu"])
+@pytest.mark.parametrize("particles", [1, MANY])
+@pytest.mark.parametrize("what", ["z nan", "z inf", "charge nan"])
+def test_starts_that_are_no_numbers(field, particles, what):
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+
+    fields = _fields(field)[0]
+    part, _ = D.ideal_particle(3.0, [1e-5, -2e-5, -1.0], [3e-6, -5e-6, 1])
+    odd = _lib.Particle(part.x0, part.beta0, float("nan") if what == "charge nan" else part.qomg)
+    if what != "charge nan":
+        odd.x0[2] = float(what.split()[1])
+    parts = [part] * (particles - 1) + [odd]
+    got = D.trajectory(fields, parts, 0.0, 2.0, 0.0, 601)
+    ref = D.trajectory(fields + _fields("nothing")[0], [part] * (MANY - particles) + parts, 0.0, 2.0, 0.0, 601)
+    torch.cuda.synchronize()
+    assert not ref.x[-1].isfinite().all()
+    for a in ("x", "beta", "aoc"):
+        assert _same(getattr(got, a), getattr(ref, a)[-particles:]), a
