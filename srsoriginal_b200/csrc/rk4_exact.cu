@@ -105,6 +105,7 @@ struct Job {
   int64_t stride;          // doubles per component of an item's states
   int maxblk;              // pass blocks of the longest chain
   bool by_runs;            // the chains' additions by runs (kRunsMinSteps)
+  double reach;            // with undulators: a bound on |z| within which their phases are below 1e5
 };
 
 struct Scratch {
@@ -199,7 +200,11 @@ struct Fields {
     long long *b = reinterpret_cast<long long *>(und);
     for (int k = threadIdx.x; k < kN * (int)(sizeof(UndField) / 8); k += blockDim.x) b[k] = a[k];
   }
-  __device__ __forceinline__ Increments step(int, double qomg, double h, double hh, double h6, V3 pos, V3 vel) const {
+  // An iterate may lie anywhere, or be no number, where a trajectory's state does not: one out of reach, or faster
+  // than any particle, is not stepped, and fails the check.
+  __device__ __forceinline__ Increments step(int, const Job &J, double qomg, double h, double hh, double h6, V3 pos,
+                                             V3 vel) const {
+    if (!(fabs(pos.z) < J.reach) || !(mag2(vel) < 1.05 * kC * kC)) pos.z = vel.x = vel.y = vel.z = 0.0;
     return und_increments<kN>(und, qomg, h, hh, h6, pos, vel);
   }
 };
@@ -210,7 +215,7 @@ struct Fields<0> {
   __device__ __forceinline__ void load(const srs_field *gf, const Scratch &W, int nfields) {
     copy_fields(sf, sp, gf, W.prep, nfields);
   }
-  __device__ __forceinline__ Increments step(int nfields, double qomg, double h, double hh, double h6, V3 pos,
+  __device__ __forceinline__ Increments step(int nfields, const Job &, double qomg, double h, double hh, double h6, V3 pos,
                                              V3 vel) const {
     return increments(sp, sf, nfields, qomg, h, hh, h6, pos, vel);
   }
@@ -439,7 +444,7 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
   __syncthreads();
   Increments o;
   o.d = v3(0, 0, 0);
-  if (active) o = fields.step(nfields, I.qomg, h, hh, h6, pos, vel);
+  if (active) o = fields.step(nfields, J, I.qomg, h, hh, h6, pos, vel);
   if (kN == 0 && pass == 0) {  // (its order does not matter: it decides how the same bits are reached)
     float turn = sqrtf((float)mag2(o.d));
 #pragma unroll
@@ -535,7 +540,7 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_steps_kernel(const srs_fie
       S[2 * J.stride + i] = pos.z;
     }
     const double hh = I.h * 0.5, h6 = I.h / 6.0;
-    o = fields.step(nfields, I.qomg, I.h, hh, h6, pos, vel);
+    o = fields.step(nfields, J, I.qomg, I.h, hh, h6, pos, vel);
     const V3 *const part[4] = {&o.r1, &o.r2, &o.r3, &o.d};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -887,9 +892,11 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
     }
   // (the undulators' phases are bounded by the way light goes: a step that turns the velocity by less than a
   // radian does not lengthen it; RK4 grows beyond 2.8)
-  int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time);
+  double reach = 0.0;
+  int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time, &reach);
   if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
-  const Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
+  Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
+  J.reach = reach;
   if (undulators && nparticles > kExactMaxParticles)
     return routed(launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x,
                                    d_b, d_a, d_specs, s),

@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(64 * kPairs) rk4_lanes_kernel(const srs_field 
             o[3 * ld] = vel.x; o[4 * ld] = vel.y; o[5 * ld] = vel.z;
             o[6 * ld] = acc.x; o[7 * ld] = acc.y; o[8 * ld] = acc.z;
           }
+          if (k * steps + s + 1 >= own.records) continue;  // (the phases' bound ends with the chain)
           const Increments d = und_increments<kN>(held, qomg, h, hh, h6, pos, vel);
           pos = v3(pos.x + advance(h6, vel.x, d.r1.x, d.r2.x, d.r3.x), pos.y + advance(h6, vel.y, d.r1.y, d.r2.y, d.r3.y),
                    pos.z + advance(h6, vel.z, d.r1.z, d.r2.z, d.r3.z));
@@ -149,7 +150,8 @@ cudaError_t launch(const srs_field *d_fields, int nfields, const srs_particle *d
 
 }  // namespace
 
-int undulators_along_z(const srs_field *f, int nfields, const srs_particle *particles, int nparticles, double time) {
+int undulators_along_z(const srs_field *f, int nfields, const srs_particle *particles, int nparticles, double time,
+                       double *reach) {
   if (nfields < 1 || nfields > kMaxUndulators) return 0;
   double far = kC * time;  // |z| stays below
   for (int p = 0; p < nparticles; ++p) {
@@ -162,9 +164,10 @@ int undulators_along_z(const srs_field *f, int nfields, const srs_particle *part
     if (f[i].kind != SRS_FIELD_UNDULATOR || f[i].taper != 0 || f[i].period[0] != 0 || f[i].period[1] != 0 ||
         !(lambda > 1e-100 && lambda < 1e100))
       return 0;
-    // the phases stay below 1e5 rad (twice the reach)
+    // the phases stay below 1e5 rad up to twice that
     if (!((2.0 * far + std::fabs(f[i].center[2])) / lambda + std::fabs(f[i].phase) < 1.5e4)) return 0;
   }
+  if (reach) *reach = 1.05 * far;
   return nfields;
 }
 

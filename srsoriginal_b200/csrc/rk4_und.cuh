@@ -2,9 +2,10 @@
 // rk4_exact.cu; compiled with -fmad=false).  The operations and their order are field_one's, force's and
 // the serial kernel's (rk4_fields.cuh, rk4.cu), so the results are theirs bit for bit; what is left out is
 // exact: products with the direction's zeros and one, the taper's 1 + 0 D, sums with zero.  Only the
-// stages' z is formed, and the sines of two stages run side by side: their phases are known to be below
-// 1e5, which lets the compiler drop sin's large-argument branch and interleave two calls (two calls 533
-// -> 356 cycles).
+// stages' z is formed, and the sines of two stages run side by side: their phases are below 1e5 for every state of
+// a trajectory (undulators_along_z bounds them), which lets the compiler drop sin's large-argument branch and
+// interleave two calls (two calls 533 -> 356 cycles).  A caller whose states are only iterates keeps them within that
+// bound.
 #pragma once
 
 #include <cuda_runtime.h>
