@@ -39,12 +39,14 @@ __device__ __forceinline__ double und_phase(const UndField &f, double D) {
   return div_rn(two_pi() * (D - f.ps), f.plen, f.rplen);
 }
 
-// field_one's value at D for the sine s
+// field_one's value at D for the sine s, added to the field sum's zero as field_sum starts it: a component of -0
+// (a field component of zero, or outside) is +0, as there; the fused operation rounds the product as a multiplication
+// does.
 __device__ __forceinline__ V3 und_value(const UndField &f, double D, double s) {
   const double *e = f.edge;
   const bool out = D > e[5] || D < e[0], end = D < e[2] || D > e[3], tip = D < e[1] || D > e[4];
   const double fac = out ? 0.0 : end ? (tip ? 0.25 : 0.75) : 1.0;
-  return v3(f.F[0] * fac * s, f.F[1] * fac * s, f.F[2] * fac * s);
+  return v3(__fma_rn(f.F[0] * fac, s, 0.0), __fma_rn(f.F[1] * fac, s, 0.0), __fma_rn(f.F[2] * fac, s, 0.0));
 }
 
 __device__ __forceinline__ double und_sine(double x) {
