@@ -783,6 +783,7 @@ Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const Tra
   const int64_t m = std::max<int64_t>(std::max(mf, mb), 0);
   J.stride = (m + 2) / 2 * 2;
   J.maxblk = (int)((m + kStepsPerBlock - 1) / kStepsPerBlock);
+  J.reach = 0.0;
   J.by_runs = m >= kRunsMinSteps + kRunsStepsPerBlock * J.nparticles * J.chains * J.maxblk;
   return J;
 }
@@ -838,6 +839,18 @@ constexpr int64_t kExactMaxSteps = (int64_t)1 << 26;
 // passes and sweeps ran for it, 537 and 2518).
 constexpr double kExactMaxTurn = 3.0, kExactMaxTurnUndulators = 2.2;
 
+// More particles through undulators go one chain per lane (rk4_lanes.cu), where that is the faster kernel: from 128
+// steps (257 to 4096 particles of 20 points 53-66 against 53-76 us, of 2 26-42 against 40-57, of 100 133-181 against
+// 114-169), and not just above the counts where its time nearly doubles at once, as the warps' lanes fill beyond 16
+// and as a second warp per scheduler begins (1001 points, serial against lanes: 9400 particles 1.44 / 0.97 ms, 9500
+// 1.55 / 1.65, 10000 1.77 / 1.66; 18944 2.90 / 1.70, 19000 2.89 / 3.27, 20000 3.33 / 3.28; 60000 8.8 / 6.8; through two
+// undulators, and with two chains, only the second).
+constexpr int64_t kLanesMinSteps = 128, kSchedulers = 148 * 4;
+static bool lanes_pay(int undulators, int64_t items, int chains) {
+  auto just_above = [&](int64_t count) { return items > count && items < count + count / 20; };
+  return !(undulators == 1 && chains == 1 && just_above(kSchedulers * 16)) && !just_above(kSchedulers * 32);
+}
+
 static double turn_bound(const srs_field *fields, int nfields, const srs_particle *particles, int nparticles, double time) {
   double b = 0.0, q = 0.0;
   for (int f = 0; f < nfields; ++f)
@@ -885,32 +898,34 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   const int64_t stage_doubles = nfields > 0 ? grid_stage_doubles(host_fields, nfields) : 0;
   const bool electric = has_electric(host_fields, nfields);
   double time = dt * (double)(nfwd + nbwd), step = dt;
+  int64_t steps = std::max(nfwd - 1, nbwd);
   if (host_specs)
     for (int p = 0; p < nparticles; ++p) {
       time = std::max(time, host_specs[p].dt * (double)(host_specs[p].nfwd + host_specs[p].nbwd));
       step = std::max(step, host_specs[p].dt);
+      steps = std::max({steps, host_specs[p].nfwd - 1, host_specs[p].nbwd});
     }
-  // (the undulators' phases are bounded by the way light goes: a step that turns the velocity by less than a
-  // radian does not lengthen it; RK4 grows beyond 2.8)
-  double reach = 0.0;
-  int undulators = electric ? 0 : undulators_along_z(host_fields, nfields, host_particles, nparticles, time, &reach);
-  if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
   Job J = make_job(d_particles, d_specs, host_specs, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a);
-  J.reach = reach;
-  if (undulators && nparticles > kExactMaxParticles)
-    return routed(launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x,
-                                   d_b, d_a, d_specs, s),
-                  nullptr);
+  const int64_t items = (int64_t)nparticles * J.chains, padded = (int64_t)J.maxblk * kStepsPerBlock;
   auto serial = [&](const int *d_skip) {
     if (d_route && !d_skip)
       if (cudaError_t e = cudaMemsetAsync(d_route, 0, sizeof(int32_t) * (size_t)nparticles, s)) return e;
     return launch_rk4(d_fields, nfields, d_particles, nparticles, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles,
                       electric, d_specs, d_skip);
   };
-  const int64_t items = (int64_t)nparticles * J.chains;
-  if (electric || (int64_t)J.maxblk * kStepsPerBlock <= kExactMinSteps || nparticles > kExactMaxParticles ||
-      (int64_t)J.maxblk * kStepsPerBlock > kExactMaxSteps)
+  const bool few = nparticles <= kExactMaxParticles;
+  if (electric || (few ? padded <= kExactMinSteps || padded > kExactMaxSteps : steps < kLanesMinSteps))
     return serial(nullptr);
+  // (the undulators' phases are bounded by the way light goes: a step that turns the velocity by less than a
+  // radian does not lengthen it; RK4 grows beyond 2.8)
+  int undulators = undulators_along_z(host_fields, nfields, host_particles, nparticles, time, &J.reach);
+  if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
+  if (!few) {
+    if (!undulators || !lanes_pay(undulators, items, J.chains)) return serial(nullptr);
+    return routed(launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x,
+                                   d_b, d_a, d_specs, s),
+                  nullptr);
+  }
   if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) <
         (undulators ? kExactMaxTurnUndulators : kExactMaxTurn)))
     return serial(nullptr);

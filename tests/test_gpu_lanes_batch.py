@@ -29,3 +29,30 @@ def test_short_chains_beside_long_ones(field):
     for k in range(n):
         for a in ("x", "beta", "aoc"):
             assert torch.equal(getattr(got[k], a), getattr(ref[k], a)), (k, a)
+
+
+# The counts of steps and chains between which a batch takes the lanes: 128 steps; not up to a twentieth above 16
+# lanes of a warp on each of 592 schedulers (one undulator, one chain), nor above 32.
+@pytest.mark.parametrize("field,particles,npoints,start,route", [
+    ("undulator", MANY, 128, 0.0, "SERIAL"), ("undulator", MANY, 129, 0.0, "LANES"), ("epu", MANY, 260, -1.0, "LANES"),
+    ("undulator", 9472, 129, 0.0, "LANES"), ("undulator", 9473, 129, 0.0, "SERIAL"),
+    ("undulator", 9944, 129, 0.0, "SERIAL"), ("undulator", 9945, 129, 0.0, "LANES"), ("epu", 9473, 129, 0.0, "LANES"),
+    ("undulator", 4800, 260, -1.0, "LANES"), ("epu", 18944, 129, 0.0, "LANES"), ("epu", 18945, 129, 0.0, "SERIAL"),
+    ("undulator", 9473, 260, -1.0, "SERIAL"), ("undulator", 19891, 129, 0.0, "LANES"),
+])
+def test_route_and_bits_at_the_edges_of_the_rule(field, particles, npoints, start, route):
+    import torch
+
+    from srsoriginal_b200 import _lib, device as D
+    from test_gpu_exact_route import _route
+
+    fields = _fields(field)[0]
+    z0 = -1.0 if start == 0.0 else 0.0
+    parts = [D.ideal_particle(3.0 - 1e-2 * k, [1e-6 * k, 0, z0], [1e-6 * k, 0, 1])[0] for k in range(7)]
+    parts = (parts * (particles // 7 + 1))[:particles]
+    got, taken = _route(fields, parts, start, npoints)
+    ref = D.trajectory(fields + _fields("nothing")[0], parts, start, start + 2.0, 0.0, npoints)
+    torch.cuda.synchronize()
+    assert (taken == getattr(_lib, "ROUTE_" + route)).all()
+    for a in ("x", "beta", "aoc"):
+        assert torch.equal(getattr(got, a), getattr(ref, a)), a
