@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(128) rk4_warp_kernel(const srs_field *__restri
     prepare(sf[i], sp[i]);
   }
   __syncthreads();
-  if (stage_doubles > 0) stage_grids(sf, sp, nfields);
+  if (stage_doubles > 0) stage_grids<false>(sf, sp, nfields);
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1), gbase = lane - gl;
   // G == 32: the block's four warps all integrate the block's one particle (the same instruction
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(64) rk4_thread_kernel(const srs_field *__restr
     prepare(sf[i], sp[i]);
   }
   __syncthreads();
-  if (stage_doubles > 0) stage_grids(sf, sp, nfields);
+  if (stage_doubles > 0) stage_grids<false>(sf, sp, nfields);
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nparticles) return;
   const srs_particle P = particles[p];

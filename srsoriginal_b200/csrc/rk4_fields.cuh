@@ -178,18 +178,27 @@ __device__ __forceinline__ void copy_fields(srs_field *sf, Prepared *sp, const s
 // the total when that fits) and points the prepared fields at the copies: the interpolation then
 // reads shared memory instead of global memory inside the serial RK4 chain.
 extern __shared__ __align__(16) double g_stage[];
+// kAsync: by asynchronous copies, all in flight at once (2001 samples 1.5 us; by a loop of loads and stores 9 us), in
+// the shooting passes, which copy once per pass.  The serial kernels copy once per call, and the compiler schedules
+// their step worse beside the asynchronous form (10001 points 8.80 -> 8.95 ms).
+template <bool kAsync>
 __device__ void stage_grids(const srs_field *sf, Prepared *sp, int nfields) {
   int64_t off = 0;
   for (int i = 0; i < nfields; ++i) {
     if (field_shape(sf[i].kind) != SRS_FIELD_GRID) continue;
     const int64_t cnt = 3 * sf[i].n[0] * sf[i].n[1] * sf[i].n[2];
-    // asynchronous copies, all in flight at once (a loop of loads and stores: 9 us for 2001 samples, 1.5 so)
-    const double *const data = sf[i].data;
-    for (int64_t k = threadIdx.x; k < cnt; k += blockDim.x) __pipeline_memcpy_async(g_stage + off + k, data + k, 8);
+    if constexpr (kAsync) {
+      const double *const data = sf[i].data;
+      for (int64_t k = threadIdx.x; k < cnt; k += blockDim.x) __pipeline_memcpy_async(g_stage + off + k, data + k, 8);
+    } else {
+      for (int64_t k = threadIdx.x; k < cnt; k += blockDim.x) g_stage[off + k] = sf[i].data[k];
+    }
     off += cnt;
   }
-  __pipeline_commit();
-  __pipeline_wait_prior(0);
+  if constexpr (kAsync) {
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     off = 0;

@@ -212,7 +212,7 @@ __device__ __forceinline__ void shoot_pass(PassShared<kShootThreads / G> &sh, co
     for (int k = t; k < M * 6; k += blockDim.x) W.U[6 * g0 + k] = sU[k / 6][k % 6];
     if (t < 6) rec[126 + t] = sU[0][t];
   }
-  if (stage_doubles > 0) stage_grids(sf, sp, nfields);  // (ends with a barrier)
+  if (stage_doubles > 0) stage_grids<true>(sf, sp, nfields);  // (ends with a barrier)
 
   // (2) integrate
   const Seg S = seg_of(P, g);
