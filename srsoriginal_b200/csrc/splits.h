@@ -6,19 +6,19 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
-#include <utility>
+#include <tuple>
 
 namespace srs {
 
 // Resident CTAs of `kernel` (`threads` threads, no dynamic shared memory) on the current device, queried
-// once per (kernel, device): the launchers ask on every call.
+// once per (kernel, device, threads): the launchers ask on every call.
 template <typename K>
 inline int64_t wave_slots(K kernel, int threads) {
   static std::mutex mu;
-  static std::map<std::pair<const void *, int>, int64_t> cache;
+  static std::map<std::tuple<const void *, int, int>, int64_t> cache;
   int dev = 0, sms = 148, occ = 1;
   const bool have_dev = cudaGetDevice(&dev) == cudaSuccess;
-  const auto key = std::make_pair(reinterpret_cast<const void *>(kernel), dev);
+  const auto key = std::make_tuple(reinterpret_cast<const void *>(kernel), dev, threads);
   {
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
