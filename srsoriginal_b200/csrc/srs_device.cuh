@@ -130,6 +130,26 @@ __device__ __forceinline__ double div_rn(double a, double b, double rb) {
   return __fma_rn(r, rb, q);
 }
 
+// m = RN(sqrt(a)) and y = 1/sqrt(a) to about an ulp, for normal positive a: the hardware's approximation
+// (rsqrt.approx.ftz.f64, ~20 bits), one third-order Newton step, and the correctly rounded root from the
+// exact remainder a - g^2 (P. Markstein, IBM J. Res. Dev. 34(1), 1990).
+__device__ __forceinline__ void sqrt_both(double a, double &m, double &y) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+  const double e = __fma_rn(-(a * y0), y0, 1.0);
+  y = __fma_rn(y0 * e, __fma_rn(0.375, e, 0.5), y0);
+  const double g = a * y, r = __fma_rn(-g, g, a);
+  m = __fma_rn(r, 0.5 * y, g);
+}
+
+// 1/a to about an ulp, for normal a: the hardware's approximation and two Newton steps.
+__device__ __forceinline__ double reciprocal(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  x = __fma_rn(x, __fma_rn(-a, x, 1.0), x);
+  return __fma_rn(x, __fma_rn(-a, x, 1.0), x);
+}
+
 __device__ inline V3 grid_at(const double *data, const srs_field &f, int64_t ix, int64_t iy, int64_t iz) {
   return ld3(data + 3 * (ix * f.n[1] * f.n[2] + iy * f.n[2] + iz));
 }
@@ -257,8 +277,9 @@ __device__ __forceinline__ double reduce_2pi(double x) {
   return r;
 }
 
-// Whether a phase may lie beyond the reduction of sincos_reduced (7.4 MeV at 30 m); NaN too.
-__device__ __forceinline__ bool phases_far(double omega, double tau) { return !(fabs(omega) * fabs(tau) < 0x1p50); }
+// Whether a phase may lie beyond the reduction of sincos_reduced (1.8 MeV at 30 m); NaN too.
+constexpr double kFarPhase = 0x1p48;
+__device__ __forceinline__ bool phases_far(double omega, double tau) { return !(fabs(omega) * fabs(tau) < kFarPhase); }
 
 // An upper bound on the |v| of a block of four warps (from their high words), complete after the next barrier.
 struct BlockBound {
@@ -272,17 +293,10 @@ struct BlockBound {
   }
 };
 
-// sin and cos of x for |x| < 2^50: x = k pi/2 + r by Cody & Waite's steps (k from the 1.5 * 2^52 shift; a
-// third part of pi/2, below |k| * 2e-33, would not be seen), then sin r = r + r^3 S(r^2) and cos r = 1 -
-// r^2/2 + r^4 C(r^2) with S and C the degree-5 interpolants at the Chebyshev nodes of [0, (pi/4)^2] of
-// (sin(r)/r - 1)/r^2 and (cos(r) - 1 + r^2/2)/r^4: 1e-17 and 5e-19 from the functions.
-__device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs) {
-  const double shift = 6755399441055744.0;
-  const double kd = __fma_rn(x, 0.6366197723675814, shift);
-  const int k = __double2loint(kd);
-  const double kf = kd - shift;
-  double r = __fma_rn(-kf, 1.5707963267948966, x);
-  r = __fma_rn(-kf, 6.123233995736766e-17, r);
+// sin and cos of k pi/2 + r, |r| <= pi/4: sin r = r + r^3 S(r^2) and cos r = 1 - r^2/2 + r^4 C(r^2) with S and C the
+// degree-5 interpolants at the Chebyshev nodes of [0, (pi/4)^2] of (sin(r)/r - 1)/r^2 and (cos(r) - 1 +
+// r^2/2)/r^4: 1e-17 and 5e-19 from the functions (up to |r| = 0.81 5e-17 and 3e-18).
+__device__ __forceinline__ void sincos_quadrant(double r, int k, double &sn, double &cs) {
   const double w = r * r;
   double s = __fma_rn(w, 1.5918129266803394e-10, -2.5051131844614108e-08);
   double c = __fma_rn(w, -1.1382632407965617e-11, 2.087614626815952e-09);
@@ -301,14 +315,35 @@ __device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs)
   cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((k + 1) & 2) << 30), __double2loint(b));
 }
 
-// The same for any x: phases beyond 2^50 rad are accepted, though a double holds them to a quarter of a radian
-// only, and reduced first (beyond 2^103 more than once).  A tile is summed this way when a bound on its phases
-// (phases_far) says so: testing every phase cost the sums 5 %.
+// sin and cos of x for |x| < kFarPhase: x = k pi/2 + r by Cody & Waite's steps, k from the 1.5 * 2^52 shift (a third
+// part of pi/2, below |k| * 2e-33, would not be seen).  The rounding of 2/pi makes k a neighbour's near a tie: |r| <=
+// pi/4 + 1e-16 |k|, 0.81 at most; at 2^50 rad it would be 0.89, and the sine 1e-15 off.  Within 2.4e-16 to 2^46 rad
+// (measured 1.7e-16), 3e-16 to 2^48.
+__device__ __forceinline__ void sincos_reduced(double x, double &sn, double &cs) {
+  const double shift = 6755399441055744.0;
+  const double kd = __fma_rn(x, 0.6366197723675814, shift);
+  const double kf = kd - shift;
+  double r = __fma_rn(-kf, 1.5707963267948966, x);
+  r = __fma_rn(-kf, 6.123233995736766e-17, r);
+  sincos_quadrant(r, __double2loint(kd), sn, cs);
+}
+
+// The same for any x: phases beyond are accepted, though a double holds them to a tenth of a radian or worse, with k
+// corrected to the nearest (and reduced modulo 2 pi before, beyond 2^50; beyond 2^103 more than once).  A tile is
+// summed this way when a bound on its phases (phases_far) says so: testing every phase cost the sums 5 %.
 template <bool kFar>
 __device__ __forceinline__ void sincos_phase(double x, double &sn, double &cs) {
-  if constexpr (kFar)
+  if constexpr (!kFar) {
+    sincos_reduced(x, sn, cs);
+  } else {
     for (int k = 0; k < 20 && fabs(x) >= 0x1p50; ++k) x = reduce_2pi(x);
-  sincos_reduced(x, sn, cs);
+    double k = rint(x * 0.6366197723675814);
+    const double over = __fma_rn(-k, 1.5707963267948966, x);
+    if (fabs(over) > 0.7853981633974483) k += copysign(1.0, over);
+    double r = __fma_rn(-k, 1.5707963267948966, x);
+    r = __fma_rn(-k, 6.123233995736766e-17, r);
+    sincos_quadrant(r, (int)(__double2ll_rn(k) & 3), sn, cs);
+  }
 }
 
 // reduce_2pi in FP32 arithmetic, for arguments of a few hundred radians at most.

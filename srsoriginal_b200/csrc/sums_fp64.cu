@@ -44,26 +44,6 @@ namespace {
 
 constexpr int kTile = 128;     // outputs per CTA and trajectory points per shared-memory tile
 
-// m = RN(sqrt(a)) and y = 1/sqrt(a) to about an ulp, for normal positive a: the hardware's approximation
-// (rsqrt.approx.ftz.f64, ~20 bits), one third-order Newton step, and the correctly rounded root from the
-// exact remainder a - g^2 (P. Markstein, IBM J. Res. Dev. 34(1), 1990).
-__device__ __forceinline__ void sqrt_both(double a, double &m, double &y) {
-  double y0;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
-  const double e = __fma_rn(-(a * y0), y0, 1.0);
-  y = __fma_rn(y0 * e, __fma_rn(0.375, e, 0.5), y0);
-  const double g = a * y, r = __fma_rn(-g, g, a);
-  m = __fma_rn(r, 0.5 * y, g);
-}
-
-// 1/a to about an ulp, for normal a: the hardware's approximation and two Newton steps.
-__device__ __forceinline__ double reciprocal(double a) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
-  x = __fma_rn(x, __fma_rn(-a, x, 1.0), x);
-  return __fma_rn(x, __fma_rn(-a, x, 1.0), x);
-}
-
 // Trajectory points per CTA for `ctas` tiles of outputs: the split of least waves * (points + overhead)
 // over the launches of up to six full waves, in multiples of 32 points (a small output then still
 // spreads over the GPU).

@@ -26,3 +26,8 @@ def _run(name, tmp_path):
 def test_wave_slots_of_several_block_sizes(tmp_path):
     r = _run("wave_slots_check", tmp_path)
     assert r.returncode == 0 and "bad 0" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_own_roots_reciprocals_and_sines(tmp_path):
+    r = _run("device_math_check", tmp_path)
+    assert r.returncode == 0 and "bad 0" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
