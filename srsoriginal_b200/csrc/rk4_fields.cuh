@@ -96,9 +96,15 @@ __device__ __forceinline__ bool along_axis(const Prepared &p, V3 X, double &x) {
 
 // The cell (0 .. last) of the quotient q by the step, as grid_interp limits it.  A position that is not a number
 // passes along_axis (both of its comparisons are false); its q is in no cell and takes the last one, whose samples
-// it then only multiplies into a NaN.  (A conversion to int alone would give INT_MIN.)
+// it then only multiplies into a NaN.  On the GPU a conversion to unsigned gives 0 below zero and 2^31 for NaN, and
+// whatever it gives the minimum is a cell (a conversion to int gave INT_MIN; two comparisons in place of the
+// minimum made a gradient pass 0.7 % longer).
 __host__ __device__ __forceinline__ int axis_cell(double q, int last) {
+#ifdef __CUDA_ARCH__
+  return (int)min(__double2uint_rz(q), (unsigned)last);
+#else
   return !(q < (double)last) ? last : q > 0.0 ? (int)q : 0;
+#endif
 }
 
 __device__ inline V3 field_one(const Prepared &p, const srs_field &f, V3 X) {
