@@ -286,6 +286,12 @@ def run_reference(args, world, rank):
     if rank != 0:
         return 0
     threads = os.cpu_count() or 1
+    try:
+        reference_module()
+    except ImportError as e:  # built by oracle/Makefile where the reference's sources are
+        print(json.dumps({"impl": "reference", "unavailable": f"the reference is not built in oracle/_ref: {e}"}),
+              flush=True)
+        return 0
     dt, ev = reference_sample(2, threads)
     # each step: a bounded sample sized so warmup + steps stay within a few minutes
     per_step_target = max(1.0, 150.0 / max(1, args.steps + args.warmup))
