@@ -405,7 +405,8 @@ def measure_configs(dev, peaks=None):
                                           "without the per-call launch overhead",
                             "mixed_error_vs_fp64": error_floors(spm.cpu().numpy(), sp.cpu().numpy())}
 
-    # the trajectory: serial RK4 chain against the parallel-in-time integration (configs 0/1 and 2)
+    # the trajectory (configs 0/1 and 2): with the serial chain's bits, which the library forms in parallel too, and
+    # by shooting
     epu = und + [D.undulator([0.6, 0, 0], [0, 0, W.PERIOD], W.NPERIODS, phase=np.pi / 2)]
     rec = {}
     for npts, fields in ((NT, und), (40001, epu)):
@@ -417,7 +418,7 @@ def measure_configs(dev, peaks=None):
         torch.cuda.synchronize()
         s = st.cpu().tolist()
         rec[f"{npts}_points_{len(fields)}_undulators"] = {
-            "serial_ms": ms_ser, "parallel_in_time_ms": ms_sho, "speedup": ms_ser / ms_sho,
+            "serial_bits_ms": ms_ser, "shooting_ms": ms_sho,
             "newton_iterations": int(s[1]), "converged": bool(s[0]),
             "max_abs_dx_m": float((sho.x - ser.x).abs().max()), "max_abs_dbeta": float((sho.beta - ser.beta).abs().max())}
     out["trajectory"] = rec
@@ -685,11 +686,11 @@ def run_ours(args, world, rank, local):
         torch.cuda.synchronize()
         return max_over_ranks(time.perf_counter() - t0, world)
 
-    # the same steps with the serial RK4 chain, for comparison (not the reported value)
+    # the same steps with the serial chain's bits, for comparison (not the reported value)
     o.set_trajectory_mode("serial")
     e2e_serial_s = timed_e2e(min(3, e2e_steps))
     o.set_trajectory_mode("auto")
-    # the same steps in plain FP64 (the drop-in: serial RK4 in the reference's arithmetic, FP64 maps),
+    # the same steps in plain FP64 (the drop-in: the serial RK4's bits in the reference's arithmetic, FP64 maps),
     # the like-precision comparison with the reference's CPU path
     fp64_steps = max(1, min(3, e2e_steps))
 
@@ -724,7 +725,7 @@ def run_ours(args, world, rank, local):
     e2e_fp64 = {"value": world * EVALS_PER_STEP * fp64_steps / e2e_fp64_s, "unit": UNIT,
                 "h2d_bytes_per_step": 56, "d2h_bytes_per_step": len(ENERGIES) * npts * 8,
                 "ms_per_step": 1e3 * e2e_fp64_s / fp64_steps,
-                "includes": "plain FP64 through the same API: serial RK4 trajectory, both FP64 maps, host copies"}
+                "includes": "plain FP64 through the same API: the serial RK4's bits, both FP64 maps, host copies"}
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
@@ -754,7 +755,7 @@ def run_ours(args, world, rank, local):
 
 
 PROFILE_CASES = ("flux_mixed_cfg1", "flux_fp64_cfg1", "pd_fp64_51x51", "spectrum_mixed_3a256", "shoot_cfg1",
-                 "spectrum_cfg0", "adjoint_cfg4")
+                 "spectrum_cfg0", "adjoint_cfg4", "exact_cfg1", "lanes_1024")
 
 
 def run_case(name):
@@ -762,7 +763,8 @@ def run_case(name):
     flux_mixed_cfg1 / flux_fp64_cfg1: the config-1 map at 3*E1 (mixed / plain FP64); pd_fp64_51x51:
     config 2's power density on 51 x 51 points (40001-point trajectory, plain FP64);
     spectrum_mixed_3a256: 256 electrons of config 3a's shape (20001 points, 2000 energies, mixed);
-    shoot_cfg1: the config-1 trajectory integrated parallel in time; spectrum_cfg0: config 0's
+    shoot_cfg1: the config-1 trajectory by shooting; exact_cfg1: with the serial chain's bits; lanes_1024: 1024
+    electrons of 5001 points; spectrum_cfg0: config 0's
     1000-energy spectrum, mixed then plain FP64; adjoint_cfg4: config 4's forward and adjoint."""
     import numpy as np
     import torch
@@ -797,6 +799,10 @@ def run_case(name):
             D.spectrum(tb, charge, current, [0, 0, W.SCREEN_Z], e, out, precision=_lib.MIXED)
         elif name == "shoot_cfg1":
             D.trajectory_shoot(und, part, 0.0, 2.0, 0.0, NT)
+        elif name == "exact_cfg1":
+            D.trajectory(und, [part], 0.0, 2.0, 0.0, NT)
+        elif name == "lanes_1024":
+            D.trajectory(und, [part] * 1024, 0.0, 2.0, 0.0, 5001)
         elif name == "adjoint_cfg4":
             from srsoriginal_b200.adjoint import backward_flux, forward_flux
             problem, grid4, ic4, de4 = W.config4_problem()

@@ -40,10 +40,10 @@
 // trajectory, bit for bit.  Both chains of the trajectory (forward from t0, backward) and several
 // particles are integrated side by side.
 //
-// Measured on a B200 (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.17 ms, 40001
-// through two 39.0 -> 0.35 ms, 12001 through a field map in two chains 14.1 -> 0.16 ms, 24 particles of
-// 10001 points 9.1 -> 0.54 ms, 2001 points 1.78 -> 0.13 ms, 300 points 0.28 -> 0.10 ms.  A pass is bound by
-// latency (~7 us: launch, loads, four field evaluations, 2 x 128 additions in order); a sweep takes 0.16 ms
+// Measured on a B200 around a call (serial kernel -> here): 20001 points through one undulator 17.6 -> 0.20 ms,
+// 40001 through two 39.0 -> 0.35 ms, 12001 through a field map in two chains 14.1 -> 0.14 ms, 24 particles of
+// 10001 points 9.1 -> 0.44 ms, 2001 points 1.78 -> 0.14 ms, 300 points 0.28 -> 0.11 ms.  A pass is bound by
+// latency (~6.5 us: launch, loads, four field evaluations, 2 x 128 additions in order); a sweep takes 0.16 ms
 // by the chain kernel on 20001 points, 0.05 ms by runs (20 us per list, 10 us per kernel of blocks).
 #include <cuda_runtime.h>
 
@@ -834,8 +834,8 @@ constexpr int64_t kExactMaxSteps = (int64_t)1 << 26;
 // And only where the iteration contracts: the angle by which the fields could turn a particle over the
 // whole trajectory, |q/(m gamma)| sum |B| T (grids not counted: their samples are on the device).  3 GeV
 // electrons in 1 T over 2 m: 0.2.  Through an undulator at 2.0 300, 2001 and 20001 points settle, at 2.4 two of
-// the three do not; other shapes may fill a part of the way only.  What is given up after the first pass costs 45 to
-// 75 us before the serial kernel (0.1 GeV through a 1 T map: 300 points 375 -> 449 us, 2001 2317 -> 2380; when all
+// the three do not; other shapes may fill a part of the way only.  What is given up after the first pass costs 55 to
+// 80 us before the serial kernel (0.1 GeV through a 1 T map: 300 points 376 -> 458 us, 2001 2335 -> 2391; when all
 // passes and sweeps ran for it, 537 and 2518).
 constexpr double kExactMaxTurn = 3.0, kExactMaxTurnUndulators = 2.2;
 

@@ -4,10 +4,10 @@
 // rk4.cu spends a warp's lanes on one particle (fields and stages side by side, shuffles to combine): a
 // step costs ~0.87 us there, and a batch is bound by the instructions per particle.  Here one lane
 // integrates one chain (forward or backward) of one particle with the step of rk4_und.cuh, bit for bit
-// rk4.cu's, bound by the latency of the step (~0.78 us, four sines two by two) whether one lane of the
-// warp is used or all 32.  So up to 592 x 32 chains take the time of one; they are spread over one warp
-// per scheduler first.  Measured (rk4.cu -> here): 1024 particles of 20001 points 22.1 -> 15.9 ms, 300
-// 38.6 -> 15.7 ms, 4096 of 10001 points 13.2 -> 8.6 ms.  (One double-double sincos per step rotated to the
+// rk4.cu's, bound by the latency of the step (~0.79 us, four sines two by two) whether one lane of the
+// warp is used or 16.  So up to 592 x 16 chains take about the time of one, and 592 x 32 twice that; they are spread
+// over one warp per scheduler first.  Measured (rk4.cu -> here): 1024 particles of 20001 points 22.0 -> 15.9 ms, 300
+// 38.6 -> 15.7 ms, 4096 of 10001 points 12.7 -> 8.4 ms, 18944 of 1001 points 2.9 -> 1.7 ms.  (One double-double sincos per step rotated to the
 // other stages took 8.9 ms for 1024, but an ulp in 2 % of the sines flips a last bit of a velocity
 // along the flight in some particles, which moves all later phases by ~1e-6 rad: not kept.)
 //
