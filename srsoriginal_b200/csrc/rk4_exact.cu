@@ -346,7 +346,7 @@ __global__ void pit_init_kernel(Job J, Scratch W, const srs_field *__restrict__ 
 // shift[0..2] of its start position, shift[3..5] of its start velocity (a velocity shift moves the
 // positions of all later blocks).  Every thread gets them; returns whether the item has settled: the
 // transverse mismatches at the rounding of the speed and none in a component that carries the flight
-// (its bits decide the phases); lost: some are above kLostMismatch.
+// (its bits decide the phases); lost: one that this thread looked at is above kLostMismatch.
 __device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I, int it, int s, int k,
                                   double (*red)[kStepsPerBlock / 32], double shift[6], bool *lost) {
   const double *const T = W.starts(k) + 6 * (int64_t)it * J.maxblk, *const E = W.ends(k) + 6 * (int64_t)it * J.maxblk;
@@ -383,8 +383,7 @@ __device__ inline bool mismatches(const Job &J, const Scratch &W, const Item &I,
     shift[c] = 0.0;
     for (int w = 0; w < kStepsPerBlock / 32; ++w) shift[c] += red[c][w];
   }
-  // (a barrier of its own: __syncthreads_or returns whether any argument was not zero, not their bits)
-  *lost = k >= kContracted && __syncthreads_or(big2 > kLostMismatch * kLostMismatch * v2);
+  *lost = k >= kContracted && big2 > kLostMismatch * kLostMismatch * v2;
   return !any;
 }
 
@@ -421,14 +420,15 @@ __global__ void __launch_bounds__(kStepsPerBlock) pit_pass_kernel(const srs_fiel
     double shift[6];
     bool lost;
     const bool ready = mismatches(J, W, I, it, s, pass - 1, red, shift, &lost);
-    if (lost || (kN == 0 && turn > (float)kMaxTurn * sqrtf((float)mag2(ld3(I.s0 + 3))))) {
+    const bool turned = kN == 0 && turn > (float)kMaxTurn * sqrtf((float)mag2(ld3(I.s0 + 3)));
+    if (lost || (turned && t == 0)) {
       // all items go to the serial kernel: no further pass of any (one that has settled keeps its number, which
       // its blocks are reading)
-      for (int q = t; q < (int)gridDim.y; q += kStepsPerBlock)
+      for (int q = 0; q < (int)gridDim.y; ++q)
         if (W.ready[q] == kPasses) W.ready[q] = pass - 1;
-      if (t == 0) *W.failed = 1;
-      return;
+      *W.failed = 1;
     }
+    if (turned) return;
     if (ready) {
       if (t == 0) W.ready[it] = pass - 1;
       return;
