@@ -105,7 +105,7 @@ struct Job {
   int64_t stride;          // doubles per component of an item's states
   int maxblk;              // pass blocks of the longest chain
   bool by_runs;            // the chains' additions by runs (kRunsMinSteps)
-  double reach;            // with undulators: a bound on |z| within which their phases are below 1e5
+  double reach, fast2;     // with undulators: bounds on |z| and |v|^2 of all states, which keep the phases below 1e5
 };
 
 struct Scratch {
@@ -200,11 +200,11 @@ struct Fields {
     long long *b = reinterpret_cast<long long *>(und);
     for (int k = threadIdx.x; k < kN * (int)(sizeof(UndField) / 8); k += blockDim.x) b[k] = a[k];
   }
-  // An iterate may lie anywhere, or be no number, where a trajectory's state does not: one out of reach, or faster
-  // than any particle, is not stepped, and fails the check.
+  // An iterate may lie anywhere, or be no number, where a trajectory's state does not: one out of the bounds is not
+  // stepped, and fails the check.
   __device__ __forceinline__ Increments step(int, const Job &J, double qomg, double h, double hh, double h6, V3 pos,
                                              V3 vel) const {
-    if (!(fabs(pos.z) < J.reach) || !(mag2(vel) < 1.05 * kC * kC)) pos.z = vel.x = vel.y = vel.z = 0.0;
+    if (!(fabs(pos.z) < J.reach) || !(mag2(vel) < J.fast2)) pos.z = vel.x = vel.y = vel.z = 0.0;
     return und_increments<kN>(und, qomg, h, hh, h6, pos, vel);
   }
 };
@@ -783,7 +783,7 @@ Job make_job(const srs_particle *d_particles, const TrajSpec *d_specs, const Tra
   const int64_t m = std::max<int64_t>(std::max(mf, mb), 0);
   J.stride = (m + 2) / 2 * 2;
   J.maxblk = (int)((m + kStepsPerBlock - 1) / kStepsPerBlock);
-  J.reach = 0.0;
+  J.reach = J.fast2 = 0.0;
   J.by_runs = m >= kRunsMinSteps + kRunsStepsPerBlock * J.nparticles * J.chains * J.maxblk;
   return J;
 }
@@ -916,19 +916,23 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   const bool few = nparticles <= kExactMaxParticles;
   if (electric || (few ? padded <= kExactMinSteps || padded > kExactMaxSteps : steps < kLanesMinSteps))
     return serial(nullptr);
-  // (the undulators' phases are bounded by the way light goes: a step that turns the velocity by less than a
-  // radian does not lengthen it; RK4 grows beyond 2.8)
-  int undulators = undulators_along_z(host_fields, nfields, host_particles, nparticles, time, &J.reach);
-  if (undulators && !(turn_bound(host_fields, nfields, host_particles, nparticles, step) < 1.0)) undulators = 0;
+  // The undulators' phases are bounded by the way that the particles can go.  In one field a step of less than 2.8
+  // rad does not lengthen the velocity, but its stages may lie in different fields: then v' = (1 + A + ...) v with A
+  // antisymmetric, |A| <= t, the step's turn, and further terms of t^2 / 2, t^3 / 6 and t^4 / 24 at most, so |v'| <= |v|
+  // (1 + t^2 + ...) < |v| exp(1.2 t^2) for t < 1, and exp(1.2 T t) over all steps of T rad together.
+  const double turn = turn_bound(host_fields, nfields, host_particles, nparticles, time);
+  const double step_turn = turn_bound(host_fields, nfields, host_particles, nparticles, step);
+  const double growth = exp(1.2 * turn * step_turn);
+  int undulators = 0;
+  if (step_turn < 1.0) undulators = undulators_along_z(host_fields, nfields, host_particles, nparticles, time * growth, &J.reach);
+  J.fast2 = 1.05 * kC * kC * growth * growth;
   if (!few) {
     if (!undulators || !lanes_pay(undulators, items, J.chains)) return serial(nullptr);
     return routed(launch_rk4_lanes(undulators, d_fields, nfields, d_particles, nparticles, J.chains, dt, nfwd, nbwd, d_x,
                                    d_b, d_a, d_specs, s),
                   nullptr);
   }
-  if (!(turn_bound(host_fields, nfields, host_particles, nparticles, time) <
-        (undulators ? kExactMaxTurnUndulators : kExactMaxTurn)))
-    return serial(nullptr);
+  if (!(turn < (undulators ? kExactMaxTurnUndulators : kExactMaxTurn))) return serial(nullptr);
   const size_t bytes = carve(J, nfields, nullptr, nullptr);
   if (bytes > kExactMaxScratch && nparticles > 1) {
     const int half = nparticles / 2;

@@ -88,7 +88,7 @@ __device__ inline V3 rotate_pre(V3 v, const Prepared &p) {
 }
 
 // The coordinate on a grid along one axis, and whether it is inside: grid_interp's arithmetic, from which the
-// identity rotation and the other axes' tests are left out (exact).
+// identity rotation and the other axes' tests are left out (exact where the other coordinates are finite).
 __device__ __forceinline__ bool along_axis(const Prepared &p, V3 X, double &x) {
   x = (p.kind == kGridAlong ? X.x : p.kind == kGridAlong + 1 ? X.y : X.z) - p.ps;
   return !(x <= p.b_lo || x >= p.b_hi);

@@ -115,8 +115,8 @@ cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particl
                        cudaStream_t s, int64_t stage_doubles, bool electric = false, const TrajSpec *d_specs = nullptr,
                        const int *d_skip = nullptr);
 // The number of fields if all are undulators that rk4_und.cuh integrates (at most two, period along +z, no
-// taper, phases of the given particles below 1e5 rad over the time [s]), else 0.  reach (optional): a bound on |z| for
-// all of their states, from which a step of at most 1.75 c stays within those phases too.
+// taper, phases of the given particles below 1e5 rad on a way of c times the time [s]), else 0.  reach (optional): a
+// bound on |z| for all of their states; from there a step of up to 0.9 of that way stays within those phases too.
 int undulators_along_z(const srs_field *host_fields, int nfields, const srs_particle *host_particles, int nparticles,
                        double time, double *reach = nullptr);
 // Trajectories of many particles through them, bit for bit launch_rk4's; chains: 2 when some particle has points before t0.
