@@ -24,6 +24,8 @@
 // first, earliest at index 0), so no reversal pass is needed.
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "rk4_fields.cuh"
 #include "srs_internal.h"
 
@@ -367,6 +369,13 @@ bool has_electric(const srs_field *host_fields, int nfields) {
   for (int i = 0; i < nfields; ++i)
     if (field_electric(host_fields[i].kind)) return true;
   return false;
+}
+
+bool finite_starts(const srs_particle *host_particles, int nparticles) {
+  for (int p = 0; p < nparticles; ++p)
+    for (int c = 0; c < 3; ++c)
+      if (!(std::fabs(host_particles[p].x0[c]) < 1e300) || !std::isfinite(host_particles[p].beta0[c])) return false;
+  return true;
 }
 
 cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,

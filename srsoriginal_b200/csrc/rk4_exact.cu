@@ -916,6 +916,7 @@ cudaError_t launch_trajectories(const srs_field *d_fields, int nfields, const sr
   const bool few = nparticles <= kExactMaxParticles;
   if (electric || (few ? padded <= kExactMinSteps || padded > kExactMaxSteps : steps < kLanesMinSteps))
     return serial(nullptr);
+  if (few && !finite_starts(host_particles, nparticles)) return serial(nullptr);
   // The undulators' phases are bounded by the way that the particles can go.  In one field a step of less than 2.8
   // rad does not lengthen the velocity, but its stages may lie in different fields: then v' = (1 + A + ...) v with A
   // antisymmetric, |A| <= t, the step's turn, and further terms of t^2 / 2, t^3 / 6 and t^4 / 24 at most, so |v'| <= |v|

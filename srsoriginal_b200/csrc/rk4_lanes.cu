@@ -152,17 +152,18 @@ cudaError_t launch(const srs_field *d_fields, int nfields, const srs_particle *d
 
 int undulators_along_z(const srs_field *f, int nfields, const srs_particle *particles, int nparticles, double time,
                        double *reach) {
-  if (nfields < 1 || nfields > kMaxUndulators) return 0;
+  if (nfields < 1 || nfields > kMaxUndulators || !finite_starts(particles, nparticles)) return 0;
   double far = kC * time;  // |z| stays below
   for (int p = 0; p < nparticles; ++p) {
     const double *const b = particles[p].beta0;
-    if (!(b[0] * b[0] + b[1] * b[1] + b[2] * b[2] <= 1.0 + 1e-9) || !std::isfinite(particles[p].x0[2])) return 0;
+    if (!(b[0] * b[0] + b[1] * b[1] + b[2] * b[2] <= 1.0 + 1e-9)) return 0;
     far = std::max(far, kC * time + std::fabs(particles[p].x0[2]));
   }
   for (int i = 0; i < nfields; ++i) {
     const double lambda = f[i].period[2];
     if (f[i].kind != SRS_FIELD_UNDULATOR || f[i].taper != 0 || f[i].period[0] != 0 || f[i].period[1] != 0 ||
-        !(lambda > 1e-100 && lambda < 1e100))
+        !(lambda > 1e-100 && lambda < 1e100) || !(std::fabs(f[i].center[0]) < 1e300) ||
+        !(std::fabs(f[i].center[1]) < 1e300))
       return 0;
     // the phases stay below 1e5 rad up to twice that
     if (!((2.0 * far + std::fabs(f[i].center[2])) / lambda + std::fabs(f[i].phase) < 1.5e4)) return 0;

@@ -605,8 +605,12 @@ cudaError_t launch_rk4_shoot(const srs_field *d_fields, int nfields, const srs_p
   const int iters = max_iterations > 0 ? max_iterations : kDefaultIters;
   const Plan P = make_plan(nfwd, nbwd, dt, steps_per_segment, nfields);
   const int segs = P.sfp + P.sbp;
-  if (segs == 0)  // nothing to integrate in parallel (a single point): the serial kernel
+  // nothing to integrate in parallel (a single point), or a start that is no number: the serial kernel
+  if (segs == 0 || !finite_starts(&host_particle, 1)) {
+    if (d_stats)
+      if (cudaError_t e = cudaMemsetAsync(d_stats, 0, 4 * sizeof(double), s)) return e;
     return launch_rk4(d_fields, nfields, d_particle, 1, dt, nfwd, nbwd, d_x, d_b, d_a, s, stage_doubles);
+  }
   Scratch W = carve(scratch, P);
   // scales of the convergence test: the trajectory's extent and speed
   const double C = kC;

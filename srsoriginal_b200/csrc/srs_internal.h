@@ -108,6 +108,9 @@ cudaError_t efield_time(const srs_traj_view &t, double charge, const double obs[
 int64_t grid_stage_doubles(const srs_field *host_fields, int nfields);
 // electric: some of the fields are electric (SRS_FIELD_ELECTRIC); has_electric tells from a HOST array
 bool has_electric(const srs_field *host_fields, int nfields);
+// Whether the particles (HOST array) start at numbers.  The serial kernel multiplies a coordinate that is none by a
+// direction's zeros, which gives NaN; undulators along z and maps along one axis leave those products out elsewhere.
+bool finite_starts(const srs_particle *host_particles, int nparticles);
 // d_specs: per-particle settings and outputs instead of the common ones; d_skip: return at once when
 // *d_skip != 0.
 cudaError_t launch_rk4(const srs_field *d_fields, int nfields, const srs_particle *d_particles, int nparticles,
